@@ -4,21 +4,18 @@
 // (CollisionManifold.cs:393-566) run fused; colliding pairs append one record (key,
 // normal, up to four point pairs) to the compacted contact stream.
 //
-// Lanes of a warp hold identical copies of the MPR state; point-cloud support maps, the
-// EPA face scans (closest face, visibility, fan construction) and the manifold's segment
-// intersections are split across lanes.  EPA keeps its face data in FP32; FP64 is used
-// only when a face normal is too cancelled to trust (exact expansion recomputation, as
-// the reference's ExpansionArithmetic.Normal) and when the FP32 orientation filter cannot
-// prove a sign (the reference's double filter, then exact expansions).  The device
-// polytope holds 64 vertices / 128 faces (the reference: 128 / 256); running out ends
-// EPA with the MPR result, the reference's behaviour on any EPA failure.
+// In the warp-per-pair stages the lanes hold identical copies of the MPR state; point-cloud
+// support maps, the EPA face scans (closest face, visibility, horizon), the FP64 face geometry
+// (four lanes per face) and the manifold's segment intersections are split across lanes.  EPA
+// keeps the reference's FP64 face data and polytope capacity (128 vertices, 256 faces); side
+// tests run an FP32 filter, the reference's FP64 filter, then exact expansions.  Running out
+// of capacity ends EPA with the MPR result, the reference's behaviour on any EPA failure.
 //
 // The MPR follows code the reference adapted from XenoCollide (zlib license, (c) 2007-2014
 // Gary Snethen, http://xenocollide.com): provided 'as-is', without any express or implied
 // warranty; altered source versions must be plainly marked as such; this notice may not
 // be removed or altered from any source distribution.
 #include "jg_shapes.cuh"
-#include <math_constants.h>
 
 namespace {
 
@@ -207,116 +204,182 @@ __device__ __forceinline__ bool safe_coord(float v) {
 }
 __device__ __forceinline__ bool is_safe(v3 p) { return safe_coord(p.x) && safe_coord(p.y) && safe_coord(p.z); }
 
-// FP64 vector helpers in the reference's evaluation order (ConvexPolytope.Double3).
-struct d3 { double x, y, z; };
-__device__ __forceinline__ d3 dv(v3 v) { return d3{(double)v.x, (double)v.y, (double)v.z}; }
-__device__ __forceinline__ double ddot(d3 a, d3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ d3 dcross(d3 a, d3 b) { return d3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
-__device__ __forceinline__ d3 dsub(d3 a, d3 b) { return d3{a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ d3 dadd(d3 a, d3 b) { return d3{a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ d3 dmul(d3 a, double s) { return d3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ bool dfinite(d3 a) { return isfinite(a.x) && isfinite(a.y) && isfinite(a.z); }
-__device__ __forceinline__ double dclamp01(double x) { return x < 0.0 ? 0.0 : (x > 1.0 ? 1.0 : x); }
+// ---- FP64 face geometry, four lanes per face ----------------------------------------------
+// An FP64 instruction holds its warp scheduler for 64 cycles on this part, whatever the number
+// of active lanes (measured, add, multiply and FMA alike; a division takes nine of them), and a
+// face needs about 250 when one lane evaluates it.  Here lane c of a group of four holds
+// component c of the vectors (the fourth repeats the first), so that an operation on three
+// components is one instruction, and the sums and quotients of a face that do not depend on
+// each other take one lane each: about 85 instructions for up to eight faces.  Every operation
+// and its order are the reference's, so the values are those of the one-lane form bit for bit.
+// k_epa, bound by this pipe: 1374 -> 734 us on a settled 100k-body pile (7.2k deep pairs), 545 ->
+// 300 us where a few hundred pairs leave only the latency of the longest one; k_edge 513 -> 384.
+// Signs and maxima of finite doubles are decided on their bit patterns (integer pipe).
+__device__ __forceinline__ double grp(double x, int src) { return __shfl_sync(FULL, x, src, 4); }
+__device__ __forceinline__ bool x_nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+__device__ __forceinline__ bool d_lt0(double x) { return __double_as_longlong(x) < 0 && x_nonzero(x); }
+__device__ __forceinline__ bool d_ge0(double x) { return !d_lt0(x); }
+__device__ __forceinline__ bool d_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ long long d_absbits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
 
-// ConvexPolytope.CalcBarycentric (ConvexPolytope.cs:328-395), FP64.
-__device__ bool calc_bary(d3 a, d3 b, d3 c, d3 n, double nscale, double nsq, d3& out) {
-    d3 u = dsub(a, b), v = dsub(a, c);
-    double gamma = (ddot(dcross(u, a), n) / nsq) / nscale;
-    double beta = (ddot(dcross(a, v), n) / nsq) / nscale;
-    double alpha = 1.0 - gamma - beta;
-    bool clamped = false;
-    if (alpha >= 0 && beta < 0) {
-        double t = ddot(a, u);
-        if (gamma < 0 && t > 0) { beta = fmin(1.0, t / ddot(u, u)); alpha = 1 - beta; gamma = 0; }
-        else { gamma = dclamp01(ddot(a, v) / ddot(v, v)); alpha = 1 - gamma; beta = 0; }
-        clamped = true;
-    } else if (beta >= 0 && gamma < 0) {
-        d3 w = dsub(b, c);
-        double t = ddot(b, w);
-        if (alpha < 0 && t > 0) { gamma = fmin(1.0, t / ddot(w, w)); beta = 1 - gamma; alpha = 0; }
-        else { alpha = dclamp01(-ddot(b, u) / ddot(u, u)); beta = 1 - alpha; gamma = 0; }
-        clamped = true;
-    } else if (gamma >= 0 && alpha < 0) {
-        d3 w = dsub(b, c);
-        double t = -ddot(c, v);
-        if (beta < 0 && t > 0) { alpha = fmin(1.0, t / ddot(v, v)); gamma = 1 - alpha; beta = 0; }
-        else { beta = dclamp01(-ddot(c, w) / ddot(w, w)); gamma = 1 - beta; alpha = 0; }
-        clamped = true;
-    }
-    out = d3{alpha, beta, gamma};
-    return clamped;
+// (x0 + x1) + x2 of up to four vectors at once: lane k of the group returns the sum of the
+// components of the k-th argument, in the order of the reference's dot products.
+__device__ __forceinline__ double grp_sums(int c, double p, double q, double r, double s) {
+    const double p0 = grp(p, 0), p1 = grp(p, 1), p2 = grp(p, 2);
+    const double q0 = grp(q, 0), q1 = grp(q, 1), q2 = grp(q, 2);
+    const double r0 = grp(r, 0), r1 = grp(r, 1), r2 = grp(r, 2);
+    const double s0 = grp(s, 0), s1 = grp(s, 1), s2 = grp(s, 2);
+    const double x0 = c == 0 ? p0 : (c == 1 ? q0 : (c == 2 ? r0 : s0));
+    const double x1 = c == 0 ? p1 : (c == 1 ? q1 : (c == 2 ? r1 : s1));
+    const double x2 = c == 0 ? p2 : (c == 1 ? q2 : (c == 2 ? r2 : s2));
+    return (x0 + x1) + x2;
 }
 
-// The FP64 geometry of a face (ConvexPolytope.CreateTriangle, ConvexPolytope.cs:267-318):
-// p0, p1, p2 are the corners in creation order; `swapped` when the orientation test
-// exchanged the first two.  The raw normal is the FP64 plane filter's cross product of the
-// creation order (PlaneFilter.cs:29-45), negated on a swap, and replaced by the exact
-// expansion normal of the final order when the filter calls it unreliable
-// (PlaneFilter.cs:24-27).  Returns false on a numerical failure.
-struct FaceGeo { d3 sn; double nscale, nsq; d3 bc, cl; double d2; };
-__device__ __noinline__ bool face_geo(v3 p0, v3 p1, v3 p2, bool swapped, FaceGeo& g, NpStats& st) {
+// The FP64 geometry of a face (ConvexPolytope.CreateTriangle, ConvexPolytope.cs:267-318, and
+// CalcBarycentric, :328-395) from its corners in creation order i0, i1, i2; `swapped` when the
+// orientation test exchanged the first two.  The raw normal is the FP64 plane filter's cross
+// product of the creation order (PlaneFilter.cs:29-45), negated on a swap, and replaced by the
+// exact expansion normal of the final order when the filter calls it unreliable
+// (PlaneFilter.cs:24-27).  sn, cl: this lane's component; bc: all three weights; ok is false on
+// a numerical failure.  Called by the whole warp; the coordinates are safe_coord's, so that no
+// value up to the quotients overflows.
+struct FaceGeo { double sn, cl, d2; double bx, by, bz; bool ok; };
+__device__ __noinline__ FaceGeo face_geo(const EpaSmem& E, int i0, int i1, int i2, bool swapped, bool count, NpStats& st) {
     const double EF = 16 * 1.1102230246251565e-16;
-    double ux = (double)p0.x - p1.x, uy = (double)p0.y - p1.y, uz = (double)p0.z - p1.z;
-    double vx = (double)p0.x - p2.x, vy = (double)p0.y - p2.y, vz = (double)p0.z - p2.z;
-    double yz = uy * vz, zy = uz * vy, zx = uz * vx, xz = ux * vz, xy = ux * vy, yx = uy * vx;
-    d3 raw{yz - zy, zx - xz, xy - yx};
-    double ex = EF * (fabs(yz) + fabs(zy)), ey = EF * (fabs(zx) + fabs(xz)), ez = EF * (fabs(xy) + fabs(yx));
-    if (swapped) raw = d3{-raw.x, -raw.y, -raw.z};
-    v3 a = swapped ? p1 : p0, b = swapped ? p0 : p1, c = p2;
-    if (!(fmax(fabs(raw.x), fmax(fabs(raw.y), fabs(raw.z))) > 1048576 * fmax(ex, fmax(ey, ez)))) {
-        st.exact++;
-        Exp::normal(a, b, c, raw.x, raw.y, raw.z);
+    const int c = threadIdx.x & 3, k = c == 3 ? 0 : c, k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
+    const double p0 = (double)(&E.vV[i0].x)[k], p1 = (double)(&E.vV[i1].x)[k], p2 = (double)(&E.vV[i2].x)[k];
+    FaceGeo g;
+    const double u = p0 - p1, v = p0 - p2;
+    double raw;
+    long long rmax, emax;
+    {
+        const double s = grp(u, k1) * grp(v, k2), t = grp(u, k2) * grp(v, k1);
+        raw = s - t;
+        const long long e = d_absbits(EF * (fabs(s) + fabs(t)));
+        if (swapped) raw = -raw;
+        const long long m = d_absbits(raw);
+        rmax = max(max(__shfl_sync(FULL, m, 0, 4), __shfl_sync(FULL, m, 1, 4)), __shfl_sync(FULL, m, 2, 4));
+        emax = max(max(__shfl_sync(FULL, e, 0, 4), __shfl_sync(FULL, e, 1, 4)), __shfl_sync(FULL, e, 2, 4));
     }
-    double ns = fmax(fabs(raw.x), fmax(fabs(raw.y), fabs(raw.z)));
-    if (!(ns > 0) || !isfinite(ns)) return false;
-    g.nscale = ns;
-    g.sn = d3{raw.x / ns, raw.y / ns, raw.z / ns};
-    g.nsq = ddot(g.sn, g.sn);
-    d3 va = dv(a), vb = dv(b), vc = dv(c);
-    bool clamped = calc_bary(va, vb, vc, g.sn, ns, g.nsq, g.bc);
-    g.cl = clamped ? dadd(dadd(dmul(va, g.bc.x), dmul(vb, g.bc.y)), dmul(vc, g.bc.z))
-                   : dmul(g.sn, ddot(g.sn, va) / g.nsq);
-    g.d2 = ddot(g.cl, g.cl);
-    return dfinite(g.cl) && dfinite(g.bc) && isfinite(g.d2);
+    const double a = swapped ? p1 : p0, b = swapped ? p0 : p1;
+    // unreliable unless the largest component exceeds 2^20 times the largest error bound
+    const bool exact = !(rmax > (emax ? emax + (20ll << 52) : 0));
+    if (__any_sync(FULL, exact)) {
+        double x = 0, y = 0, z = 0;
+        if (exact) {
+            if (count) st.exact++;
+            if (c == 0) {
+                const int ia = swapped ? i1 : i0, ib = swapped ? i0 : i1;
+                Exp::normal(mk3(E.vV[ia]), mk3(E.vV[ib]), mk3(E.vV[i2]), x, y, z);
+            }
+        }
+        __syncwarp();
+        x = grp(x, 0); y = grp(y, 0); z = grp(z, 0);
+        if (exact) {
+            raw = k == 0 ? x : (k == 1 ? y : z);
+            rmax = max(max(d_absbits(x), d_absbits(y)), d_absbits(z));
+        }
+    }
+    const double ns = __longlong_as_double(rmax);
+    g.ok = rmax > 0 && d_finite(ns);
+    const double sn = raw / ns;
+    g.sn = sn;
+    const double nn = sn * sn;
+    const double nsq = (grp(nn, 0) + grp(nn, 1)) + grp(nn, 2);
+    const double uf = a - b, vf = a - p2;  // of the final order
+    const double a1 = grp(a, k1), a2 = grp(a, k2), uf1 = grp(uf, k1), uf2 = grp(uf, k2), vf1 = grp(vf, k1), vf2 = grp(vf, k2);
+    // lane 0: gamma, lane 1: beta, lane 2: the plane's distance, each over nsq in one division
+    const double num = grp_sums(c, (uf1 * a2 - uf2 * a1) * sn, (a1 * vf2 - a2 * vf1) * sn, sn * a, 0.0);
+    const double q1 = num / nsq;
+    const double q2 = q1 / ns;
+    const double dq = grp(q1, 2);
+    double gamma = grp(q2, 0), beta = grp(q2, 1);
+    double alpha = 1.0 - gamma - beta;
+    g.cl = sn * dq;
+    const bool c1 = d_ge0(alpha) && d_lt0(beta), c2 = !c1 && d_ge0(beta) && d_lt0(gamma),
+               c3 = !c1 && !c2 && d_ge0(gamma) && d_lt0(alpha);
+    const bool clamped = c1 || c2 || c3;
+    if (__any_sync(FULL, clamped)) {
+        // the three cases differ in the corner P, the edge Q tried first and the edge R taken
+        // otherwise: (a, u, v), (b, w, u), (c, v, w)
+        const double w = b - p2;
+        const double P = c1 ? a : (c2 ? b : p2), Q = c1 ? uf : (c2 ? w : vf), R = c1 ? vf : (c2 ? uf : w);
+        const double s = grp_sums(c, P * Q, P * R, Q * Q, R * R);
+        double t = grp(s, 0), o = grp(s, 1);
+        if (c3) t = -t;
+        if (!c1) o = -o;
+        const bool first = d_lt0(c1 ? gamma : (c2 ? alpha : beta)) && !d_lt0(t) && x_nonzero(t);
+        const double qq = grp(s, 2), rr = grp(s, 3);
+        double r = (first ? t : o) / (first ? qq : rr);
+        if (first) r = fmin(1.0, r);
+        else r = d_lt0(r) ? 0.0 : (r > 1.0 ? 1.0 : r);
+        const double q = 1.0 - r;
+        if (clamped) {
+            if (c1) { alpha = q; beta = first ? r : 0.0; gamma = first ? 0.0 : r; }
+            else if (c2) { beta = q; gamma = first ? r : 0.0; alpha = first ? 0.0 : r; }
+            else { gamma = q; alpha = first ? r : 0.0; beta = first ? 0.0 : r; }
+            g.cl = (a * alpha + b * beta) + p2 * gamma;
+        }
+        __syncwarp();
+    }
+    const double cc = g.cl * g.cl;
+    g.d2 = (grp(cc, 0) + grp(cc, 1)) + grp(cc, 2);
+    g.bx = alpha; g.by = beta; g.bz = gamma;
+    g.ok = g.ok && d_finite(g.cl) && d_finite(alpha) && d_finite(beta) && d_finite(gamma) && d_finite(g.d2);
+    const unsigned bad = __ballot_sync(FULL, !g.ok);
+    g.ok = ((bad >> (threadIdx.x & 28)) & 15u) == 0;
+    return g;
 }
 
-// The face's geometry from its stored corners and flags.
-__device__ __forceinline__ bool face_geo_of(const EpaSmem& E, int f, FaceGeo& g, NpStats& st) {
+// The geometry of a stored face, by every group of the warp alike.
+__device__ __forceinline__ FaceGeo face_geo_of(const EpaSmem& E, int f, NpStats& st) {
     uchar4 t = E.fi[f];
     bool sw = (t.w & EPA_SWAPPED) != 0;
-    int p0 = sw ? t.y : t.x, p1 = sw ? t.x : t.y;
-    return face_geo(mk3(E.vV[p0]), mk3(E.vV[p1]), mk3(E.vV[t.z]), sw, g, st);
+    return face_geo(E, sw ? t.y : t.x, sw ? t.x : t.y, t.z, sw, true, st);
 }
 
 // The FP32 normal of a face and its squared length (Triangle.Normal / NormalSq).
 __device__ __forceinline__ float4 face_normal32(const FaceGeo& g) {
-    v3 n = mk3((float)g.sn.x, (float)g.sn.y, (float)g.sn.z);
+    const float s = (float)g.sn;
+    v3 n = mk3(__shfl_sync(FULL, s, 0), __shfl_sync(FULL, s, 1), __shfl_sync(FULL, s, 2));
     return f4(n, len2(n));
 }
 
-// ConvexPolytope.CreateTriangle (ConvexPolytope.cs:267-318), one lane per face.
-__device__ __noinline__ int create_tri(EpaSmem& E, int a, int b, int c, int slot, NpStats& st) {
+// ConvexPolytope.CreateTriangle (ConvexPolytope.cs:267-318), four lanes per face, eight faces
+// per call; `live` is false for the groups beyond the last face (they repeat another face's
+// arithmetic and store nothing).  Called by the whole warp.
+__device__ __noinline__ int create_tris(EpaSmem& E, int a, int b, int c, int slot, bool live, NpStats& st) {
+    const int comp = threadIdx.x & 3;
+    NpStats mine;
+    mine.exact = 0;
     v3 va = mk3(E.vV[a]), vb = mk3(E.vV[b]), vc = mk3(E.vV[c]);
-    v3 p0 = va, p1 = vb;
+    const int i0 = a, i1 = b;
     int orient = 0;
     for (int i = 0; i < 4 && orient == 0; i++) {
         if (i == a || i == b || i == c) continue;
-        orient = -side_pt(va, vb, vc, mk3(E.vV[i]), st);
+        orient = -side_pt(va, vb, vc, mk3(E.vV[i]), mine);
     }
-    if (orient == 0) return DEGENERATE;
     const bool swapped = orient < 0;
     if (swapped) { int t = a; a = b; b = t; v3 tv = va; va = vb; vb = tv; }
-    bool facing = side_pt(va, vb, vc, mk3(0.f), st) <= 0;
-    FaceGeo g;
-    if (!face_geo(p0, p1, vc, swapped, g, st)) return NUMERICAL;
-    v3 cl = mk3((float)g.cl.x, (float)g.cl.y, (float)g.cl.z);
-    float d2 = (float)g.d2;
-    if (!isfinite(cl.x) || !isfinite(cl.y) || !isfinite(cl.z) || !isfinite(d2)) return NUMERICAL;
-    E.fi[slot] = make_uchar4((unsigned char)a, (unsigned char)b, (unsigned char)c,
-                             (unsigned char)((facing ? EPA_FACING : 0) | (swapped ? EPA_SWAPPED : 0)));
-    E.fd[slot] = g.d2;
-    E.fc[slot] = f4(cl, d2);
-    return ADDED;
+    bool facing = orient != 0 && side_pt(va, vb, vc, mk3(0.f), mine) <= 0;
+    __syncwarp();
+    const bool counts = live && comp == 0;  // one lane counts for its face
+    if (counts) st.exact += mine.exact;
+    const FaceGeo g = face_geo(E, i0, i1, c, swapped, counts && orient != 0, st);
+    const float out = (float)(comp == 3 ? g.d2 : g.cl);
+    const unsigned bad = __ballot_sync(FULL, !isfinite(out));
+    int r = ADDED;
+    if (orient == 0) r = DEGENERATE;
+    else if (!g.ok || ((bad >> (threadIdx.x & 28)) & 15u)) r = NUMERICAL;
+    if (live && r == ADDED) {
+        (&E.fc[slot].x)[comp] = out;
+        if (comp == 0) {
+            E.fi[slot] = make_uchar4((unsigned char)a, (unsigned char)b, (unsigned char)c,
+                                     (unsigned char)((facing ? EPA_FACING : 0) | (swapped ? EPA_SWAPPED : 0)));
+            E.fd[slot] = g.d2;
+        }
+    }
+    return live ? r : ADDED;
 }
 
 // ConvexPolytope.InitTetrahedron (ConvexPolytope.cs:113-132)
@@ -328,8 +391,8 @@ __device__ bool epa_init(EpaSmem& E, NpStats& st) {
     for (int i = 0; i < 4; i++) safe = safe && is_safe(mk3(E.vV[i]));
     if (!safe) return false;
     const int idx[12] = {0, 2, 1, 0, 1, 3, 0, 3, 2, 1, 2, 3};
-    int r = ADDED;
-    if (lane < 4) r = create_tri(E, idx[3 * lane], idx[3 * lane + 1], idx[3 * lane + 2], lane, st);
+    const int f = min(lane >> 2, 3);
+    int r = create_tris(E, idx[3 * f], idx[3 * f + 1], idx[3 * f + 2], f, lane < 16, st);
     bool ok = __all_sync(FULL, r == ADDED);
     __syncwarp();
     if (ok && lane == 0) E.nt = 4;
@@ -341,20 +404,19 @@ __device__ bool epa_init(EpaSmem& E, NpStats& st) {
 // distance, the first such face on a tie.
 __device__ int epa_closest(EpaSmem& E) {
     const int lane = threadIdx.x & 31;
-    double best = CUDART_INF;
+    // squared distances are finite and not negative: they order as their bit patterns
+    unsigned long long best = ~0ull;
     int bi = 0x7fffffff;
     bool notfacing = false;
     int nt = E.nt;
     for (int i = lane; i < nt; i += 32) {
-        double d = E.fd[i];
+        const unsigned long long d = (unsigned long long)__double_as_longlong(E.fd[i]);
         if (d < best) { best = d; bi = i; }
         if (!(E.fi[i].w & EPA_FACING)) notfacing = true;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        double ob = __shfl_xor_sync(FULL, best, off);
-        int oi = __shfl_xor_sync(FULL, bi, off);
-        if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
+    const unsigned hi = __reduce_min_sync(FULL, (unsigned)(best >> 32));
+    const unsigned lo = __reduce_min_sync(FULL, (unsigned)(best >> 32) == hi ? (unsigned)best : 0xffffffffu);
+    bi = (int)__reduce_min_sync(FULL, best == (((unsigned long long)hi << 32) | lo) ? (unsigned)bi : 0x7fffffffu);
     bool any_nf = __any_sync(FULL, notfacing);
     bool skip = E.enclosed != 0;
     __syncwarp();
@@ -385,31 +447,60 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
         if (lane == 0) E.lit[base >> 5] = m;
     }
     __syncwarp();
-    // horizon edges in the reference's order (faces from last to first), one lane
-    if (lane == 0) {
-        int ne = 0;
-        for (int index = nt; index-- > 0;) {
-            if (!((E.lit[index >> 5] >> (index & 31)) & 1u)) continue;
-            uchar4 f = E.fi[index];
-            unsigned char cs[3] = {f.x, f.y, f.z};
+    // Horizon edges in the reference's order (faces from last to first; an edge met twice
+    // leaves the list, the last edge taking its place).  The list lives in registers, edge e in
+    // lane e, so that a search is one vote; a list that outgrows the warp is rebuilt by one lane
+    // in shared memory.
+    int ne = 0, edge = 0;
+    bool wide = false;
+    for (int word = (nt - 1) >> 5; word >= 0 && !wide; word--) {
+        for (unsigned m = E.lit[word]; m && !wide;) {
+            const int bit = 31 - __clz(m);
+            m ^= 1u << bit;
+            const uchar4 f = E.fi[word * 32 + bit];
+            const int cs[4] = {f.x, f.y, f.z, f.x};
+#pragma unroll
             for (int k = 0; k < 3; k++) {
-                unsigned char A = cs[k], B = cs[(k + 1) % 3];
-                bool added = true;
-                for (int e = ne; e-- > 0;) {
-                    bool match = (E.ea[e] == A && E.eb[e] == B) || (E.ea[e] == B && E.eb[e] == A);
-                    if (!match) continue;
+                const int key = cs[k] | (cs[k + 1] << 8), rev = cs[k + 1] | (cs[k] << 8);
+                const unsigned hit = __ballot_sync(FULL, lane < ne && (edge == key || edge == rev));
+                if (hit) {
                     --ne;
-                    E.ea[e] = E.ea[ne]; E.eb[e] = E.eb[ne];
-                    added = false;
-                    break;
+                    const int last = __shfl_sync(FULL, edge, ne);
+                    if (lane == 31 - __clz(hit)) edge = last;
+                } else {
+                    if (ne == 32) { wide = true; break; }
+                    if (lane == ne) edge = key;
+                    ne++;
                 }
-                if (added && ne < 3 * JG_EPA_MAXT) { E.ea[ne] = A; E.eb[ne] = B; ne++; }
             }
         }
-        E.ne = ne;
     }
-    __syncwarp();
-    int ne = E.ne;
+    if (wide) {
+        if (lane == 0) {
+            int n = 0;
+            for (int index = nt; index-- > 0;) {
+                if (!((E.lit[index >> 5] >> (index & 31)) & 1u)) continue;
+                uchar4 f = E.fi[index];
+                unsigned char cs[3] = {f.x, f.y, f.z};
+                for (int k = 0; k < 3; k++) {
+                    unsigned char A = cs[k], B = cs[(k + 1) % 3];
+                    bool added = true;
+                    for (int e = n; e-- > 0;) {
+                        bool match = (E.ea[e] == A && E.eb[e] == B) || (E.ea[e] == B && E.eb[e] == A);
+                        if (!match) continue;
+                        --n;
+                        E.ea[e] = E.ea[n]; E.eb[e] = E.eb[n];
+                        added = false;
+                        break;
+                    }
+                    if (added && n < 3 * JG_EPA_MAXT) { E.ea[n] = A; E.eb[n] = B; n++; }
+                }
+            }
+            E.ne = n;
+        }
+        __syncwarp();
+        ne = E.ne;
+    }
     if (ne == 0) return NO_HORIZON;
     int nlit = 0;
     for (int k = 0; k < (nt + 31) / 32; k++) nlit += __popc(E.lit[k] & (k * 32 + 32 <= nt ? 0xffffffffu : ((1u << (nt & 31)) - 1u)));
@@ -428,17 +519,16 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
         surv += __popc(m);
         __syncwarp();
     }
-    // the new fan, one face per lane
+    // the new fan, eight faces at a time
     int res = ADDED;
-    for (int base = 0; base < ne; base += 32) {
-        int e = base + lane;
-        int r = ADDED;
-        if (e < ne) r = create_tri(E, E.ea[e], E.eb[e], nv, surv + e, st);
-        for (int off = 16; off > 0; off >>= 1) {
-            int o = __shfl_xor_sync(FULL, r, off);
-            if (o != ADDED && (r == ADDED || o < r)) r = o;
-        }
-        if (r != ADDED && res == ADDED) res = r;
+    for (int base = 0; base < ne; base += 8) {
+        const int e = min(base + (lane >> 2), ne - 1);
+        int ea, eb;
+        if (wide) { ea = E.ea[e]; eb = E.eb[e]; }
+        else { const int k = __shfl_sync(FULL, edge, e); ea = k & 255; eb = k >> 8; }
+        const int r = create_tris(E, ea, eb, nv, surv + e, base + (lane >> 2) < ne, st);
+        const unsigned worst = __reduce_min_sync(FULL, r == ADDED ? 0x7fffffffu : (unsigned)r);
+        if (worst != 0x7fffffffu && res == ADDED) res = (int)worst;
     }
     __syncwarp();
     if (res != ADDED) {
@@ -467,9 +557,7 @@ __device__ __noinline__ bool solve_epa(EpaSmem& E, const ShapeRef& sa, const Sha
         if (!E.enclosed) sd = -sd;
         if (fc.w < 1e-16f) {
             // search along the face normal (Triangle.Normal / NormalSq)
-            FaceGeo g;
-            face_geo_of(E, ci, g, st);
-            float4 fn = face_normal32(g);
+            const float4 fn = face_normal32(face_geo_of(E, ci, st));
             sd = mk3(fn); sdsq = fn.w;
         }
         MV v;
@@ -489,12 +577,13 @@ converged:
         // ConvexPolytope.CalculatePoints (ConvexPolytope.cs:169-185): the FP64 barycentric
         // combination of the corners' support points, rounded to FP32
         uchar4 f = E.fi[ci];
-        FaceGeo g;
-        face_geo_of(E, ci, g, st);
-        d3 a = dadd(dadd(dmul(dv(mk3(E.vA[f.x])), g.bc.x), dmul(dv(mk3(E.vA[f.y])), g.bc.y)), dmul(dv(mk3(E.vA[f.z])), g.bc.z));
-        d3 b = dadd(dadd(dmul(dv(mk3(E.vB[f.x])), g.bc.x), dmul(dv(mk3(E.vB[f.y])), g.bc.y)), dmul(dv(mk3(E.vB[f.z])), g.bc.z));
-        p1 = mk3((float)a.x, (float)a.y, (float)a.z);
-        p2 = mk3((float)b.x, (float)b.y, (float)b.z);
+        const FaceGeo g = face_geo_of(E, ci, st);
+        // lanes 0-2: the components of A's point, lanes 4-6: of B's
+        const int lane = threadIdx.x & 31, k = (lane & 3) == 3 ? 0 : lane & 3;
+        const float4* P = (lane & 4) ? E.vB : E.vA;
+        const float pt = (float)(((double)(&P[f.x].x)[k] * g.bx + (double)(&P[f.y].x)[k] * g.by) + (double)(&P[f.z].x)[k] * g.bz);
+        p1 = mk3(__shfl_sync(FULL, pt, 0), __shfl_sync(FULL, pt, 1), __shfl_sync(FULL, pt, 2));
+        p2 = mk3(__shfl_sync(FULL, pt, 4), __shfl_sync(FULL, pt, 5), __shfl_sync(FULL, pt, 6));
         float4 fn = face_normal32(g);
         n = mk3(fn) * (1.0f / sqrtf(fn.w));
         pen = sqrtf(E.fc[ci].w);

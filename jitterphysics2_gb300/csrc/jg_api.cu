@@ -17,6 +17,7 @@ void jg_flip_store(WorldDev& w);
 void jg_launch_count_contacts(WorldDev& w, cudaStream_t s, int nsm);
 void jg_launch_update_contacts(WorldDev& w, cudaStream_t s, int nsm);
 void jg_solver_reset_launch_cache(WorldDev& w);
+void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
 int jg_solver_init();
 int jg_schedule_init();
 void jg_launch_activate(WorldDev& w, int body, cudaStream_t s);
@@ -159,6 +160,10 @@ int allocate(jg_world* w) {
     DA(d.sc_task, JG_SCHED_MAXTASKS); DA(d.sc_cursor, JG_SCHED_MAXTASKS); DA(d.sc_tnc, JG_SCHED_MAXTASKS);
     DA(d.sc_tcell, JG_SCHED_MAXTASKS); DA(d.sc_tdep, 2 * JG_SCHED_MAXTASKS); DA(d.sc_done, JG_SCHED_MAXTASKS);
     DA(d.sc_tcol, (size_t)JG_SCHED_MAXTASKS * (JG_TASK_MAXC + 1));
+    DA(d.gr, 1); DA(d.gr_root, d.cap_bodies); DA(d.gr_slot, d.cap_bodies);
+    DA(d.gr_narb, d.cap_bodies); DA(d.gr_njoint, d.cap_bodies); DA(d.gr_nbody, d.cap_bodies); DA(d.gr_ncon, d.cap_bodies);
+    DA(d.gr_pos, d.cap_arb + d.cap_joints); DA(d.gr_part, d.cap_bodies); DA(d.gr_rec, JG_GROUP_CLASSES * (size_t)d.cap_bodies);
+    DA(d.gr_arb, d.cap_arb); DA(d.gr_joint, d.cap_joints); DA(d.gr_body, d.cap_bodies);
     DA(d.ev_created, d.cap_arb); DA(d.ev_removed, d.cap_arb); DA(d.remaining, 2); DA(d.dst_index, d.cap_arb);
     CK(cudaMallocHost((void**)&w->h_ctr, sizeof(DevCounters)));
     memset(w->h_ctr, 0, sizeof(DevCounters));
@@ -248,6 +253,9 @@ StepParams make_params(const jg_world* w, float dt) {
     if (sp.task_maxb < 64) sp.partition = 0;  // a block too large for a useful task
     sp.cells_per_sm = p.sched_cells_per_sm;  // 0: chosen on the device (cell count and arbiter count)
     sp.solve_blocks = w->nsm * (p.solver_ctas_per_sm > 0 ? p.solver_ctas_per_sm : JG_TASK_CTAS);
+    // groups are keyed by body or world; the recording of residuals and training targets
+    // belongs to the task solve
+    sp.groups = sp.partition && !p.record_residual && !w->d.rec_on && w->d.nworlds <= w->d.cap_bodies ? 1 : 0;
     return sp;
 }
 
@@ -283,6 +291,11 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     jg_flip_store(d);
     if (timed) cudaEventRecord(w->ev[4], s);
     jg_launch_count_contacts(d, s, w->nsm);
+    if (sp.groups) {
+        jg_launch_groups(d, s, w->nsm);
+        jg_launch_solve_groups(d, sp, s, w->nsm);
+        w->launches += jg_group_launches(d) + JG_GROUP_CLASSES;
+    }
     if (jg_launch_solve(d, sp, s, w->nsm, w->prm.solver_block, w->prm.solver_ctas_per_sm) < 0) {
         g_err = "cooperative launch of the solver failed";
         return JG_ERR_CUDA;
@@ -958,6 +971,7 @@ int jg_stabilize(jg_world* w, float dt, int32_t iterations, int32_t relax) {
     sp.iterations = iterations;
     sp.relax = relax;
     sp.stabilize = 1;
+    sp.groups = 0;
     sp.record_residual = 0;
     WorldDev& d = w->d;
     cudaStream_t s = w->stream;

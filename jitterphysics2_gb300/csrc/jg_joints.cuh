@@ -7,7 +7,8 @@
 // (LinearServo.cs:149-201), LinearAxisServo (LinearAxisServo.cs:169-224) and TwistServo
 // (TwistServo.cs:150-192), PointOnLine (PointOnLine.cs:149-465) and EllipticalConeLimit
 // (EllipticalConeLimit.cs:257-429).  Included by the solver translation unit.  Matrices are
-// row-major float[3][3].
+// row-major float[3][3].  W is the world, or the view of one solve group (bodies in shared
+// memory under local indices).
 //
 // JointDev fields of the one-row kinds: la1/la2 anchors (DistanceLimit) or local axes
 // (ConeLimit); axis / q0 the twist axis and reference rotation (TwistAngle); lim = (min, max,
@@ -15,6 +16,9 @@
 // impulse, bias.x the bias, bil.x the effective mass, bil.w the hemisphere (TwistAngle);
 // Jacobian blocks in eff[0..2] and jac[0] (the ConeLimit block persists between steps).
 #pragma once
+
+__device__ __forceinline__ int joint_b1(const WorldDev&, const JointDev& J) { return J.hdr.y; }
+__device__ __forceinline__ int joint_b2(const WorldDev&, const JointDev& J) { return J.hdr.z; }
 
 struct M3x { float a[3][3]; };
 __device__ __forceinline__ M3x mzero() { M3x m; for (int i = 0; i < 3; i++) for (int j = 0; j < 3; j++) m.a[i][j] = 0.f; return m; }
@@ -177,8 +181,9 @@ __device__ __forceinline__ M3x sym_transform_full(const sym6& S, const M3x& T) {
 }
 
 // BallSocket.PrepareForIterationBallSocket (BallSocket.cs:140-183)
-__device__ void ballsocket_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void ballsocket_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     v3 r1 = rotate(mk3(J.la1), q1), r2 = rotate(mk3(J.la2), q2);
@@ -211,8 +216,9 @@ __device__ void ballsocket_prepare(const WorldDev& w, JointDev& J, const StepPar
     jstore_m(J.eff, eff);
 }
 // BallSocket.IterateBallSocket (BallSocket.cs:223-252)
-__device__ void ballsocket_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void ballsocket_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     M3x cr1 = mskew(mk3(J.r1)), cr2 = mskew(mk3(J.r2));
     v3 acc = mk3(J.acc);
@@ -264,8 +270,9 @@ __device__ M3x calc_jacobian(q4 left, q4 right, v3& err, int& hemi) {
 }
 
 // HingeAngle.PrepareForIterationHingeAngle (HingeAngle.cs:133-220)
-__device__ void hinge_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void hinge_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     v3 axis = mk3(J.axis);
@@ -344,8 +351,9 @@ __device__ void hinge_prepare(const WorldDev& w, JointDev& J, const StepParams& 
     J.cpl = make_float4(cx, cy, 0.f, 0.f);
 }
 // HingeAngle.IterateHingeAngle (HingeAngle.cs:313-364)
-__device__ void hinge_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void hinge_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     M3x jac = jload_m(J.jac), eff = jload_m(J.eff);
     v3 jv = mtv(jac, b1.w - b2.w);
@@ -395,8 +403,9 @@ __device__ __forceinline__ sym6 sym_add(const sym6& a, const sym6& b) {
 
 // DistanceLimit.PrepareForIterationDistanceLimit (DistanceLimit.cs:227-306): the distance
 // between the anchors against [distance + min, distance + max]
-__device__ void distance_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void distance_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 r1 = rotate(mk3(J.la1), mkq(w.q[i1])), r2 = rotate(mk3(J.la2), mkq(w.q[i2]));
     v3 dp = (mk3(w.pos[i2]) + r2) - (mk3(w.pos[i1]) + r1);
@@ -431,10 +440,11 @@ __device__ void distance_prepare(const WorldDev& w, JointDev& J, const StepParam
     }
 }
 // DistanceLimit.IterateDistanceLimit (DistanceLimit.cs:344-391)
-__device__ void distance_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
+template <class W>
+__device__ void distance_iterate(const W& w, JointDev& J, const StepParams& sp) {
     const int clamp = (int)J.lim.w;
     if (clamp == 0) return;
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 j0 = mk3(J.eff[0]), j1 = mk3(J.eff[1]), j2 = mk3(J.eff[2]), j3 = mk3(J.jac[0]);
     float jv = dot(b1.v, j0) + dot(b1.w, j1) + dot(b2.v, j2) + dot(b2.w, j3);
@@ -458,8 +468,9 @@ __device__ void distance_iterate(const WorldDev& w, JointDev& J, const StepParam
 // ConeLimit.PrepareForIterationConeLimit (ConeLimit.cs:262-356): the angle between the
 // bodies' axes against [min, max]; the Jacobian row persists, and its sign flip drops the
 // cached impulse
-__device__ void cone_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void cone_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 a1 = rotate(mk3(J.la1), mkq(w.q[i1])), a2 = rotate(mk3(J.la2), mkq(w.q[i2]));
     v3 prev = mk3(J.eff[0]);
@@ -499,10 +510,11 @@ __device__ void cone_prepare(const WorldDev& w, JointDev& J, const StepParams& s
     if (b2.flags & SB_DYNAMIC) { b2.w = b2.w + sym_mul(b2.I, acc * j1); store_vel(w.body, i2, b2); }
 }
 // ConeLimit.IterateConeLimit (ConeLimit.cs:378-404)
-__device__ void cone_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
+template <class W>
+__device__ void cone_iterate(const W& w, JointDev& J, const StepParams& sp) {
     const int clamp = (int)J.lim.w;
     if (clamp == 0) return;
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 j0 = mk3(J.eff[0]), j1 = mk3(J.eff[1]);
     float jv = dot(b1.w, j0) + dot(b2.w, j1);
@@ -551,8 +563,9 @@ __device__ float calc_twist(q4 left, q4 right, v3 axis, v3& jac, int& hemi) {
     return 2.0f * StableMathF::atan2(proj, cosine);
 }
 // TwistAngle.PrepareForIterationTwistAngle (TwistAngle.cs:170-233)
-__device__ void twist_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void twist_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     v3 jr;
@@ -590,10 +603,11 @@ __device__ void twist_prepare(const WorldDev& w, JointDev& J, const StepParams& 
     if (b2.flags & SB_DYNAMIC) { b2.w = b2.w - sym_mul(b2.I, acc * jr); store_vel(w.body, i2, b2); }
 }
 // TwistAngle.IterateTwistAngle (TwistAngle.cs:296-323)
-__device__ void twist_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
+template <class W>
+__device__ void twist_iterate(const W& w, JointDev& J, const StepParams& sp) {
     const int clamp = (int)J.lim.w;
     if (clamp == 0) return;
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 jr = mk3(J.eff[0]);
     float jv = dot(b1.w - b2.w, jr);
@@ -610,8 +624,9 @@ __device__ void twist_iterate(const WorldDev& w, JointDev& J, const StepParams& 
 // FixedAngle.PrepareForIterationFixedAngle (FixedAngle.cs:87-128): three angular rows, the
 // Jacobian -2 x the rotation-log derivative of Q0 conj(q1) q2 (q0), softness prm.y, bias
 // factor prm.x; Jacobian in jac[0..2], inverse effective mass in eff[0..2], hemisphere bil.w
-__device__ void fixed_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void fixed_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 err;
     int hemi;
@@ -636,8 +651,9 @@ __device__ void fixed_prepare(const WorldDev& w, JointDev& J, const StepParams& 
     J.bil = make_float4(0.f, 0.f, 0.f, (float)hemi);
 }
 // FixedAngle.IterateFixedAngle (FixedAngle.cs:159-181)
-__device__ void fixed_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void fixed_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     M3x jac = jload_m(J.jac), eff = jload_m(J.eff);
     v3 jv = mv(jac, b1.w - b2.w);
@@ -653,8 +669,9 @@ __device__ void fixed_iterate(const WorldDev& w, JointDev& J, const StepParams& 
 // PointOnPlane.PrepareForIterationPointOnPlane (PointOnPlane.cs:128-200): one row along the
 // plane normal (axis, local to body 1), the arm of body 1 measured to the second anchor; the
 // same row layout and iteration as DistanceLimit (PointOnPlane.cs:218-256)
-__device__ void plane_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void plane_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     v3 axis = rotate(mk3(J.axis), q1);
@@ -699,9 +716,10 @@ __device__ __forceinline__ void motor_push(LBody& b, v3 imp, bool linear) {
     if (linear) b.v = b.v + cmul(imp, b.im);
     else b.w = b.w + sym_mul(b.I, imp);
 }
-__device__ void motor_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
+template <class W>
+__device__ void motor_prepare(const W& w, JointDev& J, const StepParams& sp) {
     const bool lin = J.hdr.x == JG_CONSTRAINT_LINEARMOTOR;
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 j1 = rotate(mk3(J.la1), mkq(w.q[i1])), j2 = rotate(mk3(J.la2), mkq(w.q[i2]));
     float m = motor_response(b1, j1, lin) + motor_response(b2, j2, lin);
@@ -714,9 +732,10 @@ __device__ void motor_prepare(const WorldDev& w, JointDev& J, const StepParams& 
     if (b1.flags & SB_DYNAMIC) { motor_push(b1, -(j1 * a), lin); store_vel(w.body, i1, b1); }
     if (b2.flags & SB_DYNAMIC) { motor_push(b2, j2 * a, lin); store_vel(w.body, i2, b2); }
 }
-__device__ void motor_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
+template <class W>
+__device__ void motor_iterate(const W& w, JointDev& J, const StepParams& sp) {
     const bool lin = J.hdr.x == JG_CONSTRAINT_LINEARMOTOR;
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 j1 = mk3(J.eff[0]), j2 = mk3(J.eff[1]);
     float jv = lin ? dot(-j1, b1.v) + dot(j2, b2.v) : dot(-j1, b1.w) + dot(j2, b2.w);
@@ -749,8 +768,9 @@ __device__ __forceinline__ v3 servo_clamp_angular(v3 imp, const M3x& jac, float 
 // AngularServo (AngularServo.cs:125-172): three angular rows towards the target relative
 // orientation q0; Jacobian in jac[0..2], inverse effective mass in eff[0..2], maximum torque
 // lim.y, hemisphere bil.w
-__device__ void angular_servo_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void angular_servo_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 err;
     int hemi;
@@ -775,8 +795,9 @@ __device__ void angular_servo_prepare(const WorldDev& w, JointDev& J, const Step
     jstore_m(J.jac, jac);
     J.bil = make_float4(0.f, 0.f, 0.f, (float)hemi);
 }
-__device__ void angular_servo_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void angular_servo_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     M3x jac = jload_m(J.jac), eff = jload_m(J.eff);
     v3 jv = mv(jac, b1.w - b2.w);
@@ -793,21 +814,23 @@ __device__ void angular_servo_iterate(const WorldDev& w, JointDev& J, const Step
 // LinearServo (LinearServo.cs:149-201): three linear rows pulling anchor 2 to anchor 1 offset
 // by the target (axis, body 1's frame); arms in r1, r2, inverse effective mass in eff[0..2],
 // maximum force lim.y
-__device__ __forceinline__ void linear_servo_apply(const WorldDev& w, const JointDev& J, LBody& b1, LBody& b2, v3 r1,
+template <class W>
+__device__ __forceinline__ void linear_servo_apply(const W& w, const JointDev& J, LBody& b1, LBody& b2, v3 r1,
                                                    v3 r2, v3 imp) {
     if (b1.flags & SB_DYNAMIC) {
         b1.v = b1.v - cmul(imp, b1.im);
         b1.w = b1.w - sym_mul(b1.I, cross(r1, imp));
-        store_vel(w.body, J.hdr.y, b1);
+        store_vel(w.body, joint_b1(w, J), b1);
     }
     if (b2.flags & SB_DYNAMIC) {
         b2.v = b2.v + cmul(imp, b2.im);
         b2.w = b2.w + sym_mul(b2.I, cross(r2, imp));
-        store_vel(w.body, J.hdr.z, b2);
+        store_vel(w.body, joint_b2(w, J), b2);
     }
 }
-__device__ void linear_servo_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void linear_servo_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     v3 r1 = rotate(mk3(J.la1) + mk3(J.axis), q1), r2 = rotate(mk3(J.la2), q2);
@@ -829,8 +852,9 @@ __device__ void linear_servo_prepare(const WorldDev& w, JointDev& J, const StepP
     J.acc = f4(acc, 0.f);
     J.bias = f4(bias, 0.f);
 }
-__device__ void linear_servo_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void linear_servo_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 r1 = mk3(J.r1), r2 = mk3(J.r2);
     v3 jv = ((-b1.v - cross(b1.w, r1)) + b2.v) + cross(b2.w, r2);
@@ -845,20 +869,22 @@ __device__ void linear_servo_iterate(const WorldDev& w, JointDev& J, const StepP
 // LinearAxisServo (LinearAxisServo.cs:169-224): one row along an axis of body 1 (axis, local),
 // target position lim.z, maximum force lim.y; Jacobian blocks in eff[0..2] and jac[0], the
 // effective mass in bil.x
-__device__ __forceinline__ void axis_servo_apply(const WorldDev& w, const JointDev& J, LBody& b1, LBody& b2, float a) {
+template <class W>
+__device__ __forceinline__ void axis_servo_apply(const W& w, const JointDev& J, LBody& b1, LBody& b2, float a) {
     if (b1.flags & SB_DYNAMIC) {
         b1.v = b1.v + cmul(mk3(J.eff[0]) * a, b1.im);
         b1.w = b1.w + sym_mul(b1.I, mk3(J.eff[1]) * a);
-        store_vel(w.body, J.hdr.y, b1);
+        store_vel(w.body, joint_b1(w, J), b1);
     }
     if (b2.flags & SB_DYNAMIC) {
         b2.v = b2.v + cmul(mk3(J.eff[2]) * a, b2.im);
         b2.w = b2.w + sym_mul(b2.I, mk3(J.jac[0]) * a);
-        store_vel(w.body, J.hdr.z, b2);
+        store_vel(w.body, joint_b2(w, J), b2);
     }
 }
-__device__ void linear_axis_servo_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void linear_axis_servo_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     v3 axis = rotate(mk3(J.axis), q1);
@@ -877,8 +903,9 @@ __device__ void linear_axis_servo_prepare(const WorldDev& w, JointDev& J, const 
     J.acc.x = acc;
     axis_servo_apply(w, J, b1, b2, acc);
 }
-__device__ void linear_axis_servo_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void linear_axis_servo_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     float jv = dot(mk3(J.eff[0]), b1.v) + dot(mk3(J.eff[1]), b1.w) + dot(mk3(J.eff[2]), b2.v) + dot(mk3(J.jac[0]), b2.w);
     float lambda = -(jv + J.bias.x + J.acc.x * J.prm.y * sp.inv_sub_dt) * J.bil.x;
@@ -890,13 +917,15 @@ __device__ void linear_axis_servo_iterate(const WorldDev& w, JointDev& J, const 
 // TwistServo (TwistServo.cs:150-192): the twist about body 2's axis (axis, local) towards the
 // target angle lim.z, reference rotation q0, maximum torque lim.y; Jacobian row jac[0],
 // effective mass bil.x, hemisphere bil.w
-__device__ __forceinline__ void twist_servo_apply(const WorldDev& w, const JointDev& J, LBody& b1, LBody& b2, float a) {
+template <class W>
+__device__ __forceinline__ void twist_servo_apply(const W& w, const JointDev& J, LBody& b1, LBody& b2, float a) {
     const v3 jr = mk3(J.jac[0]);
-    if (b1.flags & SB_DYNAMIC) { b1.w = b1.w + sym_mul(b1.I, jr * a); store_vel(w.body, J.hdr.y, b1); }
-    if (b2.flags & SB_DYNAMIC) { b2.w = b2.w - sym_mul(b2.I, jr * a); store_vel(w.body, J.hdr.z, b2); }
+    if (b1.flags & SB_DYNAMIC) { b1.w = b1.w + sym_mul(b1.I, jr * a); store_vel(w.body, joint_b1(w, J), b1); }
+    if (b2.flags & SB_DYNAMIC) { b2.w = b2.w - sym_mul(b2.I, jr * a); store_vel(w.body, joint_b2(w, J), b2); }
 }
-__device__ void twist_servo_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void twist_servo_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     v3 jr;
     int hemi;
@@ -916,8 +945,9 @@ __device__ void twist_servo_prepare(const WorldDev& w, JointDev& J, const StepPa
     J.acc.x = acc;
     twist_servo_apply(w, J, b1, b2, acc);
 }
-__device__ void twist_servo_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void twist_servo_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     float jv = dot(b1.w - b2.w, mk3(J.jac[0]));
     float lambda = -J.bil.x * (jv + J.bias.x + J.acc.x * J.prm.y * sp.inv_sub_dt);
@@ -940,8 +970,9 @@ __device__ __forceinline__ float net_max(float a, float b) {
 // The twelve Jacobian blocks (two rows across the line and one along it, each for v1, w1,
 // v2, w2) and the error, from the current poses (PointOnLine.cs:155-185, :378-408); the line's
 // direction (axis) and anchors (la1, la2) are local
-__device__ __forceinline__ v3 line_jacobian(const WorldDev& w, const JointDev& J, v3* jb) {
-    const int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ __forceinline__ v3 line_jacobian(const W& w, const JointDev& J, v3* jb) {
+    const int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     const q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     const v3 aw = rotate(mk3(J.axis), q1);
     const v3 n1 = rotate(create_orthonormal(mk3(J.axis)), q1);
@@ -954,22 +985,24 @@ __device__ __forceinline__ v3 line_jacobian(const WorldDev& w, const JointDev& J
     jb[8] = -aw; jb[9] = -cross(r1 + u, aw); jb[10] = aw; jb[11] = cross(r2, aw);
     return mk3(dot(u, n1), dot(u, n2), dot(u, aw));
 }
-__device__ __forceinline__ void line_apply(const WorldDev& w, const JointDev& J, LBody& b1, LBody& b2, const v3* jb, v3 a) {
+template <class W>
+__device__ __forceinline__ void line_apply(const W& w, const JointDev& J, LBody& b1, LBody& b2, const v3* jb, v3 a) {
     if (b1.flags & SB_DYNAMIC) {
         b1.v = b1.v + cmul(jb[0] * a.x + jb[4] * a.y + jb[8] * a.z, b1.im);
         b1.w = b1.w + sym_mul(b1.I, jb[1] * a.x + jb[5] * a.y + jb[9] * a.z);
-        store_vel(w.body, J.hdr.y, b1);
+        store_vel(w.body, joint_b1(w, J), b1);
     }
     if (b2.flags & SB_DYNAMIC) {
         b2.v = b2.v + cmul(jb[2] * a.x + jb[6] * a.y + jb[10] * a.z, b2.im);
         b2.w = b2.w + sym_mul(b2.I, jb[3] * a.x + jb[7] * a.y + jb[11] * a.z);
-        store_vel(w.body, J.hdr.z, b2);
+        store_vel(w.body, joint_b2(w, J), b2);
     }
 }
 // Prepare: prm = (bias, softness, limit bias, limit softness), lim = (min, max, -, clamp),
 // inverse effective mass in eff[0..2], bilateral block inverse in bil, couplings in cpl
-__device__ void line_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    LBody b1 = load_body(w.body, J.hdr.y), b2 = load_body(w.body, J.hdr.z);
+template <class W>
+__device__ void line_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    LBody b1 = load_body(w.body, joint_b1(w, J)), b2 = load_body(w.body, joint_b2(w, J));
     v3 jb[12];
     v3 err = line_jacobian(w, J, jb);
     const sym6 I1 = b1.I, I2 = b2.I;
@@ -1030,8 +1063,9 @@ __device__ void line_prepare(const WorldDev& w, JointDev& J, const StepParams& s
     J.bil = make_float4(bil.x, bil.y, bil.z, 0.f);
     J.cpl = make_float4(cx, cy, 0.f, 0.f);
 }
-__device__ void line_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    LBody b1 = load_body(w.body, J.hdr.y), b2 = load_body(w.body, J.hdr.z);
+template <class W>
+__device__ void line_iterate(const W& w, JointDev& J, const StepParams& sp) {
+    LBody b1 = load_body(w.body, joint_b1(w, J)), b2 = load_body(w.body, joint_b2(w, J));
     v3 jb[12];
     line_jacobian(w, J, jb);
     v3 jv = mk3(dot(jb[0], b1.v) + dot(jb[1], b1.w) + dot(jb[2], b2.v) + dot(jb[3], b2.w),
@@ -1073,12 +1107,14 @@ __device__ __forceinline__ float ellipse_radius(float a, float b, float c, float
     derivative = c * s * (v * v - u * u) / sq;
     return scale / sqrtf(sq);
 }
-__device__ __forceinline__ void elliptical_apply(const WorldDev& w, const JointDev& J, LBody& b1, LBody& b2, v3 jac, float a) {
-    if (b1.flags & SB_DYNAMIC) { b1.w = b1.w + sym_mul(b1.I, a * jac); store_vel(w.body, J.hdr.y, b1); }
-    if (b2.flags & SB_DYNAMIC) { b2.w = b2.w - sym_mul(b2.I, a * jac); store_vel(w.body, J.hdr.z, b2); }
+template <class W>
+__device__ __forceinline__ void elliptical_apply(const W& w, const JointDev& J, LBody& b1, LBody& b2, v3 jac, float a) {
+    if (b1.flags & SB_DYNAMIC) { b1.w = b1.w + sym_mul(b1.I, a * jac); store_vel(w.body, joint_b1(w, J), b1); }
+    if (b2.flags & SB_DYNAMIC) { b2.w = b2.w - sym_mul(b2.I, a * jac); store_vel(w.body, joint_b2(w, J), b2); }
 }
-__device__ void elliptical_prepare(const WorldDev& w, JointDev& J, const StepParams& sp) {
-    int i1 = J.hdr.y, i2 = J.hdr.z;
+template <class W>
+__device__ void elliptical_prepare(const W& w, JointDev& J, const StepParams& sp) {
+    int i1 = joint_b1(w, J), i2 = joint_b2(w, J);
     LBody b1 = load_body(w.body, i1), b2 = load_body(w.body, i2);
     const q4 q1 = mkq(w.q[i1]), q2 = mkq(w.q[i2]);
     const v3 axis = rotate(mk3(J.la1), q1);
@@ -1144,10 +1180,11 @@ __device__ void elliptical_prepare(const WorldDev& w, JointDev& J, const StepPar
     J.acc.x = acc;
     elliptical_apply(w, J, b1, b2, jac, acc);
 }
-__device__ void elliptical_iterate(const WorldDev& w, JointDev& J, const StepParams& sp) {
+template <class W>
+__device__ void elliptical_iterate(const W& w, JointDev& J, const StepParams& sp) {
     const int clamp = (int)J.bil.w;
     if (clamp == 0) return;
-    LBody b1 = load_body(w.body, J.hdr.y), b2 = load_body(w.body, J.hdr.z);
+    LBody b1 = load_body(w.body, joint_b1(w, J)), b2 = load_body(w.body, joint_b2(w, J));
     const v3 jac = mk3(J.jac[0]);
     const float jv = dot(b1.w - b2.w, jac);
     const float lambda = -J.bil.x * (jv + J.bias.x + J.acc.x * J.prm.y * sp.inv_sub_dt);
@@ -1159,7 +1196,8 @@ __device__ void elliptical_iterate(const WorldDev& w, JointDev& J, const StepPar
     elliptical_apply(w, J, b1, b2, jac, acc - old);
 }
 
-__device__ __forceinline__ void joint_prepare(const WorldDev& w, int j, const StepParams& sp) {
+template <class W>
+__device__ __forceinline__ void joint_prepare(const W& w, int j, const StepParams& sp) {
     JointDev& J = w.joints[j];
     switch (J.hdr.x) {
         case JG_CONSTRAINT_BALLSOCKET: ballsocket_prepare(w, J, sp); break;
@@ -1178,7 +1216,8 @@ __device__ __forceinline__ void joint_prepare(const WorldDev& w, int j, const St
         default: twist_prepare(w, J, sp); break;
     }
 }
-__device__ __forceinline__ void joint_iterate(const WorldDev& w, int j, const StepParams& sp) {
+template <class W>
+__device__ __forceinline__ void joint_iterate(const W& w, int j, const StepParams& sp) {
     JointDev& J = w.joints[j];
     switch (J.hdr.x) {
         case JG_CONSTRAINT_BALLSOCKET: ballsocket_iterate(w, J, sp); break;

@@ -1,4 +1,4 @@
-// Substepped sequential-impulse solve in one persistent, cooperatively launched kernel:
+// Substepped sequential-impulse solve:
 //   for each substep (World.Step.cs:234-253):
 //     IntegrateForces (World.Step.cs:1060-1072)                       bodies, grid-stride
 //     Prepare, colour by colour (Contact.cs:802-924, BallSocket.cs:140-183, HingeAngle.cs:133-220)
@@ -6,10 +6,11 @@
 //     IntegrateVelocities (World.Step.cs:1106-1133)                   bodies, grid-stride
 //     relaxation x colours: Iterate without bias (World.Step.cs:1135-1153)
 // Rows of one colour share no dynamic body, so a colour is solved in parallel with no
-// atomics.  Two kernels: k_solve runs global colours with a grid barrier between them;
+// atomics.  Three kernels: k_solve runs global colours with a grid barrier between them;
 // k_solve_tasks runs the partitioned schedule (spatial tasks with their bodies in shared
 // memory and a block barrier between local colours, the three grid phases handed off task
-// by task, and the remainder in global colours).  Arbiters are stored colour-sorted, so each
+// by task, and the remainder in global colours), both persistent and cooperatively launched;
+// k_solve_groups runs a scene of small independent parts, one CTA per part for the whole step.  Arbiters are stored colour-sorted, so each
 // colour is a contiguous range of coalesced float4 rows.  The per-step body update
 // (RigidBody.Update, RigidBody.cs:716-764) is a separate kernel.
 #include "jg_sync.cuh"
@@ -163,6 +164,41 @@ __device__ __forceinline__ void iterate_contact(const ArbStore& A, int i, int mo
                             d2, l2);
 }
 
+// Staged task bodies in shared memory as four arrays of `stride` float4 (v, w, i0, i1 of
+// SBody): random slots spread over all banks, where 64-byte records would meet in two.
+__device__ __forceinline__ LBody sbody_load(const float4* sb, int slot, int stride) {
+    float4 v = sb[slot], wv = sb[stride + slot], i0 = sb[2 * stride + slot], i1 = sb[3 * stride + slot];
+    LBody b;
+    b.v = mk3(v); b.w = mk3(wv);
+    b.im = mk3(v.w, wv.w, i1.z);
+    b.I.m11 = i0.x; b.I.m12 = i0.y; b.I.m13 = i0.z; b.I.m22 = i0.w; b.I.m23 = i1.x; b.I.m33 = i1.y;
+    b.flags = __float_as_int(i1.w);
+    return b;
+}
+__device__ __forceinline__ void sbody_store(float4* sb, int slot, int stride, const LBody& b) {
+    sb[slot] = f4(b.v, b.im.x);
+    sb[stride + slot] = f4(b.w, b.im.y);
+}
+// View of one solve group for the constraint rows: bodies in shared memory as four arrays of
+// `stride` float4 under local slots, poses in global memory behind the slots' body ids, the
+// constraints' records in shared memory too.
+struct GroupBodies { float4* p; int stride; };
+struct GroupPoses {
+    const float4* g;
+    const int* ids;
+    __device__ __forceinline__ float4 operator[](int i) const { return g[ids[i]]; }
+};
+struct GroupView {
+    GroupBodies body;
+    GroupPoses pos, q;
+    JointDev* joints;
+    int b1, b2;  // the current constraint's slots
+};
+__device__ __forceinline__ LBody load_body(const GroupBodies& B, int i) { return sbody_load(B.p, i, B.stride); }
+__device__ __forceinline__ void store_vel(const GroupBodies& B, int i, const LBody& b) { sbody_store(B.p, i, B.stride, b); }
+__device__ __forceinline__ int joint_b1(const GroupView& v, const JointDev&) { return v.b1; }
+__device__ __forceinline__ int joint_b2(const GroupView& v, const JointDev&) { return v.b2; }
+
 #include "jg_joints.cuh"
 
 __device__ __forceinline__ void solve_arbiter(const WorldDev& w, const ArbStore& A, int a, int phase, const StepParams& sp,
@@ -303,24 +339,27 @@ __device__ __noinline__ v3 solve_gyroscopic(const sym6& I, v3 av, float dt) {
     return av - d;
 }
 
-// IntegrateVelocities (World.Step.cs:1106-1133) with SolveGyroscopic (World.Step.cs:1075-1104).
+// IntegrateVelocities (World.Step.cs:1106-1133) with SolveGyroscopic (World.Step.cs:1075-1104)
+// of one body; true when the gyroscopic term changed the angular velocity.
+__device__ __forceinline__ bool integrate_velocity(const WorldDev& w, const StepParams& sp, int i, int flags, v3 lv, v3& av,
+                                                   const sym6& I) {
+    float4 p = w.pos[i];
+    w.pos[i] = make_float4(p.x + lv.x * sp.sub_dt, p.y + lv.y * sp.sub_dt, p.z + lv.z * sp.sub_dt, p.w);
+    q4 rq = rotation_quaternion(av, sp.sub_dt);
+    q4 q = qnormalize(qmul(rq, mkq(w.q[i])));
+    w.q[i] = f4(q);
+    if (!((flags & JG_BODY_GYROSCOPIC) && ((flags >> 4) & 63) == 0)) return false;
+    // JSymmetricMatrix.Inverse of the world inverse inertia, then SolveGyroscopic
+    av = solve_gyroscopic(sym_inverse_ref(I), av, sp.sub_dt);
+    return true;
+}
 __device__ __forceinline__ void integrate_velocities_all(const WorldDev& w, const StepParams& sp, int tid, int nth) {
     for (int i = tid; i < w.nb; i += nth) {
         int4 bi = w.binfo[i];
         if (bi.x == JG_MOTION_STATIC || (sp.allow_deact && !(bi.y & JG_BODY_ACTIVE))) continue;
-        SBody b = w.body[i];
-        v3 lv = mk3(b.v), av = mk3(b.w);
-        float4 p = w.pos[i];
-        w.pos[i] = make_float4(p.x + lv.x * sp.sub_dt, p.y + lv.y * sp.sub_dt, p.z + lv.z * sp.sub_dt, p.w);
-        q4 rq = rotation_quaternion(av, sp.sub_dt);
-        q4 q = qnormalize(qmul(rq, mkq(w.q[i])));
-        w.q[i] = f4(q);
-        if ((bi.y & JG_BODY_GYROSCOPIC) && ((bi.y >> 4) & 63) == 0) {
-            // JSymmetricMatrix.Inverse of the world inverse inertia, then SolveGyroscopic
-            sym6 Ii;
-            Ii.m11 = b.i0.x; Ii.m12 = b.i0.y; Ii.m13 = b.i0.z; Ii.m22 = b.i0.w; Ii.m23 = b.i1.x; Ii.m33 = b.i1.y;
-            w.body[i].w = f4(solve_gyroscopic(sym_inverse_ref(Ii), av, sp.sub_dt), b.w.w);
-        }
+        const LBody b = load_body(w.body, i);
+        v3 av = b.w;
+        if (integrate_velocity(w, sp, i, bi.y, b.v, av, b.I)) w.body[i].w = f4(av, b.im.y);
     }
 }
 
@@ -419,21 +458,6 @@ __device__ __forceinline__ void stage_arbiter(float4* dst, const ArbStore& A, in
     }
 }
 
-// Staged task bodies in shared memory as four arrays of `stride` float4 (v, w, i0, i1 of
-// SBody): random slots spread over all banks, where 64-byte records would meet in two.
-__device__ __forceinline__ LBody sbody_load(const float4* sb, int slot, int stride) {
-    float4 v = sb[slot], wv = sb[stride + slot], i0 = sb[2 * stride + slot], i1 = sb[3 * stride + slot];
-    LBody b;
-    b.v = mk3(v); b.w = mk3(wv);
-    b.im = mk3(v.w, wv.w, i1.z);
-    b.I.m11 = i0.x; b.I.m12 = i0.y; b.I.m13 = i0.z; b.I.m22 = i0.w; b.I.m23 = i1.x; b.I.m33 = i1.y;
-    b.flags = __float_as_int(i1.w);
-    return b;
-}
-__device__ __forceinline__ void sbody_store(float4* sb, int slot, int stride, const LBody& b) {
-    sb[slot] = f4(b.v, b.im.x);
-    sb[stride + slot] = f4(b.w, b.im.y);
-}
 // A non-dynamic body: velocities only (zero inverse mass and inertia, as its SBody holds).
 __device__ __forceinline__ LBody fixed_body(float4 v, float4 wv) {
     LBody b;
@@ -703,6 +727,7 @@ __global__ void k_solve_tasks(WorldDev w, StepParams sp) {
     float4* ring = solve_smem + 4 * sp.task_maxb;
     volatile int* sver = (volatile int*)(ring + (size_t)JG_TASK_RING * blockDim.x * JG_TASK_STAGE_F4);
     __shared__ int s_abort;
+    if (sp.groups && !w.gr->off) return;  // k_solve_groups has solved the step
     if (threadIdx.x == 0) s_abort = 0;
     __syncthreads();
     const ArbStore& A = w.arb[w.cur];
@@ -774,6 +799,476 @@ __global__ void k_solve_tasks(WorldDev w, StepParams sp) {
                 if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
             }
         }
+    }
+}
+
+// ---- solve groups ----------------------------------------------------------------------
+// One CTA per group (jg_groups.cu): all substeps and passes, its bodies in shared memory, no
+// wait on any other CTA.  Rows run in the order k_solve_tasks gives them, by dataflow: each
+// row waits until the rows before it on its own bodies are done.  The counts keep growing
+// over the passes (row of rank r of a body with n rows runs at count pass * n + r), so that a
+// pass starts on the bodies the previous one has left, and only the prepare pass and the
+// integration steps end with a block barrier.
+constexpr int GROUP_LEVELS = JG_SCHED_GRIDS * JG_TASK_MAXC + JG_MAX_COLORS;  // order keys
+constexpr int GROUP_BUCKETS = JG_SCHED_GRIDS * JG_TASK_MAXC * 4 + JG_MAX_COLORS;
+constexpr unsigned GROUP_FIXED = 0x80000000u;  // a packed slot that orders nothing (non-dynamic body)
+constexpr int GROUP_JOINT = 1 << 30;
+
+__device__ __forceinline__ int group_level(int key) {
+    return key < JG_ORDER_REMAINDER ? (key >> 8) * JG_TASK_MAXC + (key & 255)
+                                    : JG_SCHED_GRIDS * JG_TASK_MAXC + (key - JG_ORDER_REMAINDER);
+}
+// Rows of a body below a level, from its masks of used levels (5 words).
+__device__ __forceinline__ int rows_below(const unsigned long long* mask, int level) {
+    int n = 0;
+    for (int k = 0; k < 5; k++) {
+        if (level >= 64 * (k + 1)) n += __popcll(mask[k]);
+        else if (level > 64 * k) n += __popcll(mask[k] & ((1ull << (level - 64 * k)) - 1ull));
+    }
+    return n;
+}
+static_assert(GROUP_LEVELS == 320, "five mask words");
+
+__device__ __noinline__ void group_joint_prepare(const GroupView& v, int j, const StepParams& sp) { joint_prepare(v, j, sp); }
+__device__ __noinline__ void group_joint_iterate(const GroupView& v, int j, const StepParams& sp) { joint_iterate(v, j, sp); }
+
+struct GroupMem {
+    float4* body;         // four arrays of `slots` float4
+    int slots;
+    volatile int* done;   // rows done per slot
+    const int* total;     // rows per slot and pass
+    const int* ids;       // body of each slot
+    const int4* con;      // packed slots and ranks, kind | usage | mode, arbiter or joint
+    const float2* row;    // friction, first contact
+    float4* acc;          // accumulated impulses and tangent-2 mass per contact
+    int narb, n;          // contacts, rows
+};
+
+// Iterations run each arbiter on two lanes, the first with body 1 and the second with body 2:
+// each computes its body's velocity at the contact, the two are exchanged, both compute the
+// impulses, and each applies them to its body.  A row is a chain of dependent operations that
+// one lane issues in about 205 instructions; the few arbiters of a colour that are ready at once
+// leave a warp alone on its scheduler, so that the instruction count is the latency and the
+// latencies of the colours add up.  A pair needs about 130.  (Eight lanes an arbiter, one
+// vector component each, measured slower: the shuffles between the components cost more than
+// the arithmetic they spread.)  Every value is produced by the operations of iterate_row in
+// their order (a subtraction is the addition of the exactly negated operand), so the results
+// are the same bits.
+struct PairRow { float4 n, t1, t2, r; };
+__device__ __forceinline__ PairRow pair_load(const ArbStore& A, const float4* arms, int i) {
+    return PairRow{A.cn[i], A.ct1[i], A.ct2[i], arms[i]};
+}
+
+// Passes `pass` to `end` over the group's contacts.  Pair P owns rows P, P + pairs, ... in order;
+// its next row's data is on the way while it waits or computes.  The accumulated impulses
+// and the tangent-2 mass are in shared memory: they change in every pass, and a store to global
+// memory drops its line from the L1, where the rest of the row stays.  False when the pass was
+// abandoned.
+__device__ __forceinline__ bool pair_passes(const ArbStore& A, int cap, const GroupMem& g, int pass, int end, bool bias,
+                                            volatile int* abort_flag, int* status) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, h = lane & 1;
+    const int pairs = blockDim.x >> 1, P = threadIdx.x >> 1;
+    const float4* const arms = h ? A.cr2 : A.cr1;
+    const float sgn = h ? 1.f : -1.f;
+    int j = P;
+    const int n = g.narb;
+    if (P >= n) pass = end;
+    int4 H = make_int4(-1, -1, 0, 0), N = H;      // this arbiter's header and the next one's
+    int um = 0, d = 0, target = 0, slot = -1;
+    PairRow R{};
+    if (pass < end) {
+        H = g.con[j];
+        N = g.con[j + pairs < n ? j + pairs : P];
+        um = H.z & 15;
+        d = H.w;
+        R = pair_load(A, arms, (__ffs(um) - 1) * cap + d);
+    }
+    bool fresh = true;
+    unsigned idle = 0;
+    for (;;) {
+        const bool active = pass < end;
+        if (!__any_sync(FULL, active)) break;
+        bool ok = true;
+        if (active) {
+            if (fresh) {
+                const int p = h ? H.y : H.x;
+                slot = p >= 0 ? slot_of(p) : -1;
+                target = p >= 0 ? pass * g.total[slot] + rank_of(p) : 0;
+                fresh = false;
+            }
+            ok = slot < 0 || g.done[slot] == target;
+        }
+        const unsigned wait = __ballot_sync(FULL, !ok);
+        const bool go = active && ((wait >> (lane & 30)) & 3u) == 0;
+        if (!__any_sync(FULL, go)) {
+            if (idle < 16 ? (++idle, *abort_flag != 0) : !backoff(idle, abort_flag, status)) return false;
+            continue;
+        }
+        idle = 0;
+        __threadfence_block();  // the counts before the bodies they guard
+        LBody B = fixed_body(make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f));
+        if (go) {
+            if (slot >= 0) B = sbody_load(g.body, slot, g.slots);
+            else B = fixed_body(A.sv[d], A.sv[cap + d]);
+            if (!h) {
+                B.im = -B.im;
+                B.I.m11 = -B.I.m11; B.I.m12 = -B.I.m12; B.I.m13 = -B.I.m13;
+                B.I.m22 = -B.I.m22; B.I.m23 = -B.I.m23; B.I.m33 = -B.I.m33;
+            }
+        }
+        const int mode = (H.z >> 4) & 15;
+        const bool lin = (mode >> (2 * h)) & 1, ang = (mode >> (2 * h + 1)) & 1, arm = (mode & 10) != 0;
+        const float2 extra = g.row[active ? j : 0];
+        const float mu = extra.x;
+        float4* pacc = g.acc + __float_as_int(extra.y);
+        int left = go ? um : 0;
+        for (int rows = __reduce_max_sync(FULL, __popc(left)); rows > 0; rows--) {
+            const bool run = left != 0;
+            const PairRow q = R;
+            left &= left - 1;
+            const float4 old = run ? *pacc : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (left) R = pair_load(A, arms, (__ffs(left) - 1) * cap + d);  // this arbiter's next row
+            const v3 nn = mk3(q.n), t1 = mk3(q.t1), t2 = mk3(q.t2), rel = mk3(q.r);
+            const float other_mass = __shfl_xor_sync(FULL, q.r.w, 1);
+            const float mN = h ? other_mass : q.r.w, mT1 = h ? q.r.w : other_mass, mT2 = old.w;
+            v3 vel = B.v;
+            if (arm) vel = B.v + cross(B.w, rel);
+            v3 dv;  // body 2's minus body 1's, in both lanes
+            dv.x = __fmaf_rn(__shfl_xor_sync(FULL, vel.x, 1), -sgn, sgn * vel.x);
+            dv.y = __fmaf_rn(__shfl_xor_sync(FULL, vel.y, 1), -sgn, sgn * vel.y);
+            dv.z = __fmaf_rn(__shfl_xor_sync(FULL, vel.z, 1), -sgn, sgn * vel.z);
+            float b = q.n.w;
+            if (bias && q.t1.w > 0.f) b = fmaxf(q.t1.w, q.n.w);
+            const float vn = dot(nn, dv), vt1 = dot(t1, dv), vt2 = dot(t2, dv);
+            const float max_t = mu * old.x;
+            const float aN = fmaxf(old.x + (-vn + b) * mN, 0.0f);
+            const float aT1 = fminf(fmaxf(old.y + mT1 * -vt1, -max_t), max_t);
+            const float aT2 = fminf(fmaxf(old.z + mT2 * -vt2, -max_t), max_t);
+            const float ni = aN - old.x, ti1 = aT1 - old.y, ti2 = aT2 - old.z;
+            if (run) *pacc++ = make_float4(aN, aT1, aT2, mT2);  // (by both lanes: each reads back what it wrote itself)
+            v3 imp = ni * nn;
+            imp = imp + ti1 * t1;
+            imp = imp + ti2 * t2;
+            if (run && lin) B.v = B.v + cmul(imp, B.im);
+            if (run && ang) B.w = B.w + sym_mul(B.I, cross(rel, imp));
+        }
+        if (go && slot >= 0 && (lin || ang)) {
+            if (!h) B.im = -B.im;
+            sbody_store(g.body, slot, g.slots, B);
+        }
+        __threadfence_block();  // the bodies' new velocities before the counts
+        if (go) {
+            if (slot >= 0) g.done[slot] = target + 1;
+            fresh = true;
+            j += pairs;
+            if (j >= n) { j = P; pass++; }
+            // The next arbiter's first row, and the header after it.  Not before the fence above:
+            // a fence waits for the loads in flight.
+            H = N;
+            if (pass < end) {
+                N = g.con[j + pairs < n ? j + pairs : P];
+                um = H.z & 15;
+                d = H.w;
+                R = pair_load(A, arms, (__ffs(um) - 1) * cap + d);
+            }
+        }
+    }
+    return true;
+}
+
+// The prepare pass: one lane per row.
+__device__ __forceinline__ bool group_prepare(const WorldDev& w, const ArbStore& A, const StepParams& sp, const GroupMem& g,
+                                              GroupView& v, int pass, volatile int* abort_flag, int* status) {
+    const int cap = w.cap_arb, bs = blockDim.x;
+    int m = threadIdx.x;
+    unsigned idle = 0;
+    bool loaded = false;
+    int4 c = make_int4(0, 0, 0, 0);
+    int t1 = 0, t2 = 0;
+    for (;;) {
+        const bool active = m < g.n;
+        if (!__any_sync(0xffffffffu, active)) break;
+        bool go = false;
+        if (active) {
+            if (!loaded) {
+                c = g.con[m];
+                t1 = c.x >= 0 ? pass * g.total[slot_of(c.x)] + rank_of(c.x) : 0;
+                t2 = c.y >= 0 ? pass * g.total[slot_of(c.y)] + rank_of(c.y) : 0;
+                loaded = true;
+            }
+            go = (c.x < 0 || g.done[slot_of(c.x)] == t1) && (c.y < 0 || g.done[slot_of(c.y)] == t2);
+        }
+        if (go) {
+            __threadfence_block();  // the counts before the bodies they guard
+            if (c.z & GROUP_JOINT) {
+                v.b1 = slot_of(c.x);
+                v.b2 = slot_of(c.y);
+                group_joint_prepare(v, c.w, sp);
+            } else {
+                const int d = c.w, usage = c.z & 15, mode = (c.z >> 4) & 15;
+                LBody b1 = c.x >= 0 ? sbody_load(g.body, slot_of(c.x), g.slots) : fixed_body(A.sv[d], A.sv[cap + d]);
+                LBody b2 = c.y >= 0 ? sbody_load(g.body, slot_of(c.y), g.slots) : fixed_body(A.sv[d], A.sv[cap + d]);
+                const int2 bb = A.body[d];
+                const float spec = A.mat[d].z;
+                const v3 pos1 = mk3(w.pos[bb.x]), pos2 = mk3(w.pos[bb.y]);
+                const q4 q1 = mkq(w.q[bb.x]), q2 = mkq(w.q[bb.y]);
+                for (unsigned um = (unsigned)usage; um; um &= um - 1)
+                    prepare_contact(A, (__ffs(um) - 1) * cap + d, mode, spec, b1, b2, pos1, q1, pos2, q2, sp);
+                if ((mode & 3) && c.x >= 0) sbody_store(g.body, slot_of(c.x), g.slots, b1);
+                if ((mode & 12) && c.y >= 0) sbody_store(g.body, slot_of(c.y), g.slots, b2);
+            }
+            __threadfence_block();  // the bodies' new velocities before the counts
+            if (c.x >= 0) g.done[slot_of(c.x)] = t1 + 1;
+            if (c.y >= 0) g.done[slot_of(c.y)] = t2 + 1;
+            loaded = false;
+            m += bs;
+        }
+        if (__any_sync(0xffffffffu, go)) idle = 0;
+        else if (idle < 16 ? (++idle, *abort_flag != 0) : !backoff(idle, abort_flag, status)) return false;
+    }
+    return true;
+}
+
+// One pass over the group's constraints (rows narb .. n), one lane each.  Of a few, neighbours in
+// the order go to different warps: constraints of one level differ in kind, and lanes of a warp
+// run the kinds one after another.  Relaxation passes leave the constraints alone.
+__device__ __forceinline__ bool group_joints(const StepParams& sp, const GroupMem& g, GroupView& v, int pass, bool solve,
+                                             volatile int* abort_flag, int* status) {
+    const int warps = blockDim.x >> 5;
+    int m = g.narb + (g.n - g.narb <= 32 ? (threadIdx.x & 31) * warps + (threadIdx.x >> 5) : threadIdx.x);
+    unsigned idle = 0;
+    bool loaded = false;
+    int4 c = make_int4(0, 0, 0, 0);
+    int t1 = 0, t2 = 0;
+    for (;;) {
+        const bool active = m < g.n;
+        if (!__any_sync(0xffffffffu, active)) break;
+        bool go = false;
+        if (active) {
+            if (!loaded) {
+                c = g.con[m];
+                t1 = c.x >= 0 ? pass * g.total[slot_of(c.x)] + rank_of(c.x) : 0;
+                t2 = c.y >= 0 ? pass * g.total[slot_of(c.y)] + rank_of(c.y) : 0;
+                loaded = true;
+            }
+            go = (c.x < 0 || g.done[slot_of(c.x)] == t1) && (c.y < 0 || g.done[slot_of(c.y)] == t2);
+        }
+        if (go) {
+            __threadfence_block();  // the counts before the bodies they guard
+            v.b1 = slot_of(c.x);
+            v.b2 = slot_of(c.y);
+            if (solve) group_joint_iterate(v, c.w, sp);
+            __threadfence_block();  // the bodies' new velocities before the counts
+            if (c.x >= 0) g.done[slot_of(c.x)] = t1 + 1;
+            if (c.y >= 0) g.done[slot_of(c.y)] = t2 + 1;
+            loaded = false;
+            m += blockDim.x;
+        }
+        if (__any_sync(0xffffffffu, go)) idle = 0;
+        else if (idle < 16 ? (++idle, *abort_flag != 0) : !backoff(idle, abort_flag, status)) return false;
+    }
+    return true;
+}
+
+// npass passes over the group's rows; `base` passes are done already.  Contacts come before
+// constraints in the order of every body, so a pass takes them in turn, and without
+// constraints the passes run into one another.
+__device__ __forceinline__ bool group_passes(const WorldDev& w, const ArbStore& A, const StepParams& sp, const GroupMem& g,
+                                             GroupView& v, int base, int npass, bool bias, volatile int* abort_flag,
+                                             int* status) {
+    if (g.n == g.narb) return pair_passes(A, w.cap_arb, g, base, base + npass, bias, abort_flag, status);
+    bool ok = true;
+    for (int k = base; k < base + npass && ok; k++) {
+        if (g.narb) ok = pair_passes(A, w.cap_arb, g, k, k + 1, bias, abort_flag, status);
+        ok = ok && group_joints(sp, g, v, k, bias, abort_flag, status);
+    }
+    return ok;
+}
+
+// Bodies without any row in this step: force and velocity integration only.
+__device__ __forceinline__ void integrate_free_bodies(const WorldDev& w, const StepParams& sp, int tid, int nth) {
+    for (int i = tid; i < w.nb; i += nth) {
+        const int4 bi = w.binfo[i];
+        if (w.gr_slot[i] >= 0 || bi.x == JG_MOTION_STATIC || (sp.allow_deact && !(bi.y & JG_BODY_ACTIVE))) continue;
+        const LBody b = load_body(w.body, i);
+        v3 lv = b.v, av = b.w;
+        const v3 dv = mk3(w.dv[i]), dw = mk3(w.dw[i]);
+        for (int s = 0; s < sp.substeps; s++) {
+            if (bi.x == JG_MOTION_DYNAMIC) {
+                av = mk3(av.x + dw.x, av.y + dw.y, av.z + dw.z);
+                lv = mk3(lv.x + dv.x, lv.y + dv.y, lv.z + dv.z);
+            }
+            integrate_velocity(w, sp, i, bi.y, lv, av, b.I);
+        }
+        w.body[i].v = f4(lv, b.im.x);
+        w.body[i].w = f4(av, b.im.y);
+    }
+}
+
+// The large launch takes the groups that need its shared memory, and all of them when they are
+// no more than its CTAs; the small launch takes the small groups of a step with many.
+template <bool kLarge>
+__global__ void __launch_bounds__(kLarge ? 256 : 64, kLarge ? 2 : 8) k_solve_groups(WorldDev w, StepParams sp, int large_ctas) {
+    extern __shared__ float4 solve_smem[];
+    __shared__ int s_bucket[GROUP_BUCKETS];
+    __shared__ int s_abort, s_item;
+    if (w.gr->off) return;
+    const ArbStore& A = w.arb[w.cur];
+    const int tid = threadIdx.x, bs = blockDim.x;
+    int* status = &w.ctr->status;
+    if (kLarge) integrate_free_bodies(w, sp, blockIdx.x * bs + tid, gridDim.x * bs);
+    if (tid == 0) s_abort = 0;
+    const int small = w.gr->count[0], large = w.gr->count[1];
+    const bool few = small + large <= large_ctas;
+    const int count = kLarge ? large + (few ? small : 0) : (few ? 0 : small);
+    // the first groups go one to each block in order, which spreads them over the SMs
+    for (int item = blockIdx.x; item < count; ) {
+        const GroupRec R = w.gr_rec[kLarge && item < large ? w.cap_bodies + item : item - (kLarge ? large : 0)];
+        const int slots = R.nbody + R.njoint, n = R.narb + R.njoint;
+        float4* body = solve_smem;
+        int4* con = (int4*)(body + 4 * slots);
+        float4* acc = (float4*)(con + n);
+        JointDev* joints = (JointDev*)(acc + R.ncon);
+        float2* row = (float2*)(joints + R.njoint);
+        int* done = (int*)(row + n);
+        int* total = done + slots;
+        int* ids = total + slots;
+        unsigned long long* mask = (unsigned long long*)body;  // [5 * nbody], until the bodies are loaded
+        // levels used per body, rows per bucket (level, then most contacts first)
+        for (int i = tid; i < 5 * R.nbody; i += bs) mask[i] = 0ull;
+        for (int i = tid; i < GROUP_BUCKETS; i += bs) s_bucket[i] = 0;
+        if (tid == 0) s_item = 0;
+        for (int i = tid; i < R.nbody; i += bs) ids[i] = w.gr_body[R.body + i];
+        __syncthreads();
+        auto describe = [&](int i, int& s1, int& s2, int& level, int& bucket, int& kind, int& what) {
+            int2 bb;
+            if (i < R.narb) {
+                what = w.gr_arb[R.arb + i];
+                bb = A.body[what];
+                const int4 info = A.info[what];
+                level = group_level(info.z);
+                kind = (info.x & 15) | ((info.y & 15) << 4);
+                const int pc = __popc(info.x & 15);
+                bucket = level < JG_SCHED_GRIDS * JG_TASK_MAXC ? 4 * level + (pc >= 4 ? 0 : (pc <= 1 ? 3 : 4 - pc))
+                                                               : level + 3 * JG_SCHED_GRIDS * JG_TASK_MAXC;
+            } else {
+                what = w.gr_joint[R.joint + i - R.narb];
+                const int4 h = w.joints[what].hdr;
+                bb = make_int2(h.y, h.z);
+                level = group_level(h.w);
+                kind = GROUP_JOINT;
+                bucket = level + 3 * JG_SCHED_GRIDS * JG_TASK_MAXC;
+            }
+            s1 = w.binfo[bb.x].x == JG_MOTION_DYNAMIC ? w.gr_slot[bb.x] - R.body : -1 - bb.x;
+            s2 = w.binfo[bb.y].x == JG_MOTION_DYNAMIC ? w.gr_slot[bb.y] - R.body : -1 - bb.y;
+        };
+        for (int i = tid; i < n; i += bs) {
+            int s1, s2, level, bucket, kind, what;
+            describe(i, s1, s2, level, bucket, kind, what);
+            const unsigned long long bit = 1ull << (level & 63);
+            if (s1 >= 0) atomicOr(&mask[5 * s1 + (level >> 6)], bit);
+            if (s2 >= 0) atomicOr(&mask[5 * s2 + (level >> 6)], bit);
+            atomicAdd(&s_bucket[bucket], 1);
+        }
+        __syncthreads();
+        if (tid < 32) {  // bucket counts to first rows
+            int carry = 0;
+            for (int k = 0; k < GROUP_BUCKETS; k += 32) {
+                const int x = s_bucket[k + tid];
+                int y = x;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int z = __shfl_up_sync(0xffffffffu, y, o);
+                    if (tid >= o) y += z;
+                }
+                s_bucket[k + tid] = carry + y - x;
+                carry += __shfl_sync(0xffffffffu, y, 31);
+            }
+        }
+        for (int i = tid; i < slots; i += bs) {
+            total[i] = i < R.nbody ? rows_below(mask + 5 * i, GROUP_LEVELS) : 0;
+            done[i] = 0;
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += bs) {
+            int s1, s2, level, bucket, kind, what;
+            describe(i, s1, s2, level, bucket, kind, what);
+            const int p = atomicAdd(&s_bucket[bucket], 1);
+            // a constraint's non-dynamic body takes the slot kept for the constraint
+            const int extra = R.nbody + (i - R.narb);
+            unsigned c1 = GROUP_FIXED, c2 = GROUP_FIXED;
+            if (s1 >= 0) c1 = (unsigned)s1 | ((unsigned)rows_below(mask + 5 * s1, level) << 16);
+            else if (i >= R.narb) { c1 |= (unsigned)extra; ids[extra] = -1 - s1; }
+            if (s2 >= 0) c2 = (unsigned)s2 | ((unsigned)rows_below(mask + 5 * s2, level) << 16);
+            else if (i >= R.narb) { c2 |= (unsigned)extra; ids[extra] = -1 - s2; }
+            if (i >= R.narb && s1 >= 0 && s2 >= 0) ids[extra] = -1;
+            con[p] = make_int4((int)c1, (int)c2, kind | (level << 8), i < R.narb ? what : i - R.narb);
+            if (i < R.narb) row[p] = make_float2(A.mat[what].x, __int_as_float(atomicAdd(&s_item, __popc(kind & 15))));
+        }
+        __syncthreads();
+        for (int i = tid; i < slots; i += bs) {
+            if (ids[i] < 0) continue;
+            const SBody b = w.body[ids[i]];
+            body[i] = b.v; body[slots + i] = b.w; body[2 * slots + i] = b.i0; body[3 * slots + i] = b.i1;
+        }
+        // the constraints' records, a float4 at a time
+        constexpr int JF4 = sizeof(JointDev) / 16;
+        for (int i = tid; i < R.njoint * JF4; i += bs)
+            ((float4*)joints)[i] = ((const float4*)&w.joints[w.gr_joint[R.joint + i / JF4]])[i % JF4];
+        const GroupMem g{body, slots, done, total, ids, con, row, acc, R.narb, n};
+        auto each_contact = [&](auto f) {
+            for (int m = tid; m < R.narb; m += bs) {
+                const int4 c = con[m];
+                float4* a = acc + __float_as_int(row[m].y);
+                for (int um = c.z & 15; um; um &= um - 1, a++) f(A.cacc[(__ffs(um) - 1) * w.cap_arb + c.w], a);
+            }
+        };
+        GroupView v{{body, slots}, {w.pos, ids}, {w.q, ids}, joints, 0, 0};
+        int base = 0;
+        bool ok = true;
+        for (int s = 0; s < sp.substeps && ok; s++) {
+            for (int i = tid; i < R.nbody; i += bs) {  // IntegrateForces
+                const int id = ids[i], flags = w.binfo[id].y;
+                if (sp.allow_deact && !(flags & JG_BODY_ACTIVE)) continue;
+                const float4 dv = w.dv[id], dw = w.dw[id], bv = body[i], bw = body[slots + i];
+                body[slots + i] = make_float4(bw.x + dw.x, bw.y + dw.y, bw.z + dw.z, bw.w);
+                body[i] = make_float4(bv.x + dv.x, bv.y + dv.y, bv.z + dv.z, bv.w);
+            }
+            __syncthreads();
+            ok = group_prepare(w, A, sp, g, v, base, &s_abort, status);
+            base++;
+            // prepare works on the records; the passes keep the impulses here
+            each_contact([](const float4& g, float4* c) { *c = g; });
+            __syncthreads();
+            ok = ok && group_passes(w, A, sp, g, v, base, sp.iterations, true, &s_abort, status);
+            base += sp.iterations;
+            __syncthreads();
+            for (int i = tid; i < R.nbody; i += bs) {  // IntegrateVelocities
+                const int id = ids[i], flags = w.binfo[id].y;
+                if (sp.allow_deact && !(flags & JG_BODY_ACTIVE)) continue;
+                const LBody b = sbody_load(body, i, slots);
+                v3 av = b.w;
+                if (integrate_velocity(w, sp, id, flags, b.v, av, b.I)) body[slots + i] = f4(av, b.im.y);
+            }
+            __syncthreads();
+            ok = ok && group_passes(w, A, sp, g, v, base, sp.relax, false, &s_abort, status);
+            base += sp.relax;
+            ok = __syncthreads_and(ok) != 0;
+            each_contact([](float4& g, const float4* c) { g = *c; });
+            __syncthreads();
+        }
+        for (int i = tid; i < R.nbody; i += bs) {
+            float4* dst = (float4*)&w.body[ids[i]];
+            dst[0] = body[i];
+            dst[1] = body[slots + i];
+        }
+        for (int i = tid; i < R.njoint * JF4; i += bs)
+            ((float4*)&w.joints[w.gr_joint[R.joint + i / JF4]])[i % JF4] = ((const float4*)joints)[i];
+        if (!ok) return;
+        if (tid == 0) s_item = gridDim.x + atomicAdd(&w.gr->next[kLarge], 1);
+        __syncthreads();
+        item = s_item;
+        __syncthreads();
     }
 }
 
@@ -876,7 +1371,12 @@ int jg_solver_init() {
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, (const void*)k_solve_tasks) != cudaSuccess) return -1;
     int dyn = pb - (int)fa.sharedSizeBytes;
-    return cudaFuncSetAttribute(k_solve_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) == cudaSuccess ? 0 : -1;
+    if (cudaFuncSetAttribute(k_solve_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return -1;
+    const void* groups[JG_GROUP_CLASSES] = {(const void*)k_solve_groups<false>, (const void*)k_solve_groups<true>};
+    for (int c = 0; c < JG_GROUP_CLASSES; c++)
+        if (cudaFuncSetAttribute(groups[c], cudaFuncAttributeMaxDynamicSharedMemorySize, jg_group_budget(c)) != cudaSuccess)
+            return -1;
+    return 0;
 }
 
 // Bodies a task can stage next to the arbiter ring of `block` threads when
@@ -894,6 +1394,14 @@ int jg_solver_task_maxb(int block, int ctas_per_sm) {
 
 static size_t task_smem(const StepParams& p, int block) {
     return ((size_t)4 * p.task_maxb + (size_t)JG_TASK_RING * block * JG_TASK_STAGE_F4) * 16 + (size_t)4 * p.task_maxb;
+}
+
+// The group solve.  (The two launches on two streams cost more in event records and waits than
+// their overlap gives where launches count, and nothing in between has work for both.)
+void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
+    const int large_ctas = nsm * jg_group_ctas(1);
+    k_solve_groups<true><<<large_ctas, jg_group_threads(1), jg_group_budget(1), s>>>(w, p, large_ctas);
+    k_solve_groups<false><<<nsm * jg_group_ctas(0), jg_group_threads(0), jg_group_budget(0), s>>>(w, p, large_ctas);
 }
 
 // The cooperative grid of each solve kernel is sized once per world (its device, block,

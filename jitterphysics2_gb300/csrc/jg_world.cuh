@@ -97,6 +97,7 @@ struct __align__(16) JointDev {
     float4 bil;      // bilateral block inverse xyz, hemisphere
     float4 cpl;      // coupling x, coupling y
 };
+static_assert(sizeof(JointDev) == 304, "jg_group_bytes");
 
 struct DevCounters {
     int npairs;
@@ -124,6 +125,36 @@ struct DevCounters {
     int nspec;        // speculative sweep candidates, and of those the pairs registered
     int nspec_hit;
     int pad[1];
+};
+
+// Solve groups (jg_groups.cu): independent parts of the step's constraint graph, one CTA each.
+// Two launches: many small groups (64 threads, eight CTAs an SM: 1024 limb chains solve in 0.53
+// ms, against 0.64 with 128 threads and four CTAs), and few or large ones (256 threads, two
+// an SM: 48 worlds in 1.07 ms, against 1.22 with 128 threads); the dynamic shared memory of one
+// CTA bounds a group.
+#define JG_GROUP_CLASSES 2
+// Single worlds are not split into groups above this many arbiters (a scene of that size is
+// one pile, whose components would be found for nothing), nor when a component has more rows
+// than this: a pile of 200 bodies (about 250 rows) solves in 0.79 ms as a group and 1.13 as tasks,
+// one of 400 (600 rows) in 1.35 as a group and 1.12 as tasks.
+#define JG_GROUP_MAXARB 16384
+#define JG_GROUP_MAXROWS 320
+JG_HD int jg_group_threads(int cls) { return cls == 0 ? 64 : 256; }
+JG_HD int jg_group_ctas(int cls) { return cls == 0 ? 8 : 2; }
+JG_HD int jg_group_budget(int cls) { return cls == 0 ? 23 * 1024 : 106 * 1024; }
+// Bytes of a group: per body slot (a constraint's non-dynamic body takes one too) the solver
+// record, its count and total of rows, and its id; per row its header, friction and first
+// contact; per contact its accumulated impulses; per constraint its record.
+JG_HD int jg_group_bytes(int nbody, int narb, int njoint, int ncon) {
+    return (nbody + njoint) * 76 + (narb + njoint) * 24 + ncon * 16 + njoint * 304 + 16;
+}
+
+struct GroupRec { int arb, narb, joint, njoint, body, nbody, ncon, pad; };  // a group's ranges of the member lists
+struct GroupCtl {
+    int off;                         // the groups cannot take this step
+    int arbs, joints, bodies;        // space handed out
+    int count[JG_GROUP_CLASSES];     // groups that fit the small CTA, groups that need the large one
+    int next[JG_GROUP_CLASSES];      // work cursors of the two launches
 };
 
 struct WorldDev {
@@ -218,6 +249,15 @@ struct WorldDev {
     int* sc_dst;                 // [cap_arb] final slot of a task arbiter, -1 for the remainder
     int* sc_lcol;                // [cap_arb] local colour of a task arbiter
     int4* sc_ls;                 // [cap_arb] body slots of a task arbiter
+    // solve groups
+    GroupCtl* gr;
+    int* gr_root;                // [cap_bodies] union-find parent
+    int* gr_slot;                // [cap_bodies] place of the body in gr_body, -1 if it has no row
+    int *gr_narb, *gr_njoint, *gr_nbody, *gr_ncon;  // [group_keys] members by root (component root, or world)
+    int2* gr_pos;                // [cap_arb + cap_joints] root and place of each arbiter and joint
+    int4* gr_part;               // [group_keys] first arbiter, joint and body of each root's members
+    GroupRec* gr_rec;            // [CLASSES * cap_bodies] the groups of each class
+    int *gr_arb, *gr_joint, *gr_body;  // members of each group
     // per-step scratch of the cache merge and the colour permutation (each world its own)
     int2* ev_created;            // [cap_arb] keys of the arbiters created this step
     int2* ev_removed;            // [cap_arb] keys of the arbiters removed this step
@@ -259,6 +299,7 @@ struct StepParams {
     int task_maxb;               // bodies a task may hold in the solver's shared memory
     float cells_per_sm;          // partition cells per grid and SM, before the span bound (0: chosen on the device)
     int solve_blocks;            // persistent blocks of the task solve (the default density rule)
+    int groups;                  // 1: independent parts may be solved one CTA each
 };
 
 // Partitioned-solve launch shape: threads per CTA and bytes of shared memory per
@@ -283,6 +324,8 @@ int  jg_launch_solve(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm, 
 void jg_launch_update(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
 void jg_launch_mlp_warmstart(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
 void jg_launch_islands(WorldDev& w, cudaStream_t s, int nsm);
+void jg_launch_groups(WorldDev& w, cudaStream_t s, int nsm);
+int  jg_group_launches(const WorldDev& w);
 
 // Arbiter mode word (ArbStore::info.y): SolveMode bits 0-3, and this bit when neither body
 // is an awake non-static body (the row is neither solved nor updated while it sleeps).

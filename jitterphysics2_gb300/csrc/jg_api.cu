@@ -266,12 +266,11 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     if (timed) cudaEventRecord(w->ev[0], s);
     k_reset_counters<<<1, 1, 0, s>>>(d.ctr);
     if (sp.record_residual) cudaMemsetAsync(d.resid, 0, sizeof(float) * 2 * JG_RESID_MAX, s);
-    jg_launch_aabb(d, sp.dt, s);
-    int passes = jg_launch_broadphase(d, s, w->nsm);
-    // kernels of this sequence: reset 1, aabb 2, broadphase 1 + 3 per radix pass + 4,
-    // narrowphase 3 + 5, merge 3 (+ warm-start hook), schedule, colour/permute 4, count 1,
+    w->launches = jg_launch_aabb(d, sp.dt, s);
+    w->launches += jg_launch_broadphase(d, s, w->nsm);
+    // the other kernels of this sequence: reset 1, narrowphase 3 + 5, merge 3 (+ warm-start hook), schedule, colour/permute 4, count 1,
     // solve 1, contact update 1, body update 1
-    w->launches = 1 + 2 + (d.ns >= 2 ? 5 + 3 * passes : 0) + 8 + 3 + 4 + 1 + 1 + 1 + 1 + jg_schedule_launches(sp);
+    w->launches += 1 + 8 + 3 + 4 + 1 + 1 + 1 + 1 + jg_schedule_launches(sp);
     if (timed) cudaEventRecord(w->ev[1], s);
     jg_launch_narrowphase(d, sp, s, w->nsm, w->prm.narrow_tile);
     if (timed) cudaEventRecord(w->ev[2], s);

@@ -1,6 +1,6 @@
 // Broadphase: world AABBs, a linear BVH rebuilt every step (Morton codes, an LSD radix
 // sort written here, Karras-style hierarchy, bottom-up refit) and one traversal per
-// dynamic shape that writes the pair list.
+// dynamic shape that writes the pair list; in small scenes every box against every box.
 //
 // Contract (the reference's, not its data structure): every shape pair on different
 // bodies of the same world whose exact world AABBs are not disjoint (touching counts),
@@ -22,6 +22,7 @@ __device__ __forceinline__ float ord2f(unsigned u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
+// `scene`: null when the pair search needs no bounds of the whole scene.
 __global__ void k_aabb(WorldDev w, unsigned* scene, float dt) {
     __shared__ unsigned smin[3], smax[3];
     if (threadIdx.x < 3) { smin[threadIdx.x] = 0xffffffffu; smax[threadIdx.x] = 0u; }
@@ -41,10 +42,12 @@ __global__ void k_aabb(WorldDev w, unsigned* scene, float dt) {
         }
         w.amin[i] = f4(mn, 0.f);
         w.amax[i] = f4(mx, 0.f);
+        if (!scene) continue;
         v3 c = 0.5f * (mn + mx);
         atomicMin(&smin[0], f2ord(c.x)); atomicMin(&smin[1], f2ord(c.y)); atomicMin(&smin[2], f2ord(c.z));
         atomicMax(&smax[0], f2ord(c.x)); atomicMax(&smax[1], f2ord(c.y)); atomicMax(&smax[2], f2ord(c.z));
     }
+    if (!scene) return;
     __syncthreads();
     if (threadIdx.x < 3) {
         atomicMin(&scene[threadIdx.x], smin[threadIdx.x]);
@@ -346,20 +349,104 @@ __global__ void k_traverse(WorldDev w, int n) {
     flush_pairs(w, buf, nbuf);
 }
 
+// ---- small scenes: every box against every box ---------------------------------------------
+// The tree costs a dozen and a half launches and a serial walk per shape, about 140 us for a thousand
+// shapes whose boxes fit in a few SMs' shared memory; n * n box tests take a few microseconds
+// up to several thousand shapes.  A block holds BR_TILE query shapes, one per thread, and runs
+// through its share of the shapes, a tile of them in shared memory at a time.  Whole broadphase,
+// tree and this: 28 shapes 113 and 17 us, 1,001 146 and 26, 6,600 316 and 85, 12,700 in 100
+// worlds 300 and 161, 26,000 340 and 457; the line (JG_BRUTE_MAXSHAPES) lies where they meet.
+constexpr int BR_TILE = 128;
+constexpr int BR_BUF = 1024;  // pairs a block gathers before it appends them to the list
+
+__global__ void __launch_bounds__(BR_TILE) k_pairs_brute(WorldDev w, int n) {
+    __shared__ float4 s_min[BR_TILE], s_max[BR_TILE];  // boxes, with the leaf word and the world
+    __shared__ int2 s_buf[BR_BUF];
+    __shared__ int s_n, s_base;
+    const int tid = threadIdx.x, sa = blockIdx.x * BR_TILE + tid;
+    int body = -1, word = 0, world = 0;
+    float4 qmn = make_float4(0.f, 0.f, 0.f, 0.f), qmx = qmn;
+    if (sa < n) {
+        word = leaf_word(w, sa);
+        body = word & LEAF_BODY;
+        world = w.binfo[body].z;
+        qmn = w.amin[sa]; qmx = w.amax[sa];
+    }
+    if (tid == 0) s_n = 0;
+    const bool query = sa < n && (word & LEAF_DYN);  // queries start from dynamic shapes only
+    const bool act_a = (word & LEAF_ACTIVE) != 0;
+    const int tiles = (n + BR_TILE - 1) / BR_TILE;
+    if (!__syncthreads_or(query)) return;
+    for (int t = blockIdx.y; t < tiles; t += gridDim.y) {
+        const int first = t * BR_TILE, sj = first + tid;
+        int lw = 0;
+        if (sj < n) {
+            lw = leaf_word(w, sj);
+            float4 mn = w.amin[sj], mx = w.amax[sj];
+            mn.w = __int_as_float(lw);
+            mx.w = __int_as_float(w.binfo[lw & LEAF_BODY].z);
+            s_min[tid] = mn; s_max[tid] = mx;
+        }
+        // below the block's own shapes only the non-dynamic ones are left to it
+        const bool any = __syncthreads_or(sj < n && (t >= (int)blockIdx.x || !(lw & LEAF_DYN)));
+        if (any) {
+            const int m = min(BR_TILE, n - first);
+            for (int k = 0; k < m; k++) {
+                const float4 bmn = s_min[k], bmx = s_max[k];
+                if (!query || !overlap(qmn, qmx, bmn, bmx)) continue;
+                const int sb = first + k, lf = __float_as_int(bmn.w);
+                if (sb == sa || (lf & LEAF_BODY) == body || __float_as_int(bmx.w) != world) continue;
+                if ((lf & LEAF_DYN) && sb < sa) continue;  // each dynamic pair once
+                if (!act_a && !(lf & LEAF_ACTIVE)) continue;
+                const int2 pr = make_int2(min(sa, sb), max(sa, sb));
+                const int at = atomicAdd(&s_n, 1);
+                if (at < BR_BUF) s_buf[at] = pr;
+                else {  // beyond the buffer: straight to the list
+                    const int g = atomicAdd(&w.ctr->npairs, 1);
+                    if (g < w.cap_pairs) w.pairs[g] = pr;
+                    else atomicCAS(&w.ctr->status, 0, JG_ERR_CAPACITY);
+                }
+            }
+        }
+        __syncthreads();
+        if (s_n >= BR_BUF / 2 || t + (int)gridDim.y >= tiles) {
+            const int got = min(s_n, BR_BUF);
+            if (tid == 0 && got) s_base = atomicAdd(&w.ctr->npairs, got);
+            __syncthreads();
+            for (int k = tid; k < got; k += BR_TILE) {
+                if (s_base + k < w.cap_pairs) w.pairs[s_base + k] = s_buf[k];
+                else atomicCAS(&w.ctr->status, 0, JG_ERR_CAPACITY);
+            }
+            __syncthreads();
+            if (tid == 0) s_n = 0;
+            __syncthreads();
+        }
+    }
+}
+
+bool brute(const WorldDev& w) { return w.ns <= JG_BRUTE_MAXSHAPES; }
+
 }  // namespace
 
-void jg_launch_aabb(WorldDev& w, float dt, cudaStream_t s) {
-    if (w.ns == 0) return;
-    k_scene_init<<<1, 32, 0, s>>>((unsigned*)w.scene_box);
+int jg_launch_aabb(WorldDev& w, float dt, cudaStream_t s) {
+    if (w.ns == 0) return 0;
+    unsigned* scene = brute(w) ? nullptr : (unsigned*)w.scene_box;
+    if (scene) k_scene_init<<<1, 32, 0, s>>>(scene);
     int blocks = (w.ns + 255) / 256;
     if (blocks > 1024) blocks = 1024;
-    k_aabb<<<blocks, 256, 0, s>>>(w, (unsigned*)w.scene_box, dt);
+    k_aabb<<<blocks, 256, 0, s>>>(w, scene, dt);
+    return scene ? 2 : 1;
 }
 
 int jg_launch_broadphase(WorldDev& w, cudaStream_t s, int nsm) {
-    (void)nsm;
     int n = w.ns;
     if (n < 2) return 0;
+    if (brute(w)) {
+        const int tiles = (n + BR_TILE - 1) / BR_TILE;
+        const int split = max(1, min(tiles, nsm * 8 / tiles));  // several blocks an SM
+        k_pairs_brute<<<dim3(tiles, split), BR_TILE, 0, s>>>(w, n);
+        return 1;
+    }
     k_morton<<<(n + 255) / 256, 256, 0, s>>>(w, (const unsigned*)w.scene_box);
     int bits = 30;
     int wb = 0;
@@ -387,5 +474,5 @@ int jg_launch_broadphase(WorldDev& w, cudaStream_t s, int nsm) {
     k_build<<<(n + 255) / 256, 256, 0, s>>>(w, n);
     k_refit<<<(n + 255) / 256, 256, 0, s>>>(w, n);
     k_traverse<<<(n + 127) / 128, 128, 0, s>>>(w, n);
-    return passes;
+    return 5 + 3 * passes;
 }

@@ -14,6 +14,7 @@
 
 #define JG_MAX_COLORS 128
 #define JG_RESID_MAX 2048       // iterations whose residual a step records (record_residual)
+#define JG_BRUTE_MAXSHAPES 16384 // shapes up to which the pair search tests every box against every box
 #define JG_HULL_MAX 64          // point-cloud vertices per shape handled on the device
 #define JG_EPA_MAXV 128         // EPA polytope capacity (ConvexPolytope.cs:53-54)
 #define JG_EPA_MAXT 256
@@ -314,7 +315,8 @@ struct StepParams {
 int jg_solver_task_maxb(int block, int ctas_per_sm);
 
 // ---- stage launchers (each defined in its own translation unit) ------------------------
-void jg_launch_aabb(WorldDev& w, float dt, cudaStream_t s);
+// (both return the kernels they launch)
+int  jg_launch_aabb(WorldDev& w, float dt, cudaStream_t s);
 int  jg_launch_broadphase(WorldDev& w, cudaStream_t s, int nsm);
 void jg_launch_narrowphase(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm, int tile);
 void jg_launch_merge(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);

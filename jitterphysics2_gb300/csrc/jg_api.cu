@@ -14,7 +14,6 @@
 #include <climits>
 
 void jg_flip_store(WorldDev& w);
-void jg_launch_count_contacts(WorldDev& w, cudaStream_t s, int nsm);
 void jg_launch_update_contacts(WorldDev& w, cudaStream_t s, int nsm);
 void jg_solver_reset_launch_cache(WorldDev& w);
 void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
@@ -142,7 +141,7 @@ int allocate(jg_world* w) {
     DA(d.bmask, 2 * (size_t)d.cap_bodies);
     DA(d.adj_off, d.cap_bodies + 1);
     DA(d.adj, 2 * ((size_t)d.cap_arb + d.cap_joints));
-    DA(d.deg, d.cap_bodies);
+    DA(d.deg, d.cap_bodies); DA(d.cprio, d.cap_arb + d.cap_joints);
     DA(d.color_count, JG_MAX_COLORS + 1); DA(d.color_start, JG_MAX_COLORS + 1); DA(d.jcolor_start, JG_MAX_COLORS + 1);
     DA(d.color_cursor, JG_MAX_COLORS + 1);
     DA(d.jorder, d.cap_joints + JG_MAX_COLORS);
@@ -268,9 +267,9 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     if (sp.record_residual) cudaMemsetAsync(d.resid, 0, sizeof(float) * 2 * JG_RESID_MAX, s);
     w->launches = jg_launch_aabb(d, sp.dt, s);
     w->launches += jg_launch_broadphase(d, s, w->nsm);
-    // the other kernels of this sequence: reset 1, narrowphase 3 + 5, merge 3 (+ warm-start hook), schedule, colour/permute 4, count 1,
-    // solve 1, contact update 1, body update 1
-    w->launches += 1 + 8 + 3 + 4 + 1 + 1 + 1 + 1 + jg_schedule_launches(sp);
+    // the other kernels of this sequence: reset 1, narrowphase 3 + 5, merge 3 (+ warm-start
+    // hook), schedule, colour and permute 2, solve 1, contact update 1, body update 1
+    w->launches += 1 + 8 + 3 + 2 + 1 + 1 + 1 + jg_schedule_launches(sp);
     if (timed) cudaEventRecord(w->ev[1], s);
     jg_launch_narrowphase(d, sp, s, w->nsm, w->prm.narrow_tile);
     if (timed) cudaEventRecord(w->ev[2], s);
@@ -289,7 +288,6 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     }
     jg_flip_store(d);
     if (timed) cudaEventRecord(w->ev[4], s);
-    jg_launch_count_contacts(d, s, w->nsm);
     if (sp.groups) {
         jg_launch_groups(d, s, w->nsm);
         jg_launch_solve_groups(d, sp, s, w->nsm);
@@ -980,7 +978,6 @@ int jg_stabilize(jg_world* w, float dt, int32_t iterations, int32_t relax) {
     jg_launch_schedule(d, sp, s, w->nsm);
     if (jg_launch_color(d, s, w->nsm) < 0) { g_err = "cooperative launch of the colouring failed"; return JG_ERR_CUDA; }
     jg_flip_store(d);
-    jg_launch_count_contacts(d, s, w->nsm);
     if (jg_launch_solve(d, sp, s, w->nsm, w->prm.solver_block, w->prm.solver_ctas_per_sm) < 0) {
         g_err = "cooperative launch of the solver failed";
         return JG_ERR_CUDA;

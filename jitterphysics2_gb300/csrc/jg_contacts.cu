@@ -202,9 +202,6 @@ __global__ void k_merge(WorldDev w, StepParams sp, int2* ev_created) {
 // ---- colouring -----------------------------------------------------------------------------
 __device__ __forceinline__ unsigned prio(unsigned long long key) { return hash64(key * 0x9E3779B97F4A7C15ull + 1); }
 
-struct ColorCtx {
-    int narb, nj, ncons;
-};
 __device__ __forceinline__ void cons_bodies(const WorldDev& w, const ArbStore& A, int c, int narb, int& b1, int& b2,
                                             unsigned long long& key) {
     if (c < narb) {
@@ -220,73 +217,62 @@ __device__ __forceinline__ void cons_bodies(const WorldDev& w, const ArbStore& A
     if (w.binfo[b2].x != JG_MOTION_DYNAMIC) b2 = -1;
 }
 
-// Persistent cooperative kernel: adjacency build, Jones-Plassmann rounds, colour counts.
-__global__ void k_color(WorldDev w, int* remaining) {
+// Colours of the remainder (arbiters outside the tasks, and all joints), cooperative: adjacency
+// build, Jones-Plassmann, colour counts.  A constraint takes the smallest colour free on its
+// bodies once every neighbour of higher priority has one (no neighbour of lower priority can
+// come before it), so the colours do not depend on the timing, and each thread simply
+// looks at its own constraints again until they are coloured: no barrier per round.  Without a
+// remainder the kernel only marks the arbiters, with no barrier at all.  (27 boxes: 54 -> 3 us;
+// the joints of 1024 chains 197 -> 121.)
+__global__ void k_color(WorldDev w) {
     const ArbStore& A = w.arb[w.cur];
     const int narb = w.ctr->narb < w.cap_arb ? w.ctr->narb : w.cap_arb;
     const int nj = w.nj;
     const int ncons = narb + nj;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     int* status = &w.ctr->status;
-    __shared__ int s_warp[32];
+    const bool tasks = w.sc->ntasks > 0;
+    const int first = tasks ? w.sc->narb_task : 0;  // the remainder follows the tasks
+    const int lo = w.sc->nrem ? 0 : narb;  // (without a remainder of arbiters, the joints alone)
+    for (int c = tid; c < JG_MAX_COLORS; c += nth) w.jorder[w.cap_joints + c] = 0;
+    if (nj == 0 && w.sc->nrem == 0) {
+        for (int c = tid; c < narb; c += nth) w.cstat[c] = (A.info[c].x & 15) == 0 ? -2 : -4;
+        for (int c = tid; c <= JG_MAX_COLORS; c += nth) {
+            w.color_start[c] = first;
+            w.jcolor_start[c] = 0;
+            w.color_cursor[c] = 0;
+        }
+        if (tid == 0) { w.ctr->ncolors = 0; w.remaining[0] = 0; }
+        return;
+    }
     for (int b = tid; b < w.nb; b += nth) { w.deg[b] = 0; w.bmask[2 * b] = 0ull; w.bmask[2 * b + 1] = 0ull; }
     for (int c = tid; c < JG_MAX_COLORS + 1; c += nth) { w.color_count[c] = 0; w.color_cursor[c] = 0; }
-    if (tid < 2) remaining[tid] = 0;
+    if (tid < 2) w.remaining[tid] = 0;
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    const bool tasks = w.sc->ntasks > 0;
     for (int c = tid; c < ncons; c += nth) {
         if (c < narb && (A.info[c].x & 15) == 0) { w.cstat[c] = -2; continue; }
         if (c < narb && tasks && w.sc_dst[c] >= 0) { w.cstat[c] = -4; continue; }  // solved in a task
         int b1, b2; unsigned long long key;
         cons_bodies(w, A, c, narb, b1, b2, key);
         w.cstat[c] = -1;
+        w.cprio[c] = prio(key);
         if (b1 >= 0) atomicAdd(&w.deg[b1], 1);
         if (b2 >= 0 && b2 != b1) atomicAdd(&w.deg[b2], 1);
     }
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    // exclusive scan of deg -> adj_off: per-block chunk scan, then block offsets
-    {
-        int chunk = (w.nb + gridDim.x - 1) / gridDim.x;
-        int lo = blockIdx.x * chunk, hi = min(w.nb, lo + chunk);
-        // block-local scan of [lo, hi) in passes of blockDim
-        int carry = 0;
-        for (int base = lo; base < hi; base += blockDim.x) {
-            int i = base + threadIdx.x;
-            int v = i < hi ? w.deg[i] : 0;
-            int x = v;
-            for (int o = 1; o < 32; o <<= 1) { int y = __shfl_up_sync(0xffffffffu, x, o); if ((threadIdx.x & 31) >= o) x += y; }
-            if ((threadIdx.x & 31) == 31) s_warp[threadIdx.x >> 5] = x;
-            __syncthreads();
-            if (threadIdx.x < 32) {
-                int s = threadIdx.x < (int)(blockDim.x >> 5) ? s_warp[threadIdx.x] : 0;
-                for (int o = 1; o < 32; o <<= 1) { int y = __shfl_up_sync(0xffffffffu, s, o); if ((int)threadIdx.x >= o) s += y; }
-                s_warp[threadIdx.x] = s;
-            }
-            __syncthreads();
-            int wp = (threadIdx.x >= 32) ? s_warp[(threadIdx.x >> 5) - 1] : 0;
-            if (i < hi) w.adj_off[i] = carry + wp + x - v;
-            int tot = s_warp[(blockDim.x >> 5) - 1];
-            __syncthreads();
-            carry += tot;
-        }
-        if (threadIdx.x == 0) w.hist[blockIdx.x] = carry;
+    // space for each body's list, in any order
+    for (int base = blockIdx.x * blockDim.x; base < w.nb; base += nth) {
+        const int i = base + threadIdx.x, lane = threadIdx.x & 31;
+        const int v = i < w.nb ? w.deg[i] : 0;
+        int x = v;
+        for (int o = 1; o < 32; o <<= 1) { int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+        int off = 0;
+        if (lane == 31 && x) off = atomicAdd(&w.remaining[1], x);
+        off = __shfl_sync(0xffffffffu, off, 31);
+        if (i < w.nb) { w.adj_off[i] = off + x - v; w.deg[i] = 0; }
     }
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int acc = 0;
-        for (int b = 0; b < (int)gridDim.x; b++) { int t = w.hist[b]; w.hist[b] = acc; acc += t; }
-        w.hist[gridDim.x] = acc;
-    }
-    if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    {
-        int chunk = (w.nb + gridDim.x - 1) / gridDim.x;
-        int lo = blockIdx.x * chunk, hi = min(w.nb, lo + chunk);
-        int off = w.hist[blockIdx.x];
-        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) { w.adj_off[i] += off; w.deg[i] = 0; }
-        if (blockIdx.x == 0 && threadIdx.x == 0) w.adj_off[w.nb] = w.hist[gridDim.x];
-    }
-    if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    for (int c = tid; c < ncons; c += nth) {
+    for (int c = lo + tid; c < ncons; c += nth) {
         if (w.cstat[c] < -1) continue;
         int b1, b2; unsigned long long key;
         cons_bodies(w, A, c, narb, b1, b2, key);
@@ -294,180 +280,197 @@ __global__ void k_color(WorldDev w, int* remaining) {
         if (b2 >= 0 && b2 != b1) { int s = atomicAdd(&w.deg[b2], 1); w.adj[w.adj_off[b2] + s] = c; }
     }
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    // Jones-Plassmann rounds; cstat = round * 256 + colour once coloured
-    for (int round = 1; round < 4096; round++) {
-        int left = 0;
-        for (int c = tid; c < ncons; c += nth) {
-            int st = w.cstat[c];
-            if (st != -1) continue;
+    // cstat = colour once coloured; every thread of the launch is resident, and the highest
+    // uncoloured priority can always take its colour, so the looking ends
+    const unsigned long long t0 = globaltimer_ns();
+    unsigned idle = 0;
+    for (bool pending = true; pending;) {
+        pending = false;
+        bool progress = false;
+        for (int c = lo + tid; c < ncons; c += nth) {
+            if (w.cstat[c] != -1) continue;
             int b1, b2; unsigned long long key;
             cons_bodies(w, A, c, narb, b1, b2, key);
-            unsigned pc = prio(key);
-            bool is_max = true;
-            for (int side = 0; side < 2 && is_max; side++) {
-                int b = side == 0 ? b1 : b2;
+            const unsigned pc = w.cprio[c];
+            bool ready = true;
+            for (int side = 0; side < 2 && ready; side++) {
+                const int b = side == 0 ? b1 : b2;
                 if (b < 0) continue;
-                int beg = w.adj_off[b], end = w.adj_off[b + 1];
+                const int beg = w.adj_off[b], end = beg + w.deg[b];
                 for (int e = beg; e < end; e++) {
-                    int n = w.adj[e];
-                    if (n == c) continue;
-                    int sn = w.cstat[n];
-                    bool unc = sn == -1 || (sn >= 0 && (sn >> 8) == round);
-                    if (!unc) continue;
-                    int nb1, nb2; unsigned long long nk;
-                    cons_bodies(w, A, n, narb, nb1, nb2, nk);
-                    unsigned pn = prio(nk);
-                    if (pn > pc || (pn == pc && n > c)) { is_max = false; break; }
+                    const int n = w.adj[e];
+                    if (n == c || ld_relaxed_int(&w.cstat[n]) != -1) continue;
+                    const unsigned pn = w.cprio[n];
+                    if (pn > pc || (pn == pc && n > c)) { ready = false; break; }
                 }
             }
-            if (!is_max) { left++; continue; }
+            if (!ready) { pending = true; continue; }
+            __threadfence();  // the neighbours' colours before the masks they set
             unsigned long long m0 = 0, m1 = 0;
-            if (b1 >= 0) { m0 |= w.bmask[2 * b1]; m1 |= w.bmask[2 * b1 + 1]; }
-            if (b2 >= 0) { m0 |= w.bmask[2 * b2]; m1 |= w.bmask[2 * b2 + 1]; }
+            if (b1 >= 0) { m0 |= __ldcg(&w.bmask[2 * b1]); m1 |= __ldcg(&w.bmask[2 * b1 + 1]); }
+            if (b2 >= 0) { m0 |= __ldcg(&w.bmask[2 * b2]); m1 |= __ldcg(&w.bmask[2 * b2 + 1]); }
             int color;
             if (~m0) color = __ffsll((long long)~m0) - 1;
             else if (~m1) color = 64 + __ffsll((long long)~m1) - 1;
             else { atomicCAS(status, 0, JG_ERR_CAPACITY); color = JG_MAX_COLORS - 1; }
-            if (color >= JG_MAX_COLORS) { atomicCAS(status, 0, JG_ERR_CAPACITY); color = JG_MAX_COLORS - 1; }
-            unsigned long long bit0 = color < 64 ? (1ull << color) : 0ull, bit1 = color >= 64 ? (1ull << (color - 64)) : 0ull;
-            if (b1 >= 0) { if (bit0) atomicOr(&w.bmask[2 * b1], bit0); if (bit1) atomicOr(&w.bmask[2 * b1 + 1], bit1); }
-            if (b2 >= 0) { if (bit0) atomicOr(&w.bmask[2 * b2], bit0); if (bit1) atomicOr(&w.bmask[2 * b2 + 1], bit1); }
-            w.cstat[c] = round * 256 + color;
+            unsigned long long* word = &w.bmask[color >> 6];
+            const unsigned long long bit = 1ull << (color & 63);
+            if (b1 >= 0) atomicOr(word + 2 * b1, bit);
+            if (b2 >= 0) atomicOr(word + 2 * b2, bit);
+            __threadfence();
+            *(volatile int*)&w.cstat[c] = color;
+            progress = true;
         }
-        for (int o = 16; o > 0; o >>= 1) left += __shfl_xor_sync(0xffffffffu, left, o);
-        if ((threadIdx.x & 31) == 0 && left) atomicAdd(&remaining[round & 1], left);
-        if (tid == 0) remaining[(round + 1) & 1] = 0;
-        if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-        int rem = ld_relaxed_int(&remaining[round & 1]);
-        if (tid == 0) w.ctr->color_rounds = round;
-        if (rem == 0) break;
-        if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    }
-    for (int c = tid; c < ncons; c += nth) {
-        int st = w.cstat[c];
-        if (st < 0) continue;
-        int col = st & 255;
-        if (c < narb) atomicAdd(&w.color_count[col], 1);
-        else atomicAdd(&w.color_cursor[col], 1);   // joint counts (cursor reset before use)
-    }
-    if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int acc = tasks ? w.sc->narb_task : 0, jacc = 0, nc = 0;  // the remainder follows the tasks
-        for (int c = 0; c < JG_MAX_COLORS; c++) {
-            int t = w.color_count[c], jt = w.color_cursor[c];
-            if (t || jt) nc = c + 1;
-            w.color_start[c] = acc; acc += t;
-            w.jcolor_start[c] = jacc; jacc += jt;
+        if (!pending || progress) continue;
+        if ((++idle & 63) == 0) {
+            if (ld_relaxed_int(status) == JG_ERR_TIMEOUT) break;
+            if (globaltimer_ns() - t0 > 1000000000ull) { atomicCAS(status, 0, JG_ERR_TIMEOUT); break; }
         }
+        __nanosleep(40);
+    }
+    // colour counts (joint counts in the cursor, reset before use); the last block to finish
+    // turns them into first places
+    for (int c = lo + tid; c < ncons; c += nth) {
+        const int col = w.cstat[c];
+        if (col < 0) continue;
+        int* counter = c < narb ? &w.color_count[col] : &w.color_cursor[col];
+        const unsigned act = __activemask(), same = __match_any_sync(act, (unsigned long long)counter);
+        if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(counter, __popc(same));
+    }
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&w.remaining[0], 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last || threadIdx.x >= 32) return;
+    __threadfence();
+    int acc = first, jacc = 0, nc = 0;
+    for (int base = 0; base < JG_MAX_COLORS; base += 32) {
+        const int c = base + threadIdx.x;
+        const int t = __ldcg(&w.color_count[c]), jt = __ldcg(&w.color_cursor[c]);
+        int x = t, y = jt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int px = __shfl_up_sync(0xffffffffu, x, o), py = __shfl_up_sync(0xffffffffu, y, o);
+            if ((int)threadIdx.x >= o) { x += px; y += py; }
+        }
+        const unsigned used = __ballot_sync(0xffffffffu, t || jt);
+        if (used) nc = base + 32 - __clz(used);
+        w.color_start[c] = acc + x - t;
+        w.jcolor_start[c] = jacc + y - jt;
+        w.color_cursor[c] = 0;
+        acc += __shfl_sync(0xffffffffu, x, 31);
+        jacc += __shfl_sync(0xffffffffu, y, 31);
+    }
+    if (threadIdx.x == 0) {
         w.color_start[JG_MAX_COLORS] = acc;
         w.jcolor_start[JG_MAX_COLORS] = jacc;
-        for (int c = nc; c < JG_MAX_COLORS; c++) { w.color_start[c] = acc; w.jcolor_start[c] = jacc; }
+        w.color_cursor[JG_MAX_COLORS] = 0;
         w.ctr->ncolors = nc;
-        for (int c = 0; c <= JG_MAX_COLORS; c++) w.color_cursor[c] = 0;
+        w.remaining[0] = 0;
     }
 }
 
-// Moves every arbiter with contacts to the other buffer at its colour slot.
+// Moves every arbiter with contacts to the other buffer at its colour slot, four lanes per
+// arbiter, one for each contact slot (a lane that copied them one after another waited for
+// memory four times: 22 -> 9 us at a thousand arbiters).  Counts the contacts on the way; the
+// last block sets the new arbiter count.
 __global__ void k_permute(WorldDev w, int2* ev_removed, int* dst_index) {
     const ArbStore& S = w.arb[w.cur];
     const ArbStore& D = w.arb[1 - w.cur];
     const int narb = w.ctr->narb < w.cap_arb ? w.ctr->narb : w.cap_arb;
     const int cap = w.cap_arb;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < narb; a += gridDim.x * blockDim.x) {
-        int st = w.cstat[a];
-        int d, key;
-        int4 ls;
-        if (st == -4) {  // task arbiter: slot, order key and body slots from the schedule
-            d = w.sc_dst[a];
-            key = w.sc_lcol[a];
-            ls = w.sc_ls[a];
-        } else if (st < 0) {
-            int e = atomicAdd(&w.ctr->nremoved, 1);
-            if (e < cap) ev_removed[e] = S.key[a];
-            dst_index[a] = -1;
-            if (w.allow_deact) {  // RemoveBrokenArbiters: AddToActiveList on both islands (World.Step.cs:845-846)
-                int2 bb = S.body[a];
-                atomicOr(&w.binfo[bb.x].w, 3);
-                atomicOr(&w.binfo[bb.y].w, 3);
+    const int k = threadIdx.x & 3;
+    int contacts = 0;
+    for (int base = blockIdx.x * blockDim.x; base < 4 * narb; base += gridDim.x * blockDim.x) {
+        const int a = (base + (int)threadIdx.x) >> 2;
+        const bool live = a < narb;
+        const int st = live ? w.cstat[a] : -2;
+        int4 info = make_int4(0, 0, 0, 0);
+        int2 bb = make_int2(0, 0);
+        if (live) { info = S.info[a]; bb = S.body[a]; }
+        int d = -1;
+        if (live && k == 0) {
+            if (st == -4) d = w.sc_dst[a];
+            else if (st >= 0) d = w.color_start[st] + atomicAdd(&w.color_cursor[st], 1);
+            else {
+                int e = atomicAdd(&w.ctr->nremoved, 1);
+                if (e < cap) ev_removed[e] = S.key[a];
+                if (w.allow_deact) {  // RemoveBrokenArbiters: AddToActiveList on both islands (World.Step.cs:845-846)
+                    atomicOr(&w.binfo[bb.x].w, 3);
+                    atomicOr(&w.binfo[bb.y].w, 3);
+                }
             }
-            continue;
-        } else {
-            int col = st & 255;
-            d = w.color_start[col] + atomicAdd(&w.color_cursor[col], 1);
-            key = JG_ORDER_REMAINDER + col;
-            ls = make_int4(-1, -1, 3, 0);
+            dst_index[a] = d;
         }
-        dst_index[a] = d;
-        int4 info = S.info[a];
-        int2 bb = S.body[a];
+        d = __shfl_sync(0xffffffffu, d, 0, 4);
+        if (d < 0) continue;
+        if (info.x & (1 << k)) {
+            const int s = k * cap + a, t = k * cap + d;
+            const float4 cn = S.cn[s], t1 = S.ct1[s], t2 = S.ct2[s], r1 = S.cr1[s], r2 = S.cr2[s], ac = S.cacc[s], p1 = S.cp1[s],
+                         p2 = S.cp2[s];
+            D.cn[t] = cn; D.ct1[t] = t1; D.ct2[t] = t2; D.cr1[t] = r1; D.cr2[t] = r2; D.cacc[t] = ac; D.cp1[t] = p1; D.cp2[t] = p2;
+            contacts++;
+        }
+        if (k != 0) continue;
+        const int4 i1 = w.binfo[bb.x], i2 = w.binfo[bb.y];
         // a row is solved and updated while one of its bodies is an awake non-static body
         // (memContacts activation follows the bodies, World.Step.cs:1247-1275, :1325-1345)
-        bool asleep = false;
-        if (w.allow_deact) {
-            int4 i1 = w.binfo[bb.x], i2 = w.binfo[bb.y];
-            asleep = !((i1.x != JG_MOTION_STATIC && (i1.y & JG_BODY_ACTIVE)) || (i2.x != JG_MOTION_STATIC && (i2.y & JG_BODY_ACTIVE)));
-        }
+        const bool asleep = w.allow_deact && !((i1.x != JG_MOTION_STATIC && (i1.y & JG_BODY_ACTIVE)) ||
+                                               (i2.x != JG_MOTION_STATIC && (i2.y & JG_BODY_ACTIVE)));
+        const float4 mat = S.mat[a];
         D.key[d] = S.key[a];
         D.body[d] = bb;
-        D.info[d] = make_int4(info.x, (info.y & 0xffff) | (asleep ? JG_ARB_ASLEEP : 0), key, info.w);
+        D.info[d] = make_int4(info.x, (info.y & 0xffff) | (asleep ? JG_ARB_ASLEEP : 0), st == -4 ? w.sc_lcol[a] : JG_ORDER_REMAINDER + st,
+                              info.w);
         // velocities of a non-dynamic body stay constant through the solve
-        int nd = w.binfo[bb.x].x != JG_MOTION_DYNAMIC ? bb.x : (w.binfo[bb.y].x != JG_MOTION_DYNAMIC ? bb.y : -1);
-        // task arbiters: what the iterations read besides the rows, in one record
-        if (st == -4) ls = make_int4(ls.x, ls.y, (info.x & 15) | ((info.y & 15) << 4) | (nd >= 0 ? 256 : 0) | (asleep ? JG_TASK_ASLEEP : 0),
-                                     __float_as_int(S.mat[a].x));
+        const int nd = i1.x != JG_MOTION_DYNAMIC ? bb.x : (i2.x != JG_MOTION_DYNAMIC ? bb.y : -1);
+        int4 ls = make_int4(-1, -1, 3, 0);
+        if (st == -4) {  // task arbiters: body slots, and what the iterations read besides the rows, in one record
+            ls = w.sc_ls[a];
+            ls.z = (info.x & 15) | ((info.y & 15) << 4) | (nd >= 0 ? 256 : 0) | (asleep ? JG_TASK_ASLEEP : 0);
+            ls.w = __float_as_int(mat.x);
+        }
         D.lslot[d] = ls;
         D.sv[d] = nd >= 0 ? w.body[nd].v : make_float4(0.f, 0.f, 0.f, 0.f);
         D.sv[cap + d] = nd >= 0 ? w.body[nd].w : make_float4(0.f, 0.f, 0.f, 0.f);
-        D.mat[d] = S.mat[a];
-        for (int k = 0; k < 4; k++) {
-            if (!(info.x & (1 << k))) continue;
-            int s = k * cap + a, t = k * cap + d;
-            D.cn[t] = S.cn[s]; D.ct1[t] = S.ct1[s]; D.ct2[t] = S.ct2[s]; D.cr1[t] = S.cr1[s];
-            D.cr2[t] = S.cr2[s]; D.cacc[t] = S.cacc[s]; D.cp1[t] = S.cp1[s]; D.cp2[t] = S.cp2[s];
-        }
+        D.mat[d] = mat;
     }
     const int nj = w.nj;
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nj; j += gridDim.x * blockDim.x) {
-        int st = w.cstat[narb + j];
-        int col = st >= 0 ? (st & 255) : 0;
+        const int st = w.cstat[narb + j];
+        const int col = st >= 0 ? st : 0;
         int d = w.jcolor_start[col] + atomicAdd(&w.jorder[w.cap_joints + col], 1);
         w.jorder[d] = j;
         w.joints[j].hdr.w = JG_ORDER_REMAINDER + col;
     }
-}
-
-__global__ void k_permute_done(WorldDev w) {
-    w.ctr->narb = w.color_start[JG_MAX_COLORS];
-}
-
-__global__ void k_count_contacts(WorldDev w) {
-    const ArbStore& A = w.arb[w.cur];
-    int n = w.ctr->narb;
-    int c = 0;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) c += __popc(A.info[a].x & 15);
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&w.ctr->contacts, c);
-}
-
-__global__ void k_jcursor_clear(WorldDev w) {
-    for (int c = threadIdx.x; c < JG_MAX_COLORS; c += blockDim.x) w.jorder[w.cap_joints + c] = 0;
+    contacts = __reduce_add_sync(0xffffffffu, contacts);
+    if ((threadIdx.x & 31) == 0 && contacts) atomicAdd(&w.ctr->contacts, contacts);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&w.remaining[0], 1) == (int)gridDim.x - 1) w.ctr->narb = w.color_start[JG_MAX_COLORS];
+    }
 }
 
 // ContactData.UpdatePosition (Contact.cs:238-264) / Contact.UpdatePosition (Contact.cs:762-797)
+// Four lanes per arbiter, one for each contact slot.
 __global__ void k_update_contacts(WorldDev w) {
     const ArbStore& A = w.arb[w.cur];
     const int n = w.ctr->narb, cap = w.cap_arb;
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-        int4 info = A.info[a];
-        if (info.y & JG_ARB_ASLEEP) continue;  // sleeping contacts keep their points
-        int usage = info.x & 15;
-        usage |= usage << 4;
-        int2 b = A.body[a];
-        v3 pos1 = mk3(w.pos[b.x]), pos2 = mk3(w.pos[b.y]);
-        q4 q1 = mkq(w.q[b.x]), q2 = mkq(w.q[b.y]);
-        for (int k = 0; k < 4; k++) {
-            if (!(usage & (1 << k))) continue;
-            int i = k * cap + a;
+    const int k = threadIdx.x & 3;
+    for (int base = blockIdx.x * blockDim.x; base < 4 * n; base += gridDim.x * blockDim.x) {
+        const int a = (base + (int)threadIdx.x) >> 2;
+        int4 info = make_int4(0, JG_ARB_ASLEEP, 0, 0);
+        if (a < n) info = A.info[a];
+        const bool awake = !(info.y & JG_ARB_ASLEEP);  // sleeping contacts keep their points
+        bool keep = true;
+        if (awake && (info.x & (1 << k))) {
+            const int i = k * cap + a;
+            int2 b = A.body[a];
+            v3 pos1 = mk3(w.pos[b.x]), pos2 = mk3(w.pos[b.y]);
+            q4 q1 = mkq(w.q[b.x]), q2 = mkq(w.q[b.y]);
             v3 rel1 = rotate(mk3(A.cp1[i]), q1);
             v3 p1 = rel1 + pos1;
             v3 rel2 = rotate(mk3(A.cp2[i]), q2);
@@ -478,15 +481,17 @@ __global__ void k_update_contacts(WorldDev w) {
             v3 dist = p1 - p2;
             v3 nrm = mk3(A.cn[i]);
             float pen = dot(dist, nrm);
-            bool keep = true;
             if (pen < -BreakThreshold * 0.1f) keep = false;
             else {
                 dist = dist - pen * nrm;
                 if (len2(dist) > BreakThreshold * BreakThreshold) keep = false;
             }
-            if (!keep) usage &= ~(1 << k);
         }
-        A.info[a] = make_int4(usage, info.y, info.z, 0);
+        const unsigned broken = (__ballot_sync(0xffffffffu, !keep) >> (threadIdx.x & 28)) & 15u;
+        if (awake && k == 0) {
+            const int usage = info.x & 15;
+            A.info[a] = make_int4((usage | (usage << 4)) & ~(int)broken, info.y, info.z, 0);
+        }
     }
 }
 
@@ -508,21 +513,14 @@ int jg_launch_color(WorldDev& w, cudaStream_t s, int nsm) {
         w.lc_color_grid = nsm * (occ < 2 ? occ : 2);
     }
     cudaMemsetAsync(w.bar_count, 0, sizeof(unsigned) * 2, s);
-    int* rem = w.remaining;
-    void* args[] = {(void*)&w, (void*)&rem};
+    void* args[] = {(void*)&w};
     cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_color, dim3(w.lc_color_grid), dim3(256), args, 0, s);
     if (e != cudaSuccess) return -1;
-    k_jcursor_clear<<<1, 128, 0, s>>>(w);
     k_permute<<<nsm * 4, 256, 0, s>>>(w, w.ev_removed, w.dst_index);
-    k_permute_done<<<1, 1, 0, s>>>(w);
     return 0;
 }
 
 void jg_flip_store(WorldDev& w) { w.cur = 1 - w.cur; }
-
-void jg_launch_count_contacts(WorldDev& w, cudaStream_t s, int nsm) {
-    k_count_contacts<<<nsm * 2, 256, 0, s>>>(w);
-}
 
 void jg_launch_update_contacts(WorldDev& w, cudaStream_t s, int nsm) {
     k_update_contacts<<<nsm * 4, 256, 0, s>>>(w);

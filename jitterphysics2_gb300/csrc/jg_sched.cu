@@ -44,8 +44,9 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
     return x;
 }
 
-__global__ void k_sched_reset(WorldDev w) {
+__global__ void k_sched_reset(WorldDev w, int partition) {
     SchedInfo* S = w.sc;
+    S->nrem = partition ? 0 : 1;
     S->span_bits = 0;
     S->bbox[0] = S->bbox[1] = 0xffffffffu;
     S->bbox[2] = S->bbox[3] = 0u;
@@ -267,9 +268,10 @@ __global__ void k_sched_scatter(WorldDev w) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     for (int a = tid; a < narb; a += nth) {
         int2 ga = w.sc_arb[a];
-        if (ga.x < 0 || ga.x >= JG_SCHED_GRIDS) continue;
+        if (ga.x < 0) continue;
+        if (ga.x >= JG_SCHED_GRIDS) { w.sc->nrem = 1; continue; }
         int t = w.sc_task_of[ga.x * JG_SCHED_MAXCELLS + ga.y];
-        if (t < 0) { w.sc_arb[a] = make_int2(3, -1); continue; }
+        if (t < 0) { w.sc_arb[a] = make_int2(3, -1); w.sc->nrem = 1; continue; }
         int p = atomicAdd(&w.sc_cursor[t], 1);
         w.sc_tlist[w.sc_task[t].x + p] = a;
     }
@@ -461,7 +463,7 @@ size_t jg_task_color_smem(int maxb) {
 }
 
 void jg_launch_schedule(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
-    k_sched_reset<<<1, 1, 0, s>>>(w);
+    k_sched_reset<<<1, 1, 0, s>>>(w, p.partition);
     if (p.partition) {
         k_sched_bounds<<<nsm * 4, 256, 0, s>>>(w);
         k_sched_setup<<<1, 1, 0, s>>>(w, nsm, p.cells_per_sm, p.solve_blocks);

@@ -62,7 +62,8 @@ struct SchedInfo {
     int tag;                         // step counter for the body claim stamps
     int overflow;                    // cells pushed to the remainder (too large)
     int maxc;                        // most local colours of any task
-    int pad[3];
+    int nrem;                        // nonzero: some arbiters are outside the tasks
+    int pad[2];
 };
 
 struct ArbStore {
@@ -114,7 +115,6 @@ struct DevCounters {
     int points;       // manifold points written
     int contacts;     // active contact points after the merge
     int new_contacts;
-    int color_rounds;
     int ncol;         // overlapping pairs found by the MPR stage
     int nepa_list;    // of those, deeper than the EPA threshold
     int nedge;        // of those, near a mesh edge (triangle-edge filter)
@@ -125,7 +125,7 @@ struct DevCounters {
     int edge_next;
     int nspec;        // speculative sweep candidates, and of those the pairs registered
     int nspec_hit;
-    int pad[1];
+    int pad[2];
 };
 
 // Solve groups (jg_groups.cu): independent parts of the step's constraint graph, one CTA each.
@@ -213,8 +213,9 @@ struct WorldDev {
     // colouring
     int* cstat;                  // per constraint: colour or -1
     unsigned long long* bmask;   // per body: used colours (2 words)
-    int* adj_off;                // CSR body -> constraints
+    int* adj_off;                // first of each body's constraints in adj
     int* adj;
+    unsigned* cprio;             // [cap_arb + cap_joints] colouring priority
     int* deg;
     int* color_count;            // [JG_MAX_COLORS + 1]
     int* color_start;            // [JG_MAX_COLORS + 1] arbiters
@@ -262,7 +263,7 @@ struct WorldDev {
     // per-step scratch of the cache merge and the colour permutation (each world its own)
     int2* ev_created;            // [cap_arb] keys of the arbiters created this step
     int2* ev_removed;            // [cap_arb] keys of the arbiters removed this step
-    int* remaining;              // [2] colouring: constraints still without a colour
+    int* remaining;              // [2] blocks done (colouring, then permutation), space handed out
     int* dst_index;              // [cap_arb] slot of each arbiter after the permutation, -1 if removed
     // launch shapes of the cooperative kernels, sized once per world on its device (host
     // side only; a world is driven by one host thread)

@@ -134,7 +134,7 @@ int allocate(jg_world* w) {
     if ((r = alloc_store(w, d.arb[1], d.cap_arb))) return r;
     d.cur = 0;
     DA(d.col_pair, d.cap_arb); DA(d.col_res, 3 * (size_t)d.cap_arb); DA(d.col_portal, 12 * (size_t)d.cap_arb);
-    DA(d.epa_list, d.cap_arb); DA(d.edge_list, d.cap_arb); DA(d.spec_list, d.cap_pairs);
+    DA(d.epa_list, d.cap_arb); DA(d.edge_list, d.cap_arb); DA(d.spec_list, d.cap_pairs); DA(d.qctl, 2);
     d.hcap = next_pow2(2 * d.cap_arb);
     DA(d.hkeys, d.hcap); DA(d.hvals, d.hcap);
     DA(d.cstat, d.cap_arb + d.cap_joints);
@@ -267,9 +267,9 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     if (sp.record_residual) cudaMemsetAsync(d.resid, 0, sizeof(float) * 2 * JG_RESID_MAX, s);
     w->launches = jg_launch_aabb(d, sp.dt, s);
     w->launches += jg_launch_broadphase(d, s, w->nsm);
-    // the other kernels of this sequence: reset 1, narrowphase 3 + 5, merge 3 (+ warm-start
+    // the other kernels of this sequence: reset 1, narrowphase 2 + 5, merge 3 (+ warm-start
     // hook), schedule, colour and permute 2, solve 1, contact update 1, body update 1
-    w->launches += 1 + 8 + 3 + 2 + 1 + 1 + 1 + jg_schedule_launches(sp);
+    w->launches += 1 + 7 + 3 + 2 + 1 + 1 + 1 + jg_schedule_launches(sp);
     if (timed) cudaEventRecord(w->ev[1], s);
     jg_launch_narrowphase(d, sp, s, w->nsm, w->prm.narrow_tile);
     if (timed) cudaEventRecord(w->ev[2], s);

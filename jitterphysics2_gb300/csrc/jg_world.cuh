@@ -192,13 +192,14 @@ struct WorldDev {
     float4* scene_box;           // [0] min, [1] max (reduction)
     int2* pairs;
     int* pair_order;             // [cap_pairs] pair indices grouped by the two shapes' kinds
-    int* pair_kind;              // [2 * 64] counts, then cursors, per kind combination
+    int* pair_kind;              // [2 * 64] counts, then cursors from 0, per kind combination
     // narrowphase: overlapping pairs from the MPR stage, then the contact stream
     int2* col_pair;              // [cap_arb] pair index, MPR code (1 final, 2 needs EPA)
     float4* col_res;             // [3 * cap_arb] MPR result in A's frame: pA, pB, normal|depth
     float4* col_portal;          // [12 * cap_arb] MPR portal (4 vertices: V, A, B), by EPA-list slot
     int* epa_list;               // [cap_arb] colliding-record index of each deep pair
     int* edge_list;              // [cap_arb] colliding-record index of each pair near a mesh edge
+    int* qctl;                   // [2] pair queries: deep pairs, work cursor
     int* spec_list;              // [cap_pairs] pairs without overlap that qualify for the sweep
     int2* cs_key;
     float4* cs_n;                // normal xyz, count

@@ -121,7 +121,7 @@ int allocate(jg_world* w) {
     DA(d.amin, d.cap_shapes); DA(d.amax, d.cap_shapes);
     DA(d.mkey, d.cap_shapes); DA(d.mkey_alt, d.cap_shapes); DA(d.midx, d.cap_shapes); DA(d.midx_alt, d.cap_shapes);
     int rs_blocks = (d.cap_shapes + 2047) / 2048;
-    DA(d.hist, std::max(256 * rs_blocks + 1, 8192));
+    DA(d.hist, 256 * (size_t)rs_blocks + 256);
     DA(d.node, d.cap_shapes); DA(d.node_range, d.cap_shapes); DA(d.nmin, d.cap_shapes); DA(d.nmax, d.cap_shapes);
     DA(d.cbox, 4 * (size_t)d.cap_shapes);
     DA(d.leaf_parent, d.cap_shapes); DA(d.node_parent, d.cap_shapes); DA(d.node_flag, d.cap_shapes);

@@ -757,10 +757,9 @@ __global__ void k_solve_tasks(WorldDev w, StepParams sp) {
                     for (int t = tbase[g] + blockIdx.x; t < tbase[g] + ntask[g]; t += gridDim.x) {
                         if (!wait_deps(w, t, level, status)) return;
                         if (!run_task(w, A, sp, t, kind, sbody, ring, sver, &s_abort, d2, l2)) return;
-                        if (threadIdx.x == 0) {  // run_task ended with a block barrier
-                            __threadfence();
-                            st_release_u32(&w.sc_done[t], level + 1);
-                        }
+                        // run_task ended with a block barrier, which the release covers (a fence
+                        // of its own in front of it took as long again, about 0.5 us a task)
+                        if (threadIdx.x == 0) st_release_u32(&w.sc_done[t], level + 1);
                     }
                 }
                 if (sp.record_residual && s == 0 && pass > 0 && !relax && pass <= JG_RESID_MAX)

@@ -38,8 +38,7 @@ __device__ __forceinline__ bool grid_sync(unsigned* count, unsigned* gen, int* s
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        __threadfence();
-        unsigned old = atom_add_release(count, 1u);
+        unsigned old = atom_add_release(count, 1u);  // covers the block's writes, ordered by the barrier above
         unsigned target = (old / gridDim.x + 1) * gridDim.x;
         // Polls are spaced by a short sleep: back-to-back polls from every block saturate
         // the L2 slice that holds the counter, which delays the arrivals and every other

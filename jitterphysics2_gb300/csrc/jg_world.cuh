@@ -178,7 +178,7 @@ struct WorldDev {
     // broadphase
     unsigned long long *mkey, *mkey_alt;
     int *midx, *midx_alt;
-    int *hist;                   // radix histograms
+    int *hist;                   // radix histograms: digit by tile, then the digits' totals
     int4* node;                  // internal nodes: left, right, parent, first|last packed
     int2* node_range;            // leaf range [first, last] per internal node
     float4 *nmin, *nmax;         // internal node AABBs

@@ -594,107 +594,183 @@ converged:
 // MprEpaSolver.SolveMpr (NarrowPhase.cs:98-347) up to the EPA hand-off.  Returns 0 (no
 // overlap), 1 (overlap, result final) or 2 (overlap deeper than epa_threshold: the MPR
 // result is in pA/pB/normal/pen as the fallback, and `portal` holds the tetrahedron EPA
-// starts from).  WARP: evaluated redundantly by a whole warp; otherwise one thread.
-template <bool WARP>
-__device__ int mpr_core(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, float epa_threshold,
-                        v3& pA, v3& pB, v3& normal, float& pen, MV* portal) {
-    const float eps = 1e-5f;
-    const int maxIter = 34;
-    const float NumericEpsilon = 1e-16f;
-    MV v0, v1, v2, v3v, v4;
-    v3 t1, t2, t3;
-    pen = 0.0f;
-    mk_center(sa, sb, qb, pb, v0);
-    if (fabsf(v0.V.x) < NumericEpsilon && fabsf(v0.V.y) < NumericEpsilon && fabsf(v0.V.z) < NumericEpsilon) v0.V.x = 1e-05f;
-    normal = -v0.V;
-    mk_support_t<WARP>(sa, sb, qb, pb, normal, v1);
-    pA = v1.A; pB = v1.B;
-    if (dot(v1.V, normal) <= 0.0f) return 0;
-    normal = cross(v1.V, v0.V);
-    if (len2(normal) < 1e-12f) {
-        normal = v1.V - v0.V;
-        normal = normalize(normal);
-        t1 = v1.A - v1.B;
-        pen = dot(t1, normal);
-        return 1;
+// starts from).
+// The search is a sequence of support evaluations, each followed by a few vector operations that
+// choose the next direction; here it is a machine that is handed one support point at a time,
+// so that the support maps stand in the code once and the lanes of a warp meet at them wherever
+// their searches are.  KEEP_MISS: pA and pB of a miss are wanted (the first support point).
+struct Mpr {
+    static constexpr int MAX_ITER = 34;
+    static constexpr float EPS = 1e-5f, TINY = 1e-16f;
+    v3 v0, normal, pA, pB;  // v0: the origin ray's start; normal: the direction to evaluate next
+    MV v1, v2, v3v;
+    float pen;
+    int stage, phase;       // stage 0, 1: first two points; 2: portal discovery; 3: refinement
+    bool hit;
+
+    __device__ __forceinline__ void begin(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb) {
+        MV c;
+        mk_center(sa, sb, qb, pb, c);
+        if (fabsf(c.V.x) < TINY && fabsf(c.V.y) < TINY && fabsf(c.V.z) < TINY) c.V.x = 1e-05f;
+        v0 = c.V;
+        normal = -v0;
+        pen = 0.0f;
+        stage = phase = 0;
+        hit = false;
     }
-    mk_support_t<WARP>(sa, sb, qb, pb, normal, v2);
-    if (dot(v2.V, normal) <= 0.0f) return 0;
-    t1 = v1.V - v0.V;
-    t2 = v2.V - v0.V;
-    normal = cross(t1, t2);
-    float dist = dot(normal, v0.V);
-    if (dist > 0.0f) {
-        MV t = v1;
-        v1 = v2; v2 = t;
-        normal = -normal;
+    // The portal's plane; 0 when it is degenerate, else -1.
+    __device__ __forceinline__ int face() {
+        phase++;
+        normal = cross(v2.V - v1.V, v3v.V - v1.V);
+        if (len2(normal) < TINY) return 0;
+        if (!hit) hit = dot(normal, v1.V) >= 0;
+        return -1;
     }
-    int phase2 = 0, phase1 = 0;
-    bool hit = false;
-    while (true) {
-        if (phase1 > maxIter) return 0;
-        phase1++;
-        mk_support_t<WARP>(sa, sb, qb, pb, normal, v3v);
-        if (dot(v3v.V, normal) <= 0.0f) return 0;
-        t1 = cross(v1.V, v3v.V);
-        if (dot(t1, v0.V) < 0.0f) {
-            v2 = v3v;
-            t1 = v1.V - v0.V; t2 = v3v.V - v0.V;
-            normal = cross(t1, t2);
-            continue;
-        }
-        t1 = cross(v3v.V, v2.V);
-        if (dot(t1, v0.V) < 0.0f) {
-            v1 = v3v;
-            t1 = v3v.V - v0.V; t2 = v2.V - v0.V;
-            normal = cross(t1, t2);
-            continue;
-        }
-        break;
-    }
-    while (true) {
-        phase2++;
-        t1 = v2.V - v1.V;
-        t2 = v3v.V - v1.V;
-        normal = cross(t1, t2);
-        float nsq = len2(normal);
-        if (nsq < NumericEpsilon) return 0;
-        if (!hit) {
-            float d = dot(normal, v1.V);
-            hit = d >= 0;
-        }
-        mk_support_t<WARP>(sa, sb, qb, pb, normal, v4);
-        t3 = v4.V - v3v.V;
-        float delta = dot(t3, normal);
-        pen = dot(v4.V, normal);
-        if (delta * delta <= eps * eps * nsq || pen <= 0.0f || phase2 > maxIter) {
-            if (!hit) return 0;
-            float invn = 1.0f / sqrtf(nsq);
-            pen *= invn;
-            int code = 1;
-            if (pen > epa_threshold) {
-                portal[0] = v0; portal[1] = v1; portal[2] = v2; portal[3] = v3v;
-                code = 2;
+    // Takes the support point along `normal`: -1 to go on, else the result code.
+    template <bool KEEP_MISS>
+    __device__ __forceinline__ int step(const MV& v, float epa_threshold) {
+        if (stage < 3) {
+            if (KEEP_MISS && stage == 0) { pA = v.A; pB = v.B; }
+            if (dot(v.V, normal) <= 0.0f) return 0;
+            if (stage == 0) {
+                v1 = v;
+                normal = cross(v1.V, v0);
+                if (len2(normal) < 1e-12f) {
+                    normal = v1.V - v0;
+                    normal = normalize(normal);
+                    pen = dot(v1.A - v1.B, normal);
+                    pA = v1.A; pB = v1.B;
+                    return 1;
+                }
+                stage = 1;
+                return -1;
             }
+            if (stage == 1) {
+                v2 = v;
+                normal = cross(v1.V - v0, v2.V - v0);
+                if (dot(normal, v0) > 0.0f) {
+                    const MV t = v1;
+                    v1 = v2; v2 = t;
+                    normal = -normal;
+                }
+                stage = 2;
+                phase = 1;
+                return -1;
+            }
+            v3v = v;
+            const bool first = dot(cross(v1.V, v3v.V), v0) < 0.0f;
+            if (first || dot(cross(v3v.V, v2.V), v0) < 0.0f) {
+                if (first) v2 = v3v; else v1 = v3v;
+                normal = cross(v1.V - v0, v2.V - v0);
+                if (phase > MAX_ITER) return 0;
+                phase++;
+                return -1;
+            }
+            stage = 3;
+            phase = 0;
+            return face();
+        }
+        const float nsq = len2(normal);
+        const float delta = dot(v.V - v3v.V, normal);
+        pen = dot(v.V, normal);
+        if (delta * delta <= EPS * EPS * nsq || pen <= 0.0f || phase > MAX_ITER) {
+            if (!hit) return 0;
+            const float invn = 1.0f / sqrtf(nsq);
+            pen *= invn;
             normal = normal * invn;
-            t3 = cross(v1.V, t1);
-            float gamma = dot(t3, normal) * invn;
-            t3 = cross(t2, v1.V);
-            float beta = dot(t3, normal) * invn;
-            float alpha = 1.0f - gamma - beta;
+            const float gamma = dot(cross(v1.V, v2.V - v1.V), normal) * invn;
+            const float beta = dot(cross(v3v.V - v1.V, v1.V), normal) * invn;
+            const float alpha = 1.0f - gamma - beta;
             pA = alpha * v1.A + beta * v2.A + gamma * v3v.A;
             pB = alpha * v1.B + beta * v2.B + gamma * v3v.B;
-            return code;
+            return pen > epa_threshold ? 2 : 1;
         }
-        t1 = cross(v4.V, v0.V);
-        float d = dot(t1, v1.V);
-        if (d >= 0.0f) {
-            d = dot(t1, v2.V);
-            if (d >= 0.0f) v1 = v4; else v3v = v4;
+        const v3 t = cross(v.V, v0);
+        if (dot(t, v1.V) >= 0.0f) {
+            if (dot(t, v2.V) >= 0.0f) v1 = v; else v3v = v;
         } else {
-            d = dot(t1, v3v.V);
-            if (d >= 0.0f) v2 = v4; else v1 = v4;
+            if (dot(t, v3v.V) >= 0.0f) v2 = v; else v1 = v;
         }
+        return face();
+    }
+    // The tetrahedron EPA starts from.
+    __device__ __forceinline__ MV corner(int k, const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb) const {
+        MV c;
+        mk_center(sa, sb, qb, pb, c);
+        c.V = v0;
+        return k == 0 ? c : (k == 1 ? v1 : (k == 2 ? v2 : v3v));
+    }
+};
+
+// One search by a whole warp.
+__device__ int mpr_warp(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, float epa_threshold,
+                        v3& pA, v3& pB, v3& normal, float& pen, MV* portal) {
+    Mpr M;
+    M.begin(sa, sb, qb, pb);
+    int code;
+    do {
+        MV v;
+        mk_support(sa, sb, qb, pb, M.normal, v);
+        code = M.step<true>(v, epa_threshold);
+    } while (code < 0);
+    pA = M.pA; pB = M.pB; normal = M.normal; pen = M.pen;
+    if (code == 2)
+        for (int k = 0; k < 4; k++) portal[k] = M.corner(k, sa, sb, qb, pb);
+    return code;
+}
+
+// n searches, one per lane.  Most pairs separate after one or two support points and few
+// take ten, so that a warp that waits for its last lane runs with a sixth of its lanes (5.0 of
+// 32 measured): here a lane that is done waits only until half of its warp is, which then
+// hands in its results and takes the next pairs.  A warp takes its pairs in rounds of `share`
+// neighbours, fewer than 32 where there are fewer pairs than lanes: lanes of one warp that take
+// different branches wait for each other.  load(q, sa, sb, qb, pb) returns a tag, negative for
+// a pair to skip; flush(done, code, q, tag, M, sa, sb, qb, pb) is called by whole warps.
+template <bool KEEP_MISS, class Load, class Flush>
+__device__ __forceinline__ void mpr_lanes(int n, float epa_threshold, Load load, Flush flush) {
+    const int lane = threadIdx.x & 31, per = blockDim.x >> 5;
+    const int warps = gridDim.x * per, W = blockIdx.x * per + (threadIdx.x >> 5);
+    const int rounds = (n - 1) / (32 * warps) + 1, share = (n - 1) / (warps * rounds) + 1, total = rounds * share;
+    const int refill = (share + 1) / 2;
+    Mpr M;
+    ShapeRef sa, sb;
+    q4 qb;
+    v3 pb;
+    int taken = 0, q = -1, code = 0, tag = 0;  // q: this lane's pair; code -1: in progress
+    for (;;) {
+        const unsigned running = __ballot_sync(FULL, code < 0);
+        if (!running || (taken < total && share - __popc(running) >= refill)) {
+            flush(q >= 0 && code >= 0, code, q, tag, M, sa, sb, qb, pb);
+            const bool idle = code >= 0 && lane < share;
+            const unsigned m = __ballot_sync(FULL, idle);
+            if (idle) {
+                q = -1;
+                code = 0;
+                const int k = taken + __popc(m & ((1u << lane) - 1u)), r = k / share;
+                const int i = (r * warps + W) * share + k - r * share;
+                if (k < total && i < n && (tag = load(i, sa, sb, qb, pb)) >= 0) {
+                    q = i;
+                    code = -1;
+                    M.begin(sa, sb, qb, pb);
+                }
+            }
+            taken += __popc(m);
+            if (taken >= total && !__any_sync(FULL, code < 0)) break;
+            continue;
+        }
+        if (code < 0) {
+            MV v;
+            mk_support_t<false>(sa, sb, qb, pb, M.normal, v);
+            code = M.step<KEEP_MISS>(v, epa_threshold);
+        }
+    }
+}
+__device__ __forceinline__ void save_portal(const WorldDev& w, int e, const Mpr& M, const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb) {
+    for (int k = 0; k < 4; k++) {
+        const MV c = M.corner(k, sa, sb, qb, pb);
+        w.col_portal[12 * e + 3 * k + 0] = f4(c.V, 0.f);
+        w.col_portal[12 * e + 3 * k + 1] = f4(c.A, 0.f);
+        w.col_portal[12 * e + 3 * k + 2] = f4(c.B, 0.f);
     }
 }
 
@@ -720,7 +796,7 @@ __device__ void run_epa(EpaSmem& E, const ShapeRef& sa, const ShapeRef& sb, q4 q
 __device__ __noinline__ bool solve_mpr(EpaSmem& E, const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, float epa_threshold,
                           v3& pA, v3& pB, v3& normal, float& pen, NpStats& st, int& epa_calls, int& epa_fail) {
     MV portal[4];
-    int code = mpr_core<true>(sa, sb, qb, pb, epa_threshold, pA, pB, normal, pen, portal);
+    int code = mpr_warp(sa, sb, qb, pb, epa_threshold, pA, pB, normal, pen, portal);
     if (code == 2) run_epa(E, sa, sb, qb, pb, portal, pA, pB, normal, pen, st, epa_calls, epa_fail);
     return code != 0;
 }
@@ -1228,56 +1304,49 @@ __global__ void k_pair_scatter(WorldDev w, PairList L) {
 // (NarrowPhase.MprEpa, NarrowPhase.cs:902-927, up to the EPA hand-off).  Overlapping pairs
 // are appended to the colliding list with their MPR result; deeper than the EPA threshold,
 // also to the EPA list with the MPR portal EPA starts from.  Separated pairs with a
-// speculative body go to the sweep list (World.Detect.cs:162-170).
+// speculative body go to the sweep list (World.Detect.cs:162-170).  Bound by instruction issue
+// and, where a lane takes its next pair, by the loads of the two shapes; as many warps as the
+// registers of a search allow (three or four CTAs an SM spill: 0.5 ms more on 4096 worlds).
+// Against one thread per pair to the end: 4096 worlds 1.30 -> 0.66 ms, a settled 100k pile
+// 0.62 -> 0.33, a 20k pile 0.13 -> 0.11, a 700-body pile 0.064 -> 0.044.
 __global__ void __launch_bounds__(256, 2) k_mpr(WorldDev w) {
     const int npairs = min(w.ctr->npairs, w.cap_pairs);
     const int cap = w.cap_arb;
-    for (int base = blockIdx.x * blockDim.x; base < npairs; base += gridDim.x * blockDim.x) {
-        const int q = base + threadIdx.x;
-        const int p = q < npairs ? w.pair_order[q] : npairs;
-        int code = 0;
-        bool sweep = false;
-        v3 pA, pB, n;
-        float pen = 0.f;
-        MV portal[4];
-        if (p < npairs) {
-            int2 pr = w.pairs[p];
-            int s1 = pr.x, s2 = pr.y;  // s1 < s2: ShapeId order (World.Detect.cs:141-144)
-            int b1 = w.sinfo[s1].y, b2 = w.sinfo[s2].y;
-            int4 i1 = w.binfo[b1], i2 = w.binfo[b2];
-            bool skip = (!(i1.y & JG_BODY_ACTIVE) && !(i2.y & JG_BODY_ACTIVE)) ||
-                        (i1.x != JG_MOTION_DYNAMIC && i2.x != JG_MOTION_DYNAMIC);
-            if (!skip) {
-                ShapeRef sa = load_shape(w, s1), sb = load_shape(w, s2);
-                q4 qa = mkq(w.q[b1]), qb = mkq(w.q[b2]);
-                v3 pa = mk3(w.pos[b1]), pb = mk3(w.pos[b2]);
-                q4 q = qmul(qconj(qa), qb);
-                v3 pr_ = rotate_inv(pb - pa, qa);
-                const bool spec_body = ((i1.y | i2.y) & JG_BODY_SPECULATIVE) != 0;
-                code = mpr_core<false>(sa, sb, q, pr_, 0.02f, pA, pB, n, pen, portal);
-                sweep = code == 0 && spec_body;
+    if (npairs <= 0) return;
+    mpr_lanes<false>(
+        npairs, 0.02f,
+        [&](int q, ShapeRef& sa, ShapeRef& sb, q4& rot, v3& rel) {
+            const int2 pr = w.pairs[w.pair_order[q]];
+            const int s1 = pr.x, s2 = pr.y;  // s1 < s2: ShapeId order (World.Detect.cs:141-144)
+            const int b1 = w.sinfo[s1].y, b2 = w.sinfo[s2].y;
+            const int4 i1 = w.binfo[b1], i2 = w.binfo[b2];
+            if ((!(i1.y & JG_BODY_ACTIVE) && !(i2.y & JG_BODY_ACTIVE)) ||
+                (i1.x != JG_MOTION_DYNAMIC && i2.x != JG_MOTION_DYNAMIC)) return -1;
+            sa = load_shape(w, s1);
+            sb = load_shape(w, s2);
+            const q4 qa = mkq(w.q[b1]);
+            rot = qmul(qconj(qa), mkq(w.q[b2]));
+            rel = rotate_inv(mk3(w.pos[b2]) - mk3(w.pos[b1]), qa);
+            return ((i1.y | i2.y) & JG_BODY_SPECULATIVE) != 0 ? 1 : 0;
+        },
+        [&](bool done, int code, int q, int spec_body, const Mpr& M, const ShapeRef& sa, const ShapeRef& sb, q4 rot, v3 rel) {
+            const int p = done ? w.pair_order[q] : 0;
+            const int si = warp_append(&w.ctr->nspec, done && code == 0 && spec_body);
+            if (si >= 0) w.spec_list[si] = p;
+            int c = warp_append(&w.ctr->ncol, done && code != 0);
+            if (c >= cap) { atomicCAS(&w.ctr->status, 0, JG_ERR_CAPACITY); c = -1; }
+            if (c >= 0) {
+                w.col_pair[c] = make_int2(p, code);
+                w.col_res[3 * c + 0] = f4(M.pA, 0.f);
+                w.col_res[3 * c + 1] = f4(M.pB, 0.f);
+                w.col_res[3 * c + 2] = f4(M.normal, M.pen);
             }
-        }
-        int si = warp_append(&w.ctr->nspec, sweep);
-        if (si >= 0) w.spec_list[si] = p;
-        int c = warp_append(&w.ctr->ncol, code != 0);
-        if (c >= cap) { atomicCAS(&w.ctr->status, 0, JG_ERR_CAPACITY); c = -1; }
-        if (c >= 0) {
-            w.col_pair[c] = make_int2(p, code);
-            w.col_res[3 * c + 0] = f4(pA, 0.f);
-            w.col_res[3 * c + 1] = f4(pB, 0.f);
-            w.col_res[3 * c + 2] = f4(n, pen);
-        }
-        int e = warp_append(&w.ctr->nepa_list, code == 2 && c >= 0);
-        if (e >= 0) {
-            w.epa_list[e] = c;
-            for (int k = 0; k < 4; k++) {
-                w.col_portal[12 * e + 3 * k + 0] = f4(portal[k].V, 0.f);
-                w.col_portal[12 * e + 3 * k + 1] = f4(portal[k].A, 0.f);
-                w.col_portal[12 * e + 3 * k + 2] = f4(portal[k].B, 0.f);
+            const int e = warp_append(&w.ctr->nepa_list, code == 2 && c >= 0);
+            if (e >= 0) {
+                w.epa_list[e] = c;
+                save_portal(w, e, M, sa, sb, rot, rel);
             }
-        }
-    }
+        });
 }
 
 // ---- speculative contacts: time of impact by conservative advancement --------------------
@@ -1735,38 +1804,36 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_collide_query(WorldDev w, con
     }
 }
 
-__global__ void __launch_bounds__(128) k_query_mpr(WorldDev w, const int2* pairs, int n, bool grouped, float threshold,
+__global__ void __launch_bounds__(128, 4) k_query_mpr(WorldDev w, const int2* pairs, int n, bool grouped, float threshold,
                                                    float* out, int* hit) {
-    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const int q = base + threadIdx.x;
-        int code = 0, i = 0;
-        v3 pA = mk3(0.f), pB = mk3(0.f), nn = mk3(0.f);
-        float pen = 0.f;
-        MV portal[4];
-        if (q < n) {
-            i = grouped ? w.pair_order[q] : q;
-            const int2 pr = pairs[i];
-            ShapeRef sa = load_shape(w, pr.x), sb = load_shape(w, pr.y);
+    if (n <= 0) return;
+    mpr_lanes<true>(
+        n, threshold,
+        [&](int q, ShapeRef& sa, ShapeRef& sb, q4& rot, v3& rel) {
+            const int2 pr = pairs[grouped ? w.pair_order[q] : q];
+            sa = load_shape(w, pr.x);
+            sb = load_shape(w, pr.y);
             const int b1 = w.sinfo[pr.x].y, b2 = w.sinfo[pr.y].y;
-            const q4 qa = mkq(w.q[b1]), qb = mkq(w.q[b2]);
-            const v3 pa = mk3(w.pos[b1]), pb = mk3(w.pos[b2]);
-            code = mpr_core<false>(sa, sb, qmul(qconj(qa), qb), rotate_inv(pb - pa, qa), threshold, pA, pB, nn, pen, portal);
-            hit[i] = code != 0;
-            if (code != 2) write_query(out + 10 * (size_t)i, pA, pB, nn, pen, qa, pa);
-        }
-        const int e = warp_append(&w.qctl[0], code == 2);
-        if (e >= 0) {
-            w.epa_list[e] = i;
-            w.col_res[3 * e + 0] = f4(pA, 0.f);
-            w.col_res[3 * e + 1] = f4(pB, 0.f);
-            w.col_res[3 * e + 2] = f4(nn, pen);
-            for (int k = 0; k < 4; k++) {
-                w.col_portal[12 * e + 3 * k + 0] = f4(portal[k].V, 0.f);
-                w.col_portal[12 * e + 3 * k + 1] = f4(portal[k].A, 0.f);
-                w.col_portal[12 * e + 3 * k + 2] = f4(portal[k].B, 0.f);
+            const q4 qa = mkq(w.q[b1]);
+            rot = qmul(qconj(qa), mkq(w.q[b2]));
+            rel = rotate_inv(mk3(w.pos[b2]) - mk3(w.pos[b1]), qa);
+            return b1;
+        },
+        [&](bool done, int code, int q, int b1, const Mpr& M, const ShapeRef& sa, const ShapeRef& sb, q4 rot, v3 rel) {
+            const int i = done ? (grouped ? w.pair_order[q] : q) : 0;
+            if (done) {
+                hit[i] = code != 0;
+                if (code != 2) write_query(out + 10 * (size_t)i, M.pA, M.pB, M.normal, M.pen, mkq(w.q[b1]), mk3(w.pos[b1]));
             }
-        }
-    }
+            const int e = warp_append(&w.qctl[0], done && code == 2);
+            if (e >= 0) {
+                w.epa_list[e] = i;
+                w.col_res[3 * e + 0] = f4(M.pA, 0.f);
+                w.col_res[3 * e + 1] = f4(M.pB, 0.f);
+                w.col_res[3 * e + 2] = f4(M.normal, M.pen);
+                save_portal(w, e, M, sa, sb, rot, rel);
+            }
+        });
 }
 __global__ void __launch_bounds__(NP_WARPS * 32) k_query_epa(WorldDev w, const int2* pairs, float* out) {
     extern __shared__ __align__(16) unsigned char np_smem_raw[];
@@ -1870,10 +1937,8 @@ void jg_launch_collide_query(WorldDev& w, const int2* pairs, int n, float thresh
             k_pair_hist<<<blocks, 256, 0, s>>>(w, PairList{pr, m});
             k_pair_scatter<<<blocks, 256, 0, s>>>(w, PairList{pr, m});
         }
-        int blocks = (m + 127) / 128;
-        k_query_mpr<<<blocks < nsm * 16 ? blocks : nsm * 16, 128, 0, s>>>(w, pr, m, grouped, threshold, out + 10 * (size_t)first,
-                                                                         hit + first);
-        blocks = (m + NP_WARPS - 1) / NP_WARPS;
+        k_query_mpr<<<nsm * 4, 128, 0, s>>>(w, pr, m, grouped, threshold, out + 10 * (size_t)first, hit + first);
+        const int blocks = (m + NP_WARPS - 1) / NP_WARPS;
         k_query_epa<<<blocks < nsm * 4 ? blocks : nsm * 4, NP_WARPS * 32, kNpSmem, s>>>(w, pr, out + 10 * (size_t)first);
     }
 }
@@ -1883,7 +1948,7 @@ void jg_launch_narrowphase(WorldDev& w, const StepParams& p, cudaStream_t s, int
     cudaMemsetAsync(w.pair_kind, 0, sizeof(int) * 128, s);
     k_pair_hist<<<nsm * 4, 256, 0, s>>>(w, PairList{nullptr, 0});
     k_pair_scatter<<<nsm * 4, 256, 0, s>>>(w, PairList{nullptr, 0});
-    k_mpr<<<nsm * 8, 256, 0, s>>>(w);
+    k_mpr<<<nsm * 2, 256, 0, s>>>(w);
     k_sweep<<<nsm * 2, 128, 0, s>>>(w, p);
     k_epa<<<nsm * 4, NP_WARPS * 32, kNpSmem, s>>>(w);
     k_manifold<<<nsm * 16, 128, 0, s>>>(w, p);

@@ -210,10 +210,11 @@ __device__ __forceinline__ bool is_safe(v3 p) { return safe_coord(p.x) && safe_c
 // face needs about 250 when one lane evaluates it.  Here lane c of a group of four holds
 // component c of the vectors (the fourth repeats the first), so that an operation on three
 // components is one instruction, and the sums and quotients of a face that do not depend on
-// each other take one lane each: about 85 instructions for up to eight faces.  Every operation
-// and its order are the reference's, so the values are those of the one-lane form bit for bit.
-// k_epa, bound by this pipe: 1374 -> 734 us on a settled 100k-body pile (7.2k deep pairs), 545 ->
-// 300 us where a few hundred pairs leave only the latency of the longest one; k_edge 513 -> 384.
+// each other take one lane each: about 60 instructions for up to eight faces, with what only
+// signs or orders are needed of decided without a division.  Every value that is used comes
+// from the reference's operations in their order, so it is that of the one-lane form bit for bit.
+// k_epa, bound by this pipe: 1374 -> 597 us on a settled 100k-body pile (7.2k deep pairs), 545 ->
+// 249 us where a few hundred pairs leave only the latency of the longest one; k_edge 513 -> 387.
 // Signs and maxima of finite doubles are decided on their bit patterns (integer pipe).
 __device__ __forceinline__ double grp(double x, int src) { return __shfl_sync(FULL, x, src, 4); }
 __device__ __forceinline__ bool x_nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
@@ -221,6 +222,13 @@ __device__ __forceinline__ bool d_lt0(double x) { return __double_as_longlong(x)
 __device__ __forceinline__ bool d_ge0(double x) { return !d_lt0(x); }
 __device__ __forceinline__ bool d_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 __device__ __forceinline__ long long d_absbits(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffll; }
+
+__device__ __forceinline__ int d_exp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// A float that is zero or normal, widened on the integer pipe.
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
+    return __hiloint2double((int)((u & 0x80000000u) | (m ? (m >> 3) + (896u << 20) : 0u)), (int)(u << 29));
+}
 
 // (x0 + x1) + x2 of up to four vectors at once: lane k of the group returns the sum of the
 // components of the k-th argument, in the order of the reference's dot products.
@@ -244,26 +252,32 @@ __device__ __forceinline__ double grp_sums(int c, double p, double q, double r, 
 // a numerical failure.  Called by the whole warp; the coordinates are safe_coord's, so that no
 // value up to the quotients overflows.
 struct FaceGeo { double sn, cl, d2; double bx, by, bz; bool ok; };
-__device__ __noinline__ FaceGeo face_geo(const EpaSmem& E, int i0, int i1, int i2, bool swapped, bool count, NpStats& st) {
+__device__ __noinline__ FaceGeo face_geo(const EpaSmem& E, int i0, int i1, int i2, bool swapped, bool weights, bool count, NpStats& st) {
     const double EF = 16 * 1.1102230246251565e-16;
     const int c = threadIdx.x & 3, k = c == 3 ? 0 : c, k1 = k == 2 ? 0 : k + 1, k2 = k == 0 ? 2 : k - 1;
-    const double p0 = (double)(&E.vV[i0].x)[k], p1 = (double)(&E.vV[i1].x)[k], p2 = (double)(&E.vV[i2].x)[k];
+    const double p0 = widen((&E.vV[i0].x)[k]), p1 = widen((&E.vV[i1].x)[k]), p2 = widen((&E.vV[i2].x)[k]);
     FaceGeo g;
     const double u = p0 - p1, v = p0 - p2;
+    const double a = swapped ? p1 : p0, b = swapped ? p0 : p1;
     double raw;
-    long long rmax, emax;
+    long long rmax;
+    bool exact;
     {
         const double s = grp(u, k1) * grp(v, k2), t = grp(u, k2) * grp(v, k1);
         raw = s - t;
-        const long long e = d_absbits(EF * (fabs(s) + fabs(t)));
         if (swapped) raw = -raw;
-        const long long m = d_absbits(raw);
+        const long long m = d_absbits(raw), e = max(d_absbits(s), d_absbits(t));
         rmax = max(max(__shfl_sync(FULL, m, 0, 4), __shfl_sync(FULL, m, 1, 4)), __shfl_sync(FULL, m, 2, 4));
-        emax = max(max(__shfl_sync(FULL, e, 0, 4), __shfl_sync(FULL, e, 1, 4)), __shfl_sync(FULL, e, 2, 4));
+        const long long big = max(max(__shfl_sync(FULL, e, 0, 4), __shfl_sync(FULL, e, 1, 4)), __shfl_sync(FULL, e, 2, 4));
+        // unreliable unless the largest component exceeds 2^20 times the largest error bound, which
+        // is 2^-49 (|s| + |t|): decided by 2^-28 max(|s|, |t|) where that is enough
+        exact = !(rmax > max(big - (28ll << 52), 0ll));
+        if (__any_sync(FULL, exact)) {
+            const long long r = d_absbits(EF * (fabs(s) + fabs(t)));
+            const long long emax = max(max(__shfl_sync(FULL, r, 0, 4), __shfl_sync(FULL, r, 1, 4)), __shfl_sync(FULL, r, 2, 4));
+            exact = !(rmax > (emax ? emax + (20ll << 52) : 0));
+        }
     }
-    const double a = swapped ? p1 : p0, b = swapped ? p0 : p1;
-    // unreliable unless the largest component exceeds 2^20 times the largest error bound
-    const bool exact = !(rmax > (emax ? emax + (20ll << 52) : 0));
     if (__any_sync(FULL, exact)) {
         double x = 0, y = 0, z = 0;
         if (exact) {
@@ -286,20 +300,32 @@ __device__ __noinline__ FaceGeo face_geo(const EpaSmem& E, int i0, int i1, int i
     g.sn = sn;
     const double nn = sn * sn;
     const double nsq = (grp(nn, 0) + grp(nn, 1)) + grp(nn, 2);
-    const double uf = a - b, vf = a - p2;  // of the final order
+    const double uf = swapped && x_nonzero(u) ? -u : u, vf = a - p2;  // a - b and a - c of the final order
     const double a1 = grp(a, k1), a2 = grp(a, k2), uf1 = grp(uf, k1), uf2 = grp(uf, k2), vf1 = grp(vf, k1), vf2 = grp(vf, k2);
-    // lane 0: gamma, lane 1: beta, lane 2: the plane's distance, each over nsq in one division
+    // lanes 0 to 2: gamma times nsq ns, beta times nsq ns, the plane's distance times nsq
     const double num = grp_sums(c, (uf1 * a2 - uf2 * a1) * sn, (a1 * vf2 - a2 * vf1) * sn, sn * a, 0.0);
-    const double q1 = num / nsq;
-    const double q2 = q1 / ns;
-    const double dq = grp(q1, 2);
-    double gamma = grp(q2, 0), beta = grp(q2, 1);
-    double alpha = 1.0 - gamma - beta;
-    g.cl = sn * dq;
+    const double n0 = grp(num, 0), n1 = grp(num, 1);
+    // The weights' signs decide what is closest.  Those of gamma and beta are the numerators'
+    // (coordinates and ns in this range leave no underflow); alpha = 1 - gamma - beta has that of
+    // ns nsq - (n0 + n1) if that is not within 2^-40 of the terms, where the roundings could decide.
+    // So the two divisions that give the weights themselves are left to the calls that ask for
+    // them, and to those cases.
+    const double den = ns * nsq, rest = den - (n0 + n1);
+    const int e = d_exp(ns);
+    const bool sure = e > 1023 - 200 && e < 1023 + 200 && d_exp(rest) + 40 > max(d_exp(den), max(d_exp(n0), d_exp(n1)));
+    double gamma = n0, beta = n1, alpha = rest;  // (or positive multiples of them)
+    if (__any_sync(FULL, weights || !sure)) {
+        const double q2 = (num / nsq) / ns;
+        gamma = grp(q2, 0);
+        beta = grp(q2, 1);
+        alpha = 1.0 - gamma - beta;
+    }
     const bool c1 = d_ge0(alpha) && d_lt0(beta), c2 = !c1 && d_ge0(beta) && d_lt0(gamma),
                c3 = !c1 && !c2 && d_ge0(gamma) && d_lt0(alpha);
-    const bool clamped = c1 || c2 || c3;
-    if (__any_sync(FULL, clamped)) {
+    const bool clamped = c1 || c2 || c3, some = __any_sync(FULL, clamped);
+    double top = grp(num, 2), bottom = nsq;
+    bool first = false;
+    if (some) {
         // the three cases differ in the corner P, the edge Q tried first and the edge R taken
         // otherwise: (a, u, v), (b, w, u), (c, v, w)
         const double w = b - p2;
@@ -308,11 +334,17 @@ __device__ __noinline__ FaceGeo face_geo(const EpaSmem& E, int i0, int i1, int i
         double t = grp(s, 0), o = grp(s, 1);
         if (c3) t = -t;
         if (!c1) o = -o;
-        const bool first = d_lt0(c1 ? gamma : (c2 ? alpha : beta)) && !d_lt0(t) && x_nonzero(t);
+        first = d_lt0(c1 ? gamma : (c2 ? alpha : beta)) && !d_lt0(t) && x_nonzero(t);
         const double qq = grp(s, 2), rr = grp(s, 3);
-        double r = (first ? t : o) / (first ? qq : rr);
-        if (first) r = fmin(1.0, r);
-        else r = d_lt0(r) ? 0.0 : (r > 1.0 ? 1.0 : r);
+        if (clamped) { top = first ? t : o; bottom = first ? qq : rr; }
+    }
+    double r = top / bottom;  // the plane's distance, or the point's place on its edge
+    g.cl = sn * r;
+    if (some) {
+        const long long one = 0x3ff0000000000000ll, rb = __double_as_longlong(r);
+        // to [0, 1]; 0/0 of the second edge goes through as it is unless it counts as negative
+        if (first ? rb > one : rb > one && rb <= 0x7ff0000000000000ll) r = 1.0;
+        else if (!first && d_lt0(r)) r = 0.0;
         const double q = 1.0 - r;
         if (clamped) {
             if (c1) { alpha = q; beta = first ? r : 0.0; gamma = first ? 0.0 : r; }
@@ -335,7 +367,7 @@ __device__ __noinline__ FaceGeo face_geo(const EpaSmem& E, int i0, int i1, int i
 __device__ __forceinline__ FaceGeo face_geo_of(const EpaSmem& E, int f, NpStats& st) {
     uchar4 t = E.fi[f];
     bool sw = (t.w & EPA_SWAPPED) != 0;
-    return face_geo(E, sw ? t.y : t.x, sw ? t.x : t.y, t.z, sw, true, st);
+    return face_geo(E, sw ? t.y : t.x, sw ? t.x : t.y, t.z, sw, true, true, st);
 }
 
 // The FP32 normal of a face and its squared length (Triangle.Normal / NormalSq).
@@ -365,7 +397,7 @@ __device__ __noinline__ int create_tris(EpaSmem& E, int a, int b, int c, int slo
     __syncwarp();
     const bool counts = live && comp == 0;  // one lane counts for its face
     if (counts) st.exact += mine.exact;
-    const FaceGeo g = face_geo(E, i0, i1, c, swapped, counts && orient != 0, st);
+    const FaceGeo g = face_geo(E, i0, i1, c, swapped, false, counts && orient != 0, st);
     const float out = (float)(comp == 3 ? g.d2 : g.cl);
     const unsigned bad = __ballot_sync(FULL, !isfinite(out));
     int r = ADDED;

@@ -267,9 +267,9 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     if (sp.record_residual) cudaMemsetAsync(d.resid, 0, sizeof(float) * 2 * JG_RESID_MAX, s);
     w->launches = jg_launch_aabb(d, sp.dt, s);
     w->launches += jg_launch_broadphase(d, s, w->nsm);
-    // the other kernels of this sequence: reset 1, narrowphase 2 + 5, merge 3 (+ warm-start
+    // the other kernels of this sequence: reset 1, narrowphase 2 + 4 (5 with a mesh), merge 3 (+ warm-start
     // hook), schedule, colour and permute 2, solve 1, contact update 1, body update 1
-    w->launches += 1 + 7 + 3 + 2 + 1 + 1 + 1 + jg_schedule_launches(sp);
+    w->launches += 1 + 6 + (d.ntris > 0 && sp.edge_filter) + 3 + 2 + 1 + 1 + 1 + jg_schedule_launches(sp);
     if (timed) cudaEventRecord(w->ev[1], s);
     jg_launch_narrowphase(d, sp, s, w->nsm, w->prm.narrow_tile);
     if (timed) cudaEventRecord(w->ev[2], s);

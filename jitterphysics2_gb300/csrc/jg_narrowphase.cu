@@ -35,8 +35,17 @@ __device__ __forceinline__ void mk_support_t(const ShapeRef& sa, const ShapeRef&
     v.B = v.B + pb;
     v.V = v.A - v.B;
 }
-__device__ __forceinline__ void mk_support(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, v3 d, MV& v) {
-    mk_support_t<true>(sa, sb, qb, pb, d, v);
+// (One copy of the support maps for both shapes, and a call: EPA, MPR and the manifold of a warp
+// kernel share an instruction cache that they fill.)
+__device__ __noinline__ void mk_support(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, v3 d, MV& v) {
+    const v3 db = rotate_inv(-d, qb);
+    v3 p[2];
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) p[k] = support(k ? sb : sa, k ? db : d);
+    v.A = p[0];
+    v.B = rotate(p[1], qb);
+    v.B = v.B + pb;
+    v.V = v.A - v.B;
 }
 __device__ __forceinline__ void mk_center(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, MV& c) {
     c.A = shape_center(sa);
@@ -47,7 +56,7 @@ __device__ __forceinline__ void mk_center(const ShapeRef& sa, const ShapeRef& sb
 
 // ---- exact arithmetic (double expansions), used only on unresolved EPA predicates -------
 struct Exp {
-    __device__ static int diff(double a, double b, double* o) {
+    __device__ __noinline__ static int diff(double a, double b, double* o) {
         double v = a - b, vb = a - v;
         double res = (a - (v + vb)) + (vb - b);
         int n = 0;
@@ -55,8 +64,9 @@ struct Exp {
         if (v != 0) o[n++] = v;
         return n;
     }
-    __device__ static int grow(double* e, int len, double value) {
+    __device__ __noinline__ static int grow(double* e, int len, double value) {
         int cnt = 0;
+#pragma unroll 1
         for (int i = 0; i < len; i++) {
             double part = e[i];
             double sum = value + part;
@@ -68,8 +78,10 @@ struct Exp {
         if (value != 0) e[cnt++] = value;
         return cnt;
     }
-    __device__ static int addp(double* r, int len, const double* a, int na, const double* b, int nb, bool neg, int cap) {
+    __device__ __noinline__ static int addp(double* r, int len, const double* a, int na, const double* b, int nb, bool neg, int cap) {
+#pragma unroll 1
         for (int i = 0; i < na; i++)
+#pragma unroll 1
             for (int j = 0; j < nb; j++) {
                 double x = a[i], y = b[j];
                 double p = __dmul_rn(x, y);
@@ -80,7 +92,7 @@ struct Exp {
             }
         return len;
     }
-    __device__ static int crossterm(const double* a, int na, const double* b, int nb, const double* c, int nc,
+    __device__ __noinline__ static int crossterm(const double* a, int na, const double* b, int nb, const double* c, int nc,
                                     const double* d, int nd, double* o) {
         int len = addp(o, 0, a, na, b, nb, false, 16);
         return addp(o, len, c, nc, d, nd, true, 16);
@@ -213,8 +225,8 @@ __device__ __forceinline__ bool is_safe(v3 p) { return safe_coord(p.x) && safe_c
 // each other take one lane each: about 60 instructions for up to eight faces, with what only
 // signs or orders are needed of decided without a division.  Every value that is used comes
 // from the reference's operations in their order, so it is that of the one-lane form bit for bit.
-// k_epa, bound by this pipe: 1374 -> 597 us on a settled 100k-body pile (7.2k deep pairs), 545 ->
-// 249 us where a few hundred pairs leave only the latency of the longest one; k_edge 513 -> 387.
+// EPA of a settled 100k-body pile (7.2k deep pairs) 1374 -> 597 us, of a few hundred pairs that leave
+// only the latency of the longest one 545 -> 249; pairs near mesh edges of the former 513 -> 387.
 // Signs and maxima of finite doubles are decided on their bit patterns (integer pipe).
 __device__ __forceinline__ double grp(double x, int src) { return __shfl_sync(FULL, x, src, 4); }
 __device__ __forceinline__ bool x_nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
@@ -387,6 +399,7 @@ __device__ __noinline__ int create_tris(EpaSmem& E, int a, int b, int c, int slo
     v3 va = mk3(E.vV[a]), vb = mk3(E.vV[b]), vc = mk3(E.vV[c]);
     const int i0 = a, i1 = b;
     int orient = 0;
+#pragma unroll 1
     for (int i = 0; i < 4 && orient == 0; i++) {
         if (i == a || i == b || i == c) continue;
         orient = -side_pt(va, vb, vc, mk3(E.vV[i]), mine);
@@ -468,6 +481,7 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
     __syncwarp();
     int nt = E.nt;
     // visibility of every face, lanes in parallel
+#pragma unroll 1
     for (int base = 0; base < nt; base += 32) {
         int i = base + lane;
         bool lit = false;
@@ -485,7 +499,9 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
     // in shared memory.
     int ne = 0, edge = 0;
     bool wide = false;
+#pragma unroll 1
     for (int word = (nt - 1) >> 5; word >= 0 && !wide; word--) {
+#pragma unroll 1
         for (unsigned m = E.lit[word]; m && !wide;) {
             const int bit = 31 - __clz(m);
             m ^= 1u << bit;
@@ -510,13 +526,16 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
     if (wide) {
         if (lane == 0) {
             int n = 0;
+#pragma unroll 1
             for (int index = nt; index-- > 0;) {
                 if (!((E.lit[index >> 5] >> (index & 31)) & 1u)) continue;
                 uchar4 f = E.fi[index];
                 unsigned char cs[3] = {f.x, f.y, f.z};
+#pragma unroll 1
                 for (int k = 0; k < 3; k++) {
                     unsigned char A = cs[k], B = cs[(k + 1) % 3];
                     bool added = true;
+#pragma unroll 1
                     for (int e = n; e-- > 0;) {
                         bool match = (E.ea[e] == A && E.eb[e] == B) || (E.ea[e] == B && E.eb[e] == A);
                         if (!match) continue;
@@ -535,10 +554,12 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
     }
     if (ne == 0) return NO_HORIZON;
     int nlit = 0;
+#pragma unroll 1
     for (int k = 0; k < (nt + 31) / 32; k++) nlit += __popc(E.lit[k] & (k * 32 + 32 <= nt ? 0xffffffffu : ((1u << (nt & 31)) - 1u)));
     if (nt - nlit + ne > JG_EPA_MAXT) return CAPACITY;
     // order-preserving compaction of the surviving faces
     int surv = 0;
+#pragma unroll 1
     for (int base = 0; base < nt; base += 32) {
         int i = base + lane;
         bool keep = i < nt && !((E.lit[i >> 5] >> (i & 31)) & 1u);
@@ -553,6 +574,7 @@ __device__ __noinline__ int epa_add(EpaSmem& E, const MV& v, NpStats& st) {
     }
     // the new fan, eight faces at a time
     int res = ADDED;
+#pragma unroll 1
     for (int base = 0; base < ne; base += 8) {
         const int e = min(base + (lane >> 2), ne - 1);
         int ea, eb;
@@ -882,23 +904,18 @@ __device__ __noinline__ int edge_evaluate(const WorldDev& w, int tri, q4 tq, v3 
 }
 
 // ---- one-shot manifold (CollisionManifold.cs) --------------------------------------------
-__device__ __forceinline__ void push_pt(float4* arr, int& cnt, v3 v) {
-    if (cnt > 0 && len2(mk3(arr[0]) - v) < 0.001f) return;
-    if (cnt > 1 && len2(mk3(arr[cnt - 1]) - v) < 0.001f) return;
-    if ((threadIdx.x & 31) == 0) arr[cnt] = f4(v, 0.f);
-    cnt++;
-    __syncwarp();
-}
-__device__ bool polygon_sign(const float4* poly, int cnt, v3 n, float& sign) {
+__device__ __noinline__ bool polygon_sign(const float4* poly, int cnt, v3 n, float& sign) {
     float area = 0.0f;
     v3 prev = mk3(poly[cnt - 1]);
+#pragma unroll 1
     for (int i = 0; i < cnt; i++) { v3 cur = mk3(poly[i]); area += dot(cross(prev, cur), n); prev = cur; }
     if (fabsf(area) <= 1e-6f) { sign = 0.f; return false; }
     sign = area < 0.0f ? -1.0f : 1.0f;
     return true;
 }
-__device__ bool contains_pt(const float4* poly, int cnt, v3 p, v3 n, float sign) {
+__device__ __forceinline__ bool contains_pt(const float4* poly, int cnt, v3 p, v3 n, float sign) {
     v3 prev = mk3(poly[cnt - 1]);
+#pragma unroll 1
     for (int i = 0; i < cnt; i++) {
         v3 cur = mk3(poly[i]);
         float sd = sign * dot(cross(cur - prev, p - prev), n);
@@ -907,10 +924,11 @@ __device__ bool contains_pt(const float4* poly, int cnt, v3 p, v3 n, float sign)
     }
     return true;
 }
-__device__ int clip_segment(v3 s, v3 e, const float4* poly, int pc, v3 n, float sign, v3* out) {
+__device__ __noinline__ int clip_segment(v3 s, v3 e, const float4* poly, int pc, v3 n, float sign, v3* out) {
     const float eps = 1e-3f;
     float enter = 0.0f, exit = 1.0f;
     v3 delta = e - s;
+#pragma unroll 1
     for (int i = 0; i < pc; i++) {
         v3 es = mk3(poly[i]), ee = mk3(poly[(i + 1) % pc]);
         float ss = sign * dot(cross(ee - es, s - es), n);
@@ -930,7 +948,7 @@ __device__ int clip_segment(v3 s, v3 e, const float4* poly, int pc, v3 n, float 
     return 2;
 }
 __device__ __forceinline__ float cross_along(v3 l, v3 r, v3 n) { return dot(cross(l, r), n); }
-__device__ int intersect_seg(v3 sA, v3 eA, v3 sB, v3 eB, v3 n, v3* cA, v3* cB) {
+__device__ __forceinline__ int intersect_seg(v3 sA, v3 eA, v3 sB, v3 eB, v3 n, v3* cA, v3* cB) {
     const float eps = 1e-3f;
     v3 dA = eA - sA, dB = eB - sB, off = sB - sA;
     float cr = cross_along(dA, dB, n);
@@ -961,68 +979,114 @@ __device__ int intersect_seg(v3 sA, v3 eA, v3 sB, v3 eB, v3 n, v3* cA, v3* cB) {
     return 1;
 }
 __device__ bool is_dup(const float4* m, int cnt, v3 p) {
+#pragma unroll 1
     for (int i = 0; i < cnt; i++) if (len2(mk3(m[i]) - p) < 0.001f) return true;
     return false;
 }
 struct MF {
     EpaSmem* E;
     int count;
+    __device__ __forceinline__ bool seen(const float4* m, v3 p) const {
+        const int lane = threadIdx.x & 31;
+        return __any_sync(FULL, lane < count && len2(mk3(m[lane]) - p) < 0.001f);
+    }
     __device__ void set(int i, v3 a, v3 b) {
         if ((threadIdx.x & 31) == 0) { E->mA[i] = f4(a, 0.f); E->mB[i] = f4(b, 0.f); }
         __syncwarp();
     }
-    __device__ void on_a(v3 p, v3 pB, v3 n) {
+    __device__ __noinline__ void on_a(v3 p, v3 pB, v3 n) {
         if (count == 12) return;
         float diff = dot(p - pB, n);
         if (diff < 0.0f) return;
-        if (is_dup(E->mA, count, p)) return;
+        if (seen(E->mA, p)) return;
         set(count, p, p - diff * n);
         count++;
     }
-    __device__ void on_b(v3 p, v3 pA, v3 n) {
+    __device__ __noinline__ void on_b(v3 p, v3 pA, v3 n) {
         if (count == 12) return;
         float diff = dot(p - pA, n);
         if (diff > 0.0f) return;
-        if (is_dup(E->mB, count, p)) return;
+        if (seen(E->mB, p)) return;
         set(count, p - diff * n, p);
         count++;
     }
-    __device__ void pair(v3 a, v3 b, v3 n) {
+    __device__ __noinline__ void pair(v3 a, v3 b, v3 n) {
         if (count == 12) return;
         if (dot(a - b, n) < 0.0f) return;
-        if (is_dup(E->mA, count, a)) return;
-        if (is_dup(E->mB, count, b)) return;
+        if (seen(E->mA, a)) return;
+        if (seen(E->mB, b)) return;
         set(count, a, b);
         count++;
     }
 };
 
+// The directions of the six samples around the normal.
+__device__ __constant__ float c_hex[12] = {1.0f, 0.0f, 0.5f, 0.86602540378f, -0.5f, 0.86602540378f,
+                                           -1.0f, 0.0f, -0.5f, -0.86602540378f, 0.5f, -0.86602540378f};
+// A sampled polygon from the points of lanes `first` .. `first` + 5, without the points that
+// repeat its first or last one.
+__device__ __forceinline__ int sample_polygon(float4* arr, v3 pt, int first) {
+    int cnt = 0;
+    v3 head = mk3(0.f), tail = mk3(0.f);
+#pragma unroll 1
+    for (int e = first; e < first + 6; e++) {
+        const v3 v = mk3(__shfl_sync(FULL, pt.x, e), __shfl_sync(FULL, pt.y, e), __shfl_sync(FULL, pt.z, e));
+        if (cnt > 0 && len2(head - v) < 0.001f) continue;
+        if (cnt > 1 && len2(tail - v) < 0.001f) continue;
+        if (cnt == 0) head = v;
+        tail = v;
+        if ((threadIdx.x & 31) == 0) arr[cnt] = f4(v, 0.f);
+        cnt++;
+    }
+    __syncwarp();
+    return cnt;
+}
+// A point cloud's samples, by the whole warp; lane first + e keeps the e-th.
+__device__ __noinline__ v3 sample_hull(const ShapeRef& s, q4 q, v3 dir, int first) {
+    v3 mine = mk3(0.f);
+#pragma unroll 1
+    for (int e = first; e < first + 6; e++) {
+        const v3 d = mk3(__shfl_sync(FULL, dir.x, e), __shfl_sync(FULL, dir.y, e), __shfl_sync(FULL, dir.z, e));
+        const v3 p = hull_support_warp(s.hull, s.nhull, d) + s.d;
+        if ((threadIdx.x & 31) == e) mine = p;
+    }
+    return mine;
+}
+
+// CollisionManifold.BuildManifold by a whole warp: a lane per sample, polygon corner, edge pair
+// and angle; the points are inserted in the reference's order.  (With every lane at the same
+// sample the twelve support maps stood in the code one after the other, and the warps of an SM,
+// each at another place, waited for instructions half of the time.)
 __device__ __noinline__ int build_manifold(EpaSmem& E, const ShapeRef& sa, const ShapeRef& sb, q4 qa, q4 qb, v3 pa, v3 pb,
                               v3 pA, v3 pB, v3 n, v3* outA, v3* outB) {
     const int lane = threadIdx.x & 31;
-    const float P = 0.01f, S = 0.86602540378f;
-    const float hx[12] = {1.0f, 0.0f, 0.5f, S, -0.5f, S, -1.0f, 0.0f, -0.5f, -S, 0.5f, -S};
+    const float P = 0.01f;
     v3 c1 = create_orthonormal(n);
     v3 c2 = cross(n, c1);
     v3 relB = pb - pa, pAl = pA - pa, pBl = pB - pa;
-    int lc = 0, rc = 0;
-    for (int e = 0; e < 6; e++) {
-        v3 pn = n + hx[2 * e + 0] * P * c1 + hx[2 * e + 1] * P * c2;
-        v3 np1 = rotate(support(sa, rotate_inv(pn, qa)), qa);
-        push_pt(E.left, lc, np1);
-        pn = -pn;
-        v3 np2 = rotate(support(sb, rotate_inv(pn, qb)), qb) + relB;
-        push_pt(E.right, rc, np2);
-    }
+    // lanes 0 to 5: A's samples, 6 to 11: B's
+    const bool onB = lane >= 6;
+    const int e = onB ? lane - 6 : lane, h = e < 6 ? e : 0;
+    v3 pn = n + c_hex[2 * h] * P * c1 + c_hex[2 * h + 1] * P * c2;
+    if (onB) pn = -pn;
+    const q4 q = onB ? qb : qa;
+    const v3 dir = rotate_inv(pn, q);
+    v3 pt = mk3(0.f);
+    const bool hullA = sa.kind == JG_SHAPE_POINTCLOUD, hullB = sb.kind == JG_SHAPE_POINTCLOUD;
+    if (lane < 12 && !(onB ? hullB : hullA)) pt = support_lane(onB ? sb : sa, dir);
+    __syncwarp();
+    if (hullA) { const v3 p = sample_hull(sa, qa, dir, 0); if (!onB) pt = p; }
+    if (hullB) { const v3 p = sample_hull(sb, qb, dir, 6); if (onB) pt = p; }
+    pt = rotate(pt, q);
+    if (onB) pt = pt + relB;
+    const int lc = sample_polygon(E.left, pt, 0), rc = sample_polygon(E.right, pt, 6);
     float ls = 0.f, rs = 0.f;
     bool lp = lc > 2 && polygon_sign(E.left, lc, n, ls);
     bool rp = rc > 2 && polygon_sign(E.right, rc, n, rs);
     MF m; m.E = &E; m.count = 0;
     if (lp) {
-        for (int e = 0; e < rc; e++) {
-            v3 p = mk3(E.right[e]);
-            if (!contains_pt(E.left, lc, p, n, ls)) continue;
-            m.on_b(p, pAl, n);
+        for (unsigned in = __ballot_sync(FULL, lane < rc && contains_pt(E.left, lc, mk3(E.right[lane]), n, ls)); in; in &= in - 1) {
+            m.on_b(mk3(E.right[__ffs(in) - 1]), pAl, n);
             if (m.count == 12) goto finalize;
         }
         if (rc == 2) {
@@ -1032,10 +1096,8 @@ __device__ __noinline__ int build_manifold(EpaSmem& E, const ShapeRef& sa, const
         }
     }
     if (rp) {
-        for (int e = 0; e < lc; e++) {
-            v3 p = mk3(E.left[e]);
-            if (!contains_pt(E.right, rc, p, n, rs)) continue;
-            m.on_a(p, pBl, n);
+        for (unsigned in = __ballot_sync(FULL, lane < lc && contains_pt(E.right, rc, mk3(E.left[lane]), n, rs)); in; in &= in - 1) {
+            m.on_a(mk3(E.left[__ffs(in) - 1]), pBl, n);
             if (m.count == 12) goto finalize;
         }
         if (lc == 2) {
@@ -1083,26 +1145,24 @@ finalize:
     if (count > 4) {
         // ReduceManifold (CollisionManifold.cs:321-375)
         v3 c = mk3(0.f);
+#pragma unroll 1
         for (int i = 0; i < count; i++) c = c + mk3(E.mA[i]);
         c = c * (float)(1.0 / count);
         v3 t1 = create_orthonormal(n);
         v3 t2 = cross(n, t1);
-        float ang[12];
-        int order[12];
+        // the points' places in the order of their angles (equal ones as they come)
+        const v3 d = mk3(E.mA[lane < count ? lane : 0]) - c;
+        const float ang = StableMathF::atan2(dot(d, t2), dot(d, t1));
+        int place = 0;
+#pragma unroll 1
         for (int i = 0; i < count; i++) {
-            v3 d = mk3(E.mA[i]) - c;
-            ang[i] = StableMathF::atan2(dot(d, t2), dot(d, t1));
-            order[i] = i;
+            const float o = __shfl_sync(FULL, ang, i);
+            place += o < ang || (o == ang && i < lane);
         }
-        for (int i = 1; i < count; i++) {
-            int cur = order[i];
-            float ca = ang[cur];
-            int j = i - 1;
-            while (j >= 0 && ang[order[j]] > ca) { order[j + 1] = order[j]; j--; }
-            order[j + 1] = cur;
-        }
+        if (lane >= count) place = -1;
+#pragma unroll
         for (int i = 0; i < 4; i++) {
-            int sel = order[((2 * i + 1) * count) / 8];
+            const int sel = max(__ffs(__ballot_sync(FULL, place == ((2 * i + 1) * count) / 8)) - 1, 0);
             outA[i] = mk3(E.mA[sel]) + pa;
             outB[i] = mk3(E.mB[sel]) + pa;
         }
@@ -1150,13 +1210,14 @@ __device__ __forceinline__ void push_local(float4* arr, int& cnt, v3 v) {
 
 __device__ __noinline__ int manifold_thread(const ShapeRef& sa, const ShapeRef& sb, q4 qa, q4 qb, v3 pa, v3 pb,
                                             v3 pA, v3 pB, v3 n, float4* outA, float4* outB) {
-    const float P = 0.01f, S = 0.86602540378f;
-    const float hx[12] = {1.0f, 0.0f, 0.5f, S, -0.5f, S, -1.0f, 0.0f, -0.5f, -S, 0.5f, -S};
+    const float P = 0.01f;
+    const float* hx = c_hex;
     v3 c1 = create_orthonormal(n);
     v3 c2 = cross(n, c1);
     v3 relB = pb - pa, pAl = pA - pa, pBl = pB - pa;
     float4 left[6], right[6];
     int lc = 0, rc = 0;
+#pragma unroll 1
     for (int e = 0; e < 6; e++) {
         v3 pn = n + hx[2 * e + 0] * P * c1 + hx[2 * e + 1] * P * c2;
         push_local(left, lc, rotate(support_lane(sa, rotate_inv(pn, qa)), qa));
@@ -1246,6 +1307,7 @@ finalize:
 }
 
 constexpr int NP_WARPS = 4;
+constexpr int COL_EDGE = 8;  // in a colliding record's kind: it waits in the edge list
 
 __device__ __forceinline__ int warp_append(int* counter, bool pred) {
     const int lane = threadIdx.x & 31;
@@ -1579,61 +1641,6 @@ __global__ void __launch_bounds__(128) k_sweep(WorldDev w, StepParams sp) {
     }
 }
 
-// Stage 2, one warp per deep pair: EPA from the saved portal (NarrowPhase.cs:39-95); on
-// success the colliding record takes the EPA result, otherwise the MPR result stands.
-// Next work item of a warp: lane 0 takes it from the cursor, every lane gets it.
-__device__ __forceinline__ int next_item(int* cursor, int lane) {
-    int e = 0;
-    if (lane == 0) e = atomicAdd(cursor, 1);
-    return __shfl_sync(0xffffffffu, e, 0);
-}
-
-__global__ void __launch_bounds__(NP_WARPS * 32) k_epa(WorldDev w) {
-    extern __shared__ __align__(16) unsigned char np_smem_raw[];
-    EpaSmem* smem = reinterpret_cast<EpaSmem*>(np_smem_raw);
-    const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    EpaSmem& E = smem[wib];
-    NpStats st; st.exact = 0;
-    int epa_calls = 0, epa_fail = 0;
-    const int ne = min(w.ctr->nepa_list, w.cap_arb);
-    // pairs handed out one at a time: EPA's cost varies by an order of magnitude between
-    // pairs, so a fixed share per warp would leave most warps idle behind a few
-    for (int e = next_item(&w.ctr->epa_next, lane); e < ne; e = next_item(&w.ctr->epa_next, lane)) {
-        int c = w.epa_list[e];
-        int2 pr = w.pairs[w.col_pair[c].x];
-        ShapeRef sa = load_shape(w, pr.x), sb = load_shape(w, pr.y);
-        int b1 = w.sinfo[pr.x].y, b2 = w.sinfo[pr.y].y;
-        q4 qa = mkq(w.q[b1]), qb = mkq(w.q[b2]);
-        v3 pa = mk3(w.pos[b1]), pb = mk3(w.pos[b2]);
-        MV portal[4];
-        for (int k = 0; k < 4; k++) {
-            portal[k].V = mk3(w.col_portal[12 * e + 3 * k + 0]);
-            portal[k].A = mk3(w.col_portal[12 * e + 3 * k + 1]);
-            portal[k].B = mk3(w.col_portal[12 * e + 3 * k + 2]);
-        }
-        v3 pA = mk3(w.col_res[3 * c + 0]), pB = mk3(w.col_res[3 * c + 1]);
-        float4 nr = w.col_res[3 * c + 2];
-        v3 n = mk3(nr);
-        float pen = nr.w;
-        q4 q = qmul(qconj(qa), qb);
-        v3 prl = rotate_inv(pb - pa, qa);
-        run_epa(E, sa, sb, q, prl, portal, pA, pB, n, pen, st, epa_calls, epa_fail);
-        if (lane == 0) {
-            w.col_res[3 * c + 0] = f4(pA, 0.f);
-            w.col_res[3 * c + 1] = f4(pB, 0.f);
-            w.col_res[3 * c + 2] = f4(n, pen);
-        }
-    }
-    if (lane == 0) {
-        if (epa_calls) atomicAdd(&w.ctr->nepa, epa_calls);
-        if (epa_fail) atomicAdd(&w.ctr->epa_fail, epa_fail);
-    }
-    int ex = st.exact;
-    for (int off = 16; off > 0; off >>= 1) ex += __shfl_xor_sync(FULL, ex, off);
-    if (lane == 0 && ex) atomicAdd(&w.ctr->exact, ex);
-}
-
 // Contact stream record: shape pair, normal with the point count (low byte) and
 // JG_STREAM_SPECULATIVE, and the points.
 __device__ __forceinline__ void write_stream(WorldDev& w, int idx, int s1, int s2, v3 n, int cnt, bool spec,
@@ -1644,146 +1651,181 @@ __device__ __forceinline__ void write_stream(WorldDev& w, int idx, int s1, int s
     for (int k = 0; k < cnt; k++) { w.cs_pa[4 * idx + k] = oA[k]; w.cs_pb[4 * idx + k] = oB[k]; }
 }
 
-// Stage 3, one thread per colliding record: world transform, the first test of the
-// triangle-edge filter (TriangleEdgeCollisionFilter.cs:183-240; pairs near a mesh edge
-// move to stage 4) and the one-shot manifold; appends the contact stream record.  A
-// speculative record (kind 3, already in world space) registers its one point
-// (World.Detect.cs:185-196).
-__global__ void __launch_bounds__(128) k_manifold(WorldDev w, StepParams sp) {
-    const int ncol = min(w.ctr->ncol, w.cap_arb);
-    int pts = 0;
-    for (int base = blockIdx.x * blockDim.x; base < ncol; base += gridDim.x * blockDim.x) {
-        int c = base + threadIdx.x;
-        bool emit = false, to_edge = false, spec = false;
-        int s1 = 0, s2 = 0, cnt = 0;
-        v3 n = mk3(0.f);
-        float4 oA[4], oB[4];
-        if (c < ncol) {
-            int2 cp = w.col_pair[c];
-            spec = cp.y == 3;
-            int2 pr = w.pairs[cp.x];
-            s1 = pr.x; s2 = pr.y;
-            ShapeRef sa = load_shape(w, s1), sb = load_shape(w, s2);
-            int b1 = w.sinfo[s1].y, b2 = w.sinfo[s2].y;
-            q4 qa = mkq(w.q[b1]), qb = mkq(w.q[b2]);
-            v3 pa = mk3(w.pos[b1]), pb = mk3(w.pos[b2]);
-            v3 pA = mk3(w.col_res[3 * c + 0]), pB = mk3(w.col_res[3 * c + 1]);
-            float4 nr = w.col_res[3 * c + 2];
-            n = mk3(nr);
-            float pen = nr.w;
-            if (!spec) {
-                pA = rotate(pA, qa); pA = pA + pa;
-                pB = rotate(pB, qa); pB = pB + pa;
-                n = rotate(n, qa);
-            }
-            emit = true;
-            bool c1 = sa.kind == JG_SHAPE_TRIANGLE, c2 = sb.kind == JG_SHAPE_TRIANGLE;
-            if (sp.edge_filter && c1 != c2) {
-                int4 i1 = w.binfo[b1], i2 = w.binfo[b2];
-                bool tri_dyn = c1 ? i1.x == JG_MOTION_DYNAMIC : i2.x == JG_MOTION_DYNAMIC;
-                if (!tri_dyn) {
-                    v3 tn, nn;
-                    int ev = edge_evaluate(w, c1 ? sa.tri : sb.tri, c1 ? qa : qb, c1 ? pa : pb, c2, c1 ? pA : pB, n, tn, nn);
-                    if (ev == DISCARD) emit = false;
-                    else if (ev == EDGE) { emit = false; to_edge = true; }
-                }
-            }
-            (void)pen;
-            if (emit) {
-                if (sp.aux_contacts && !spec) cnt = manifold_thread(sa, sb, qa, qb, pa, pb, pA, pB, n, oA, oB);
-                else { cnt = 1; oA[0] = f4(pA, 0.f); oB[0] = f4(pB, 0.f); }
-            }
-        }
-        int idx = warp_append(&w.ctr->nstream, emit);
-        if (idx >= 0) { write_stream(w, idx, s1, s2, n, cnt, spec, oA, oB); pts += cnt; }
-        int ei = warp_append(&w.ctr->nedge, to_edge);
-        if (ei >= 0) w.edge_list[ei] = c;
-    }
-    for (int off = 16; off > 0; off >>= 1) pts += __shfl_xor_sync(FULL, pts, off);
-    if ((threadIdx.x & 31) == 0 && pts) atomicAdd(&w.ctr->points, pts);
+// A colliding record in world space; a speculative one (kind 3) is there already.
+struct ColRec {
+    int s1, s2, b1, b2;
+    ShapeRef sa, sb;
+    q4 qa, qb;
+    v3 pa, pb, pA, pB, n;
+    float pen;
+};
+__device__ __forceinline__ void load_record(const WorldDev& w, int c, int2 cp, ColRec& r) {
+    const int2 pr = w.pairs[cp.x];
+    r.s1 = pr.x; r.s2 = pr.y;
+    r.sa = load_shape(w, r.s1); r.sb = load_shape(w, r.s2);
+    r.b1 = w.sinfo[r.s1].y; r.b2 = w.sinfo[r.s2].y;
+    r.qa = mkq(w.q[r.b1]); r.qb = mkq(w.q[r.b2]);
+    r.pa = mk3(w.pos[r.b1]); r.pb = mk3(w.pos[r.b2]);
+    r.pA = mk3(w.col_res[3 * c + 0]); r.pB = mk3(w.col_res[3 * c + 1]);
+    const float4 nr = w.col_res[3 * c + 2];
+    r.n = mk3(nr);
+    r.pen = nr.w;
+}
+__device__ __forceinline__ void record_to_world(ColRec& r) {
+    r.pA = rotate(r.pA, r.qa); r.pA = r.pA + r.pa;
+    r.pB = rotate(r.pB, r.qa); r.pB = r.pB + r.pa;
+    r.n = rotate(r.n, r.qa);
+}
+// A triangle of a body that is not dynamic against another kind of shape: the triangle-edge
+// filter decides about the record.
+__device__ __forceinline__ bool edge_filtered(const WorldDev& w, const StepParams& sp, const ColRec& r) {
+    const bool c1 = r.sa.kind == JG_SHAPE_TRIANGLE, c2 = r.sb.kind == JG_SHAPE_TRIANGLE;
+    return sp.edge_filter && c1 != c2 && w.binfo[c1 ? r.b1 : r.b2].x != JG_MOTION_DYNAMIC;
+}
+__device__ __forceinline__ int edge_test(const WorldDev& w, const ColRec& r, v3& tn, v3& nn) {
+    const bool c1 = r.sa.kind == JG_SHAPE_TRIANGLE;
+    return edge_evaluate(w, c1 ? r.sa.tri : r.sb.tri, c1 ? r.qa : r.qb, c1 ? r.pa : r.pb, !c1, c1 ? r.pA : r.pB, r.n, tn, nn);
 }
 
-// Stage 4, one warp per pair near a mesh edge: the rest of the triangle-edge filter
-// (rerun of MPR/EPA with threshold zero, normal snapping; TriangleEdgeCollisionFilter.cs:
-// 294-420) and the manifold.
-__global__ void __launch_bounds__(NP_WARPS * 32) k_edge(WorldDev w, StepParams sp) {
+// Stage 2, one thread per record that EPA does not change: the first test of the triangle-edge
+// filter (TriangleEdgeCollisionFilter.cs:183-240).  Records near a mesh edge go to the warps of
+// stage 3, discarded ones are struck out.  Not launched without triangles.
+__global__ void __launch_bounds__(128) k_edge_list(WorldDev w, StepParams sp) {
+    const int ncol = min(w.ctr->ncol, w.cap_arb);
+    for (int base = blockIdx.x * blockDim.x; base < ncol; base += gridDim.x * blockDim.x) {
+        const int c = base + threadIdx.x;
+        bool to_edge = false;
+        if (c < ncol) {
+            const int2 cp = w.col_pair[c];
+            const int2 pr = w.pairs[cp.x];
+            if (cp.y != 2 && (w.sinfo[pr.x].x == JG_SHAPE_TRIANGLE || w.sinfo[pr.y].x == JG_SHAPE_TRIANGLE)) {
+                ColRec r;
+                load_record(w, c, cp, r);
+                if (edge_filtered(w, sp, r)) {
+                    if (cp.y != 3) record_to_world(r);
+                    v3 tn, nn;
+                    const int ev = edge_test(w, r, tn, nn);
+                    to_edge = ev == EDGE;
+                    if (ev != KEEP) w.col_pair[c].y = to_edge ? cp.y | COL_EDGE : 0;
+                }
+            }
+        }
+        const int e = warp_append(&w.ctr->nedge, to_edge);
+        if (e >= 0) w.edge_list[e] = c;
+    }
+}
+
+// The rest of the triangle-edge filter for a record near a mesh edge (normal snapping,
+// TriangleEdgeCollisionFilter.cs:294-420) and its manifold, by the whole warp.  `snap` is false
+// when the rerun moved the record away from the edge.
+__device__ __noinline__ void edge_contact(WorldDev& w, const StepParams& sp, EpaSmem& E, ColRec& r, bool snap, bool spec, bool from_sweep,
+                                          v3 tn, v3 nn, int& pts) {
+    v3 &pA = r.pA, &pB = r.pB, &n = r.n;
+    if (snap) {
+        v3 mid = 0.5f * (pA + pB);
+        if (dot(tn, nn) > 0.999f) {
+            float f5 = dot(n, nn), f6 = dot(n, tn);
+            if (!spec) pA = pB = mid;
+            n = f5 > f6 ? nn : tn;
+        } else {
+            v3 cr = cross(nn, tn);
+            float crl = len2(cr);
+            v3 proj = n - (dot(cr, n) / crl) * cr;
+            if (len2(proj) < 0.5f * 0.5f) return;
+            float f1 = dot(cross(proj, nn), cr);
+            float f2 = dot(cross(proj, tn), cr);
+            bool between = f1 <= 0.0f && f2 >= 0.0f;
+            if (!between) {
+                float f3 = dot(n, nn), f4v = dot(n, tn);
+                if (!spec) pA = pB = mid;
+                n = f3 > f4v ? nn : tn;
+            }
+        }
+    }
+    v3 oA[4], oB[4];
+    int cnt;
+    if (sp.aux_contacts && !from_sweep) cnt = build_manifold(E, r.sa, r.sb, r.qa, r.qb, r.pa, r.pb, pA, pB, n, oA, oB);
+    else { cnt = 1; oA[0] = pA; oB[0] = pB; }
+    if ((threadIdx.x & 31) == 0) {
+        int idx = atomicAdd(&w.ctr->nstream, 1);
+        float4 fa[4], fb[4];
+        for (int k = 0; k < cnt; k++) { fa[k] = f4(oA[k], 0.f); fb[k] = f4(oB[k], 0.f); }
+        write_stream(w, idx, r.s1, r.s2, n, cnt, from_sweep, fa, fb);
+    }
+    pts += cnt;
+}
+
+// Next work item of a warp: lane 0 takes it from the cursor, every lane gets it.
+__device__ __forceinline__ int next_item(int* cursor, int lane) {
+    int e = 0;
+    if (lane == 0) e = atomicAdd(cursor, 1);
+    return __shfl_sync(0xffffffffu, e, 0);
+}
+
+// Stage 3, one warp per deep pair and per record near a mesh edge.  A deep pair: EPA from the
+// saved portal (NarrowPhase.cs:39-95); on success the record takes the EPA result, otherwise the
+// MPR result stands; then the triangle-edge filter, as in stage 2.  A record near an edge: MPR
+// and EPA again with threshold zero (for a deep pair that is what EPA has just returned, and is
+// counted but not repeated), then edge_contact.  The other records go on to stage 4.
+// Both kinds of work are searches of very different lengths, and a launch for each ended in a few
+// warps twice.  What bounds a full GPU is instruction fetch (half of the cycles between two
+// instructions of a warp on the 100k pile) and the FP64 pipe, so rare and repeated code is kept in
+// one copy, out of line; as many CTAs as shared memory holds.  Two launches -> one, in ms: a
+// pile of 700 0.40 -> 0.24, of 20k 0.53 -> 0.33, of 100k 0.95 -> 0.82, 4096 worlds 1.93 -> 1.69.
+__global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams sp) {
     extern __shared__ __align__(16) unsigned char np_smem_raw[];
     EpaSmem* smem = reinterpret_cast<EpaSmem*>(np_smem_raw);
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
-    EpaSmem& E = smem[wib];
+    EpaSmem& E = smem[threadIdx.x >> 5];
     NpStats st; st.exact = 0;
     int epa_calls = 0, epa_fail = 0, pts = 0;
-    const int ne = min(w.ctr->nedge, w.cap_arb);
-    for (int e = next_item(&w.ctr->edge_next, lane); e < ne; e = next_item(&w.ctr->edge_next, lane)) {
-        int c = w.edge_list[e];
-        int2 cp = w.col_pair[c];
-        const bool from_sweep = cp.y == 3;
-        int2 pr = w.pairs[cp.x];
-        int s1 = pr.x, s2 = pr.y;
-        ShapeRef sa = load_shape(w, s1), sb = load_shape(w, s2);
-        int b1 = w.sinfo[s1].y, b2 = w.sinfo[s2].y;
-        q4 qa = mkq(w.q[b1]), qb = mkq(w.q[b2]);
-        v3 pa = mk3(w.pos[b1]), pb = mk3(w.pos[b2]);
-        v3 pA = mk3(w.col_res[3 * c + 0]), pB = mk3(w.col_res[3 * c + 1]);
-        float4 nr = w.col_res[3 * c + 2];
-        v3 n = mk3(nr);
-        float pen = nr.w;
-        if (!from_sweep) {
-            pA = rotate(pA, qa); pA = pA + pa;
-            pB = rotate(pB, qa); pB = pB + pa;
-            n = rotate(n, qa);
-        }
-        bool c1 = sa.kind == JG_SHAPE_TRIANGLE, c2 = sb.kind == JG_SHAPE_TRIANGLE;
-        int tri = c1 ? sa.tri : sb.tri;
-        q4 tq = c1 ? qa : qb;
-        v3 tp = c1 ? pa : pb;
+    const int ne = min(w.ctr->nepa_list, w.cap_arb), total = ne + min(w.ctr->nedge, w.cap_arb);
+    // handed out one at a time: the cost varies by an order of magnitude between pairs, so a fixed
+    // share per warp would leave most warps idle behind a few
+    for (int e = next_item(&w.ctr->epa_next, lane); e < total; e = next_item(&w.ctr->epa_next, lane)) {
+        const bool deep = e < ne;
+        const int c = deep ? w.epa_list[e] : w.edge_list[e - ne];
+        const int2 cp = w.col_pair[c];
+        const bool from_sweep = (cp.y & ~COL_EDGE) == 3;
+        ColRec r;
+        load_record(w, c, cp, r);
+        const bool spec = !deep && r.pen < 0.0f;
         v3 tn, nn;
-        int ev = edge_evaluate(w, tri, tq, tp, c2, c1 ? pA : pB, n, tn, nn);
-        bool spec = pen < 0.0f;
-        bool keep = true, done = false;
-        if (!spec) {
-            bool res = mpr_epa_world(E, sa, sb, qa, qb, pa, pb, pA, pB, n, pen, 0.0f, st, epa_calls, epa_fail);
-            if (!res) keep = false;
-            else {
-                ev = edge_evaluate(w, tri, tq, tp, c2, c1 ? pA : pB, n, tn, nn);
-                if (ev == DISCARD) keep = false;
-                else if (ev == KEEP) done = true;
+        int ev;
+        if (deep) {
+            MV portal[4];
+            for (int k = 0; k < 4; k++) {
+                portal[k].V = mk3(w.col_portal[12 * e + 3 * k + 0]);
+                portal[k].A = mk3(w.col_portal[12 * e + 3 * k + 1]);
+                portal[k].B = mk3(w.col_portal[12 * e + 3 * k + 2]);
+            }
+            const int exact = st.exact, fail = epa_fail;
+            run_epa(E, r.sa, r.sb, qmul(qconj(r.qa), r.qb), rotate_inv(r.pb - r.pa, r.qa), portal, r.pA, r.pB, r.n, r.pen, st,
+                    epa_calls, epa_fail);
+            if (lane == 0) {
+                w.col_res[3 * c + 0] = f4(r.pA, 0.f);
+                w.col_res[3 * c + 1] = f4(r.pB, 0.f);
+                w.col_res[3 * c + 2] = f4(r.n, r.pen);
+            }
+            if (!edge_filtered(w, sp, r)) continue;
+            record_to_world(r);
+            ev = edge_test(w, r, tn, nn);
+            if (ev == KEEP) continue;
+            if (lane == 0) w.col_pair[c].y = 0;
+            if (ev == DISCARD) continue;
+            epa_calls++;
+            epa_fail += epa_fail - fail;
+            st.exact += st.exact - exact;
+        } else {
+            if (!from_sweep) record_to_world(r);
+            ev = edge_test(w, r, tn, nn);
+            if (!spec) {
+                if (!mpr_epa_world(E, r.sa, r.sb, r.qa, r.qb, r.pa, r.pb, r.pA, r.pB, r.n, r.pen, 0.0f, st, epa_calls, epa_fail)) continue;
+                ev = edge_test(w, r, tn, nn);
+                if (ev == DISCARD) continue;
             }
         }
-        if (!keep) continue;
-        if (!done) {
-            v3 mid = 0.5f * (pA + pB);
-            if (dot(tn, nn) > 0.999f) {
-                float f5 = dot(n, nn), f6 = dot(n, tn);
-                if (!spec) { pen = 0; pA = pB = mid; }
-                n = f5 > f6 ? nn : tn;
-            } else {
-                v3 cr = cross(nn, tn);
-                float crl = len2(cr);
-                v3 proj = n - (dot(cr, n) / crl) * cr;
-                if (len2(proj) < 0.5f * 0.5f) continue;
-                float f1 = dot(cross(proj, nn), cr);
-                float f2 = dot(cross(proj, tn), cr);
-                bool between = f1 <= 0.0f && f2 >= 0.0f;
-                if (!between) {
-                    float f3 = dot(n, nn), f4v = dot(n, tn);
-                    if (!spec) { pen = 0; pA = pB = mid; }
-                    n = f3 > f4v ? nn : tn;
-                }
-            }
-        }
-        v3 oA[4], oB[4];
-        int cnt;
-        if (sp.aux_contacts && !from_sweep) cnt = build_manifold(E, sa, sb, qa, qb, pa, pb, pA, pB, n, oA, oB);
-        else { cnt = 1; oA[0] = pA; oB[0] = pB; }
-        if (lane == 0) {
-            int idx = atomicAdd(&w.ctr->nstream, 1);
-            float4 fa[4], fb[4];
-            for (int k = 0; k < cnt; k++) { fa[k] = f4(oA[k], 0.f); fb[k] = f4(oB[k], 0.f); }
-            write_stream(w, idx, s1, s2, n, cnt, from_sweep, fa, fb);
-        }
-        pts += cnt;
+        edge_contact(w, sp, E, r, ev != KEEP, spec, from_sweep, tn, nn, pts);
     }
     if (lane == 0) {
         if (epa_calls) atomicAdd(&w.ctr->nepa, epa_calls);
@@ -1795,13 +1837,38 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_edge(WorldDev w, StepParams s
     if (lane == 0 && ex) atomicAdd(&w.ctr->exact, ex);
 }
 
+// Stage 4, one thread per record that is left: the one-shot manifold; appends the contact
+// stream record.  A speculative record registers its one point (World.Detect.cs:185-196).
+__global__ void __launch_bounds__(128) k_manifold(WorldDev w, StepParams sp) {
+    const int ncol = min(w.ctr->ncol, w.cap_arb);
+    int pts = 0;
+    for (int base = blockIdx.x * blockDim.x; base < ncol; base += gridDim.x * blockDim.x) {
+        const int c = base + threadIdx.x;
+        const int2 cp = c < ncol ? w.col_pair[c] : make_int2(0, 0);
+        const bool emit = cp.y > 0 && cp.y < COL_EDGE, spec = cp.y == 3;
+        int cnt = 0;
+        ColRec r;
+        float4 oA[4], oB[4];
+        if (emit) {
+            load_record(w, c, cp, r);
+            if (!spec) record_to_world(r);
+            if (sp.aux_contacts && !spec) cnt = manifold_thread(r.sa, r.sb, r.qa, r.qb, r.pa, r.pb, r.pA, r.pB, r.n, oA, oB);
+            else { cnt = 1; oA[0] = f4(r.pA, 0.f); oB[0] = f4(r.pB, 0.f); }
+        }
+        int idx = warp_append(&w.ctr->nstream, emit);
+        if (idx >= 0) { write_stream(w, idx, r.s1, r.s2, r.n, cnt, spec, oA, oB); pts += cnt; }
+    }
+    for (int off = 16; off > 0; off >>= 1) pts += __shfl_xor_sync(FULL, pts, off);
+    if ((threadIdx.x & 31) == 0 && pts) atomicAdd(&w.ctr->points, pts);
+}
+
 // Batched NarrowPhase.MprEpa query (NarrowPhase.cs:902-927) on the world's shapes and body poses.
 // out holds 10 floats per pair (pointA, pointB, normal, penetration, world frame) and hit the
 // method's return value; every slot is written, so neither buffer needs clearing.  Few pairs
 // take one launch with a warp per pair; many the two stages of a step, MPR with one thread per pair
 // (a warp per pair runs all its 32 lanes through the same arithmetic), then EPA with one warp per
 // deep pair.  The deep pairs go through the world's EPA list and portals, free between steps.
-// 30,001 pairs, mostly deep: 1773 us of kernels with a warp per pair, 1088 in two stages.
+// 30,001 pairs, mostly deep: 1773 us of kernels with a warp per pair, 780 in two stages.
 __device__ __forceinline__ void write_query(float* o, v3 pA, v3 pB, v3 n, float pen, q4 qa, v3 pa) {
     pA = rotate(pA, qa); pA = pA + pa;
     pB = rotate(pB, qa); pB = pB + pa;
@@ -1931,8 +1998,7 @@ constexpr int kNpSmem = NP_WARPS * (int)sizeof(EpaSmem);
 // Lets the warp-per-pair kernels take their polytopes' shared memory (above the 48 KB
 // default) on the current device; called when a world is created.
 int jg_narrowphase_init() {
-    cudaError_t e = cudaFuncSetAttribute(k_epa, cudaFuncAttributeMaxDynamicSharedMemorySize, kNpSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_edge, cudaFuncAttributeMaxDynamicSharedMemorySize, kNpSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_deep, cudaFuncAttributeMaxDynamicSharedMemorySize, kNpSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_collide_query, cudaFuncAttributeMaxDynamicSharedMemorySize, kNpSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_query_epa, cudaFuncAttributeMaxDynamicSharedMemorySize, kNpSmem);
     return e == cudaSuccess ? 0 : -1;
@@ -1982,7 +2048,7 @@ void jg_launch_narrowphase(WorldDev& w, const StepParams& p, cudaStream_t s, int
     k_pair_scatter<<<nsm * 4, 256, 0, s>>>(w, PairList{nullptr, 0});
     k_mpr<<<nsm * 2, 256, 0, s>>>(w);
     k_sweep<<<nsm * 2, 128, 0, s>>>(w, p);
-    k_epa<<<nsm * 4, NP_WARPS * 32, kNpSmem, s>>>(w);
+    if (w.ntris > 0 && p.edge_filter) k_edge_list<<<nsm * 8, 128, 0, s>>>(w, p);
+    k_deep<<<nsm * 3, NP_WARPS * 32, kNpSmem, s>>>(w, p);
     k_manifold<<<nsm * 16, 128, 0, s>>>(w, p);
-    k_edge<<<nsm * 4, NP_WARPS * 32, kNpSmem, s>>>(w, p);
 }

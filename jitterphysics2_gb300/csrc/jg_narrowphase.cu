@@ -1307,6 +1307,12 @@ finalize:
 }
 
 constexpr int NP_WARPS = 4;
+// Up to this many records per warp of stage 3, its warps take them all: a manifold is a long chain
+// of one thread (23 us for the 18 records of 27 boxes, 60 us for mixed shapes), which few records
+// leave alone on the GPU, and a warp shortens.  Narrowphase in us, by warps and by threads: 18 records
+// 47 and 53, 1149 (a pile of 700) 271 and 320, 6578 (48 worlds) 355 and 390, 13,700 (100 worlds) 416
+// and 406.
+constexpr int WARP_RECORDS = 4;
 constexpr int COL_EDGE = 8;  // in a colliding record's kind: it waits in the edge list
 
 __device__ __forceinline__ int warp_append(int* counter, bool pred) {
@@ -1766,32 +1772,36 @@ __device__ __forceinline__ int next_item(int* cursor, int lane) {
 // saved portal (NarrowPhase.cs:39-95); on success the record takes the EPA result, otherwise the
 // MPR result stands; then the triangle-edge filter, as in stage 2.  A record near an edge: MPR
 // and EPA again with threshold zero (for a deep pair that is what EPA has just returned, and is
-// counted but not repeated), then edge_contact.  The other records go on to stage 4.
+// counted but not repeated), then edge_contact.  The other records go on to stage 4, or are taken
+// here too when the colliding records are no more than `few`.
 // Both kinds of work are searches of very different lengths, and a launch for each ended in a few
 // warps twice.  What bounds a full GPU is instruction fetch (half of the cycles between two
 // instructions of a warp on the 100k pile) and the FP64 pipe, so rare and repeated code is kept in
 // one copy, out of line; as many CTAs as shared memory holds.  Two launches -> one, in ms: a
 // pile of 700 0.40 -> 0.24, of 20k 0.53 -> 0.33, of 100k 0.95 -> 0.82, 4096 worlds 1.93 -> 1.69.
-__global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams sp) {
+__global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams sp, int few) {
     extern __shared__ __align__(16) unsigned char np_smem_raw[];
     EpaSmem* smem = reinterpret_cast<EpaSmem*>(np_smem_raw);
     const int lane = threadIdx.x & 31;
     EpaSmem& E = smem[threadIdx.x >> 5];
     NpStats st; st.exact = 0;
     int epa_calls = 0, epa_fail = 0, pts = 0;
-    const int ne = min(w.ctr->nepa_list, w.cap_arb), total = ne + min(w.ctr->nedge, w.cap_arb);
+    const int ncol = min(w.ctr->ncol, w.cap_arb), ne = min(w.ctr->nepa_list, w.cap_arb), nk = ne + min(w.ctr->nedge, w.cap_arb);
+    const bool all = ncol <= few;
+    const int total = nk + (all ? ncol : 0);
     // handed out one at a time: the cost varies by an order of magnitude between pairs, so a fixed
     // share per warp would leave most warps idle behind a few
     for (int e = next_item(&w.ctr->epa_next, lane); e < total; e = next_item(&w.ctr->epa_next, lane)) {
         const bool deep = e < ne;
-        const int c = deep ? w.epa_list[e] : w.edge_list[e - ne];
+        const int c = deep ? w.epa_list[e] : (e < nk ? w.edge_list[e - ne] : e - nk);
         const int2 cp = w.col_pair[c];
+        if (e >= nk && (cp.y == 0 || cp.y == 2 || cp.y >= COL_EDGE)) continue;  // in the lists, or struck out
         const bool from_sweep = (cp.y & ~COL_EDGE) == 3;
         ColRec r;
         load_record(w, c, cp, r);
         const bool spec = !deep && r.pen < 0.0f;
-        v3 tn, nn;
-        int ev;
+        v3 tn = mk3(0.f), nn = mk3(0.f);
+        int ev = KEEP;
         if (deep) {
             MV portal[4];
             for (int k = 0; k < 4; k++) {
@@ -1802,20 +1812,25 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams s
             const int exact = st.exact, fail = epa_fail;
             run_epa(E, r.sa, r.sb, qmul(qconj(r.qa), r.qb), rotate_inv(r.pb - r.pa, r.qa), portal, r.pA, r.pB, r.n, r.pen, st,
                     epa_calls, epa_fail);
-            if (lane == 0) {
+            if (lane == 0 && !all) {
                 w.col_res[3 * c + 0] = f4(r.pA, 0.f);
                 w.col_res[3 * c + 1] = f4(r.pB, 0.f);
                 w.col_res[3 * c + 2] = f4(r.n, r.pen);
             }
-            if (!edge_filtered(w, sp, r)) continue;
+            const bool filtered = edge_filtered(w, sp, r);
+            if (!filtered && !all) continue;
             record_to_world(r);
-            ev = edge_test(w, r, tn, nn);
-            if (ev == KEEP) continue;
-            if (lane == 0) w.col_pair[c].y = 0;
-            if (ev == DISCARD) continue;
-            epa_calls++;
-            epa_fail += epa_fail - fail;
-            st.exact += st.exact - exact;
+            if (filtered) ev = edge_test(w, r, tn, nn);
+            if (ev == KEEP && !all) continue;
+            if (ev != KEEP) {
+                if (lane == 0) w.col_pair[c].y = 0;
+                if (ev == DISCARD) continue;
+                epa_calls++;
+                epa_fail += epa_fail - fail;
+                st.exact += st.exact - exact;
+            }
+        } else if (e >= nk) {
+            if (!from_sweep) record_to_world(r);
         } else {
             if (!from_sweep) record_to_world(r);
             ev = edge_test(w, r, tn, nn);
@@ -1839,8 +1854,9 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams s
 
 // Stage 4, one thread per record that is left: the one-shot manifold; appends the contact
 // stream record.  A speculative record registers its one point (World.Detect.cs:185-196).
-__global__ void __launch_bounds__(128) k_manifold(WorldDev w, StepParams sp) {
+__global__ void __launch_bounds__(128) k_manifold(WorldDev w, StepParams sp, int few) {
     const int ncol = min(w.ctr->ncol, w.cap_arb);
+    if (ncol <= few) return;  // stage 3 has done them
     int pts = 0;
     for (int base = blockIdx.x * blockDim.x; base < ncol; base += gridDim.x * blockDim.x) {
         const int c = base + threadIdx.x;
@@ -2049,6 +2065,7 @@ void jg_launch_narrowphase(WorldDev& w, const StepParams& p, cudaStream_t s, int
     k_mpr<<<nsm * 2, 256, 0, s>>>(w);
     k_sweep<<<nsm * 2, 128, 0, s>>>(w, p);
     if (w.ntris > 0 && p.edge_filter) k_edge_list<<<nsm * 8, 128, 0, s>>>(w, p);
-    k_deep<<<nsm * 3, NP_WARPS * 32, kNpSmem, s>>>(w, p);
-    k_manifold<<<nsm * 16, 128, 0, s>>>(w, p);
+    const int few = WARP_RECORDS * nsm * 3 * NP_WARPS;
+    k_deep<<<nsm * 3, NP_WARPS * 32, kNpSmem, s>>>(w, p, few);
+    k_manifold<<<nsm * 16, 128, 0, s>>>(w, p, few);
 }

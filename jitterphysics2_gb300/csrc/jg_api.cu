@@ -17,6 +17,7 @@ void jg_flip_store(WorldDev& w);
 void jg_launch_update_contacts(WorldDev& w, cudaStream_t s, int nsm);
 void jg_solver_reset_launch_cache(WorldDev& w);
 void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
+bool jg_groups_middle(const WorldDev& w, int nsm);
 int jg_solver_init();
 int jg_schedule_init();
 void jg_launch_activate(WorldDev& w, int body, cudaStream_t s);
@@ -291,7 +292,7 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     if (sp.groups) {
         jg_launch_groups(d, s, w->nsm);
         jg_launch_solve_groups(d, sp, s, w->nsm);
-        w->launches += jg_group_launches(d) + JG_GROUP_CLASSES;
+        w->launches += jg_group_launches(d) + 2 + jg_groups_middle(d, w->nsm);
     }
     if (jg_launch_solve(d, sp, s, w->nsm, w->prm.solver_block, w->prm.solver_ctas_per_sm) < 0) {
         g_err = "cooperative launch of the solver failed";

@@ -23,18 +23,15 @@ constexpr unsigned FULL = 0xffffffffu;
 
 struct MV { v3 V, A, B; };
 
-// MinkowskiDifference.Support (MinkowskiDifference.cs:57-69).  WARP: the 32 lanes of a
-// warp evaluate it together (point clouds split across lanes); otherwise one thread.
-template <bool WARP>
-__device__ __forceinline__ void mk_support_t(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, v3 d, MV& v) {
-    v3 tmp = -d;
-    v.A = WARP ? support(sa, d) : support_lane(sa, d);
-    v3 tmp2 = rotate_inv(tmp, qb);
-    v.B = WARP ? support(sb, tmp2) : support_lane(sb, tmp2);
+// MinkowskiDifference.Support (MinkowskiDifference.cs:57-69), by one thread.
+__device__ __forceinline__ void mk_support_lane(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, v3 d, MV& v) {
+    v.A = support_lane(sa, d);
+    v.B = support_lane(sb, rotate_inv(-d, qb));
     v.B = rotate(v.B, qb);
     v.B = v.B + pb;
     v.V = v.A - v.B;
 }
+// The same by the 32 lanes of a warp together (point clouds split across lanes).
 // (One copy of the support maps for both shapes, and a call: EPA, MPR and the manifold of a warp
 // kernel share an instruction cache that they fill.)
 __device__ __noinline__ void mk_support(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb, v3 d, MV& v) {
@@ -814,7 +811,7 @@ __device__ __forceinline__ void mpr_lanes(int n, float epa_threshold, Load load,
         }
         if (code < 0) {
             MV v;
-            mk_support_t<false>(sa, sb, qb, pb, M.normal, v);
+            mk_support_lane(sa, sb, qb, pb, M.normal, v);
             code = M.step<KEEP_MISS>(v, epa_threshold);
         }
     }
@@ -1581,7 +1578,7 @@ __device__ bool sweep_local(const ShapeRef& sa, const ShapeRef& sb, q4 qb, v3 pb
     float d2 = len2(v);
     while (d2 > 1e-4f * 1e-4f && iter-- != 0) {
         MV x;
-        mk_support_t<false>(sa, sb, qb, pos, v, x);
+        mk_support_lane(sa, sb, qb, pos, v, x);
         float vw = -dot(v, x.V);
         if (vw > 0.0f) {
             float vr = dot(v, sweep);

@@ -1110,13 +1110,15 @@ __device__ __forceinline__ void integrate_free_bodies(const WorldDev& w, const S
 }
 
 // The large launch takes the groups that need its shared memory, and all of them when they are
-// no more than its CTAs; the small launch takes the small groups of a step with many.
+// no more than its CTAs; the small and the middle launch take the others of a step with many (the
+// middle ones go to the large launch where there is no middle one).
 // Up to eight groups of an SM are at different places of this code at once, so its size is a
 // bound: with the passes in the code four times (biased or not, with and without constraints)
 // half of the small launch's issue slots waited for instructions.  One copy: 4096 worlds of
 // boxes and chains 4.35 -> 2.60 ms in the small launch, 5.19 -> 4.77 ms in the large one.
-template <bool kLarge>
-__global__ void __launch_bounds__(kLarge ? 256 : 64, kLarge ? 2 : 8) k_solve_groups(WorldDev w, StepParams sp, int large_ctas) {
+template <int kClass>
+__global__ void __launch_bounds__(64 << kClass, 8 >> kClass) k_solve_groups(WorldDev w, StepParams sp, int large_ctas, bool middle) {
+    constexpr bool kLarge = kClass == 2;
     extern __shared__ float4 solve_smem[];
     __shared__ int s_bucket[GROUP_BUCKETS];
     __shared__ int s_abort, s_item;
@@ -1126,12 +1128,14 @@ __global__ void __launch_bounds__(kLarge ? 256 : 64, kLarge ? 2 : 8) k_solve_gro
     int* status = &w.ctr->status;
     if (kLarge) integrate_free_bodies(w, sp, blockIdx.x * bs + tid, gridDim.x * bs);
     if (tid == 0) s_abort = 0;
-    const int small = w.gr->count[0], large = w.gr->count[1];
-    const bool few = small + large <= large_ctas;
-    const int count = kLarge ? large + (few ? small : 0) : (few ? 0 : small);
+    const int small = w.gr->count[0], mid = w.gr->count[1], large = w.gr->count[2];
+    const bool few = small + mid + large <= large_ctas;
+    const int more = few || !middle ? mid : 0;  // middle ones that the large launch takes
+    const int count = kLarge ? large + more + (few ? small : 0) : (few ? 0 : (kClass == 1 ? mid : small));
     // the first groups go one to each block in order, which spreads them over the SMs
     for (int item = blockIdx.x; item < count; ) {
-        const GroupRec R = w.gr_rec[kLarge && item < large ? w.cap_bodies + item : item - (kLarge ? large : 0)];
+        const int cls = !kLarge ? kClass : (item < large ? 2 : (item < large + more ? 1 : 0));
+        const GroupRec R = w.gr_rec[cls * (size_t)w.cap_bodies + item - (!kLarge || cls == 2 ? 0 : (cls == 1 ? large : large + more))];
         const int slots = R.nbody + R.njoint, n = R.narb + R.njoint;
         float4* body = solve_smem;
         int4* con = (int4*)(body + 4 * slots);
@@ -1275,7 +1279,7 @@ __global__ void __launch_bounds__(kLarge ? 256 : 64, kLarge ? 2 : 8) k_solve_gro
         for (int i = tid; i < R.njoint * JF4; i += bs)
             ((float4*)&w.joints[w.gr_joint[R.joint + i / JF4]])[i % JF4] = ((const float4*)joints)[i];
         if (!ok) return;
-        if (tid == 0) s_item = gridDim.x + atomicAdd(&w.gr->next[kLarge], 1);
+        if (tid == 0) s_item = gridDim.x + atomicAdd(&w.gr->next[kClass], 1);
         __syncthreads();
         item = s_item;
         __syncthreads();
@@ -1382,7 +1386,7 @@ int jg_solver_init() {
     if (cudaFuncGetAttributes(&fa, (const void*)k_solve_tasks) != cudaSuccess) return -1;
     int dyn = pb - (int)fa.sharedSizeBytes;
     if (cudaFuncSetAttribute(k_solve_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return -1;
-    const void* groups[JG_GROUP_CLASSES] = {(const void*)k_solve_groups<false>, (const void*)k_solve_groups<true>};
+    const void* groups[JG_GROUP_CLASSES] = {(const void*)k_solve_groups<0>, (const void*)k_solve_groups<1>, (const void*)k_solve_groups<2>};
     for (int c = 0; c < JG_GROUP_CLASSES; c++)
         if (cudaFuncSetAttribute(groups[c], cudaFuncAttributeMaxDynamicSharedMemorySize, jg_group_budget(c)) != cudaSuccess)
             return -1;
@@ -1406,12 +1410,20 @@ static size_t task_smem(const StepParams& p, int block) {
     return ((size_t)4 * p.task_maxb + (size_t)JG_TASK_RING * block * JG_TASK_STAGE_F4) * 16 + (size_t)4 * p.task_maxb;
 }
 
-// The group solve.  (The two launches on two streams cost more in event records and waits than
+// A launch between the two, for the groups that need more than a small CTA and leave most of a large
+// one idle, where they fill its CTAs several times over; below that a third launch adds a third
+// tail.  Solve in ms, without and with it: 800 worlds 3.09 and 3.61, 2000 4.73 and 4.90, 2500 5.53
+// and 5.33, 3200 6.96 and 6.25, 4096 8.44 and 7.59.
+bool jg_groups_middle(const WorldDev& w, int nsm) { return w.nworlds > 4 * nsm * jg_group_ctas(1); }
+
+// The group solve.  (The launches on streams of their own cost more in event records and waits than
 // their overlap gives where launches count, and nothing in between has work for both.)
 void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
-    const int large_ctas = nsm * jg_group_ctas(1);
-    k_solve_groups<true><<<large_ctas, jg_group_threads(1), jg_group_budget(1), s>>>(w, p, large_ctas);
-    k_solve_groups<false><<<nsm * jg_group_ctas(0), jg_group_threads(0), jg_group_budget(0), s>>>(w, p, large_ctas);
+    const int large_ctas = nsm * jg_group_ctas(2);
+    const bool middle = jg_groups_middle(w, nsm);
+    k_solve_groups<2><<<large_ctas, jg_group_threads(2), jg_group_budget(2), s>>>(w, p, large_ctas, middle);
+    if (middle) k_solve_groups<1><<<nsm * jg_group_ctas(1), jg_group_threads(1), jg_group_budget(1), s>>>(w, p, large_ctas, middle);
+    k_solve_groups<0><<<nsm * jg_group_ctas(0), jg_group_threads(0), jg_group_budget(0), s>>>(w, p, large_ctas, middle);
 }
 
 // The cooperative grid of each solve kernel is sized once per world (its device, block,

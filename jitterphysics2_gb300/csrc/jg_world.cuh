@@ -121,28 +121,27 @@ struct DevCounters {
     int ntasks;       // partitioned solve: tasks, arbiters in tasks, most local colours
     int narb_task;
     int task_colors;
-    int epa_next;     // work cursors of the warp-per-pair narrowphase stages
-    int edge_next;
+    int epa_next;     // work cursor of the narrowphase's warp-per-pair stage
     int nspec;        // speculative sweep candidates, and of those the pairs registered
     int nspec_hit;
-    int pad[2];
+    int pad[3];
 };
 
 // Solve groups (jg_groups.cu): independent parts of the step's constraint graph, one CTA each.
-// Two launches: many small groups (64 threads, eight CTAs an SM: 1024 limb chains solve in 0.53
+// Launches by size: many small groups (64 threads, eight CTAs an SM: 1024 limb chains solve in 0.53
 // ms, against 0.64 with 128 threads and four CTAs), and few or large ones (256 threads, two
-// an SM: 48 worlds in 1.07 ms, against 1.22 with 128 threads); the dynamic shared memory of one
-// CTA bounds a group.
-#define JG_GROUP_CLASSES 2
+// an SM: 48 worlds in 1.07 ms, against 1.22 with 128 threads), and one between for batches of
+// thousands; the dynamic shared memory of one CTA bounds a group.
+#define JG_GROUP_CLASSES 3
 // Single worlds are not split into groups above this many arbiters (a scene of that size is
 // one pile, whose components would be found for nothing), nor when a component has more rows
 // than this: a pile of 200 bodies (about 250 rows) solves in 0.79 ms as a group and 1.13 as tasks,
 // one of 400 (600 rows) in 1.35 as a group and 1.12 as tasks.
 #define JG_GROUP_MAXARB 16384
 #define JG_GROUP_MAXROWS 320
-JG_HD int jg_group_threads(int cls) { return cls == 0 ? 64 : 256; }
-JG_HD int jg_group_ctas(int cls) { return cls == 0 ? 8 : 2; }
-JG_HD int jg_group_budget(int cls) { return cls == 0 ? 23 * 1024 : 106 * 1024; }
+JG_HD int jg_group_threads(int cls) { return 64 << cls; }
+JG_HD int jg_group_ctas(int cls) { return 8 >> cls; }
+JG_HD int jg_group_budget(int cls) { return (cls == 0 ? 23 : (cls == 1 ? 51 : 106)) * 1024; }
 // Bytes of a group: per body slot (a constraint's non-dynamic body takes one too) the solver
 // record, its count and total of rows, and its id; per row its header, friction and first
 // contact; per contact its accumulated impulses; per constraint its record.
@@ -154,8 +153,8 @@ struct GroupRec { int arb, narb, joint, njoint, body, nbody, ncon, pad; };  // a
 struct GroupCtl {
     int off;                         // the groups cannot take this step
     int arbs, joints, bodies;        // space handed out
-    int count[JG_GROUP_CLASSES];     // groups that fit the small CTA, groups that need the large one
-    int next[JG_GROUP_CLASSES];      // work cursors of the two launches
+    int count[JG_GROUP_CLASSES];     // groups by the smallest CTA that fits them
+    int next[JG_GROUP_CLASSES];      // work cursors of the launches
 };
 
 struct WorldDev {

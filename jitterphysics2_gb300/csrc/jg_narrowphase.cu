@@ -1310,7 +1310,8 @@ constexpr int NP_WARPS = 4;
 // 47 and 53, 1149 (a pile of 700) 271 and 320, 6578 (48 worlds) 355 and 390, 13,700 (100 worlds) 416
 // and 406.
 constexpr int WARP_RECORDS = 4;
-constexpr int COL_EDGE = 8;  // in a colliding record's kind: it waits in the edge list
+constexpr int COL_WORLD = 4;  // kind of a colliding record that stage 3 has put into world space
+constexpr int COL_EDGE = 8;   // in a colliding record's kind: it waits in the edge list
 
 __device__ __forceinline__ int warp_append(int* counter, bool pred) {
     const int lane = threadIdx.x & 31;
@@ -1718,42 +1719,42 @@ __global__ void __launch_bounds__(128) k_edge_list(WorldDev w, StepParams sp) {
     }
 }
 
-// The rest of the triangle-edge filter for a record near a mesh edge (normal snapping,
-// TriangleEdgeCollisionFilter.cs:294-420) and its manifold, by the whole warp.  `snap` is false
-// when the rerun moved the record away from the edge.
-__device__ __noinline__ void edge_contact(WorldDev& w, const StepParams& sp, EpaSmem& E, ColRec& r, bool snap, bool spec, bool from_sweep,
-                                          v3 tn, v3 nn, int& pts) {
+// The rest of the triangle-edge filter for a record near a mesh edge: normal snapping
+// (TriangleEdgeCollisionFilter.cs:294-420); false when the record is discarded.
+__device__ __noinline__ bool edge_snap(ColRec& r, bool spec, v3 tn, v3 nn) {
     v3 &pA = r.pA, &pB = r.pB, &n = r.n;
-    if (snap) {
-        v3 mid = 0.5f * (pA + pB);
-        if (dot(tn, nn) > 0.999f) {
-            float f5 = dot(n, nn), f6 = dot(n, tn);
-            if (!spec) pA = pB = mid;
-            n = f5 > f6 ? nn : tn;
-        } else {
-            v3 cr = cross(nn, tn);
-            float crl = len2(cr);
-            v3 proj = n - (dot(cr, n) / crl) * cr;
-            if (len2(proj) < 0.5f * 0.5f) return;
-            float f1 = dot(cross(proj, nn), cr);
-            float f2 = dot(cross(proj, tn), cr);
-            bool between = f1 <= 0.0f && f2 >= 0.0f;
-            if (!between) {
-                float f3 = dot(n, nn), f4v = dot(n, tn);
-                if (!spec) pA = pB = mid;
-                n = f3 > f4v ? nn : tn;
-            }
-        }
+    v3 mid = 0.5f * (pA + pB);
+    if (dot(tn, nn) > 0.999f) {
+        float f5 = dot(n, nn), f6 = dot(n, tn);
+        if (!spec) pA = pB = mid;
+        n = f5 > f6 ? nn : tn;
+        return true;
     }
+    v3 cr = cross(nn, tn);
+    float crl = len2(cr);
+    v3 proj = n - (dot(cr, n) / crl) * cr;
+    if (len2(proj) < 0.5f * 0.5f) return false;
+    float f1 = dot(cross(proj, nn), cr);
+    float f2 = dot(cross(proj, tn), cr);
+    bool between = f1 <= 0.0f && f2 >= 0.0f;
+    if (!between) {
+        float f3 = dot(n, nn), f4v = dot(n, tn);
+        if (!spec) pA = pB = mid;
+        n = f3 > f4v ? nn : tn;
+    }
+    return true;
+}
+// The manifold of a record in world space and its contact stream record, by the whole warp.
+__device__ __noinline__ void warp_contact(WorldDev& w, const StepParams& sp, EpaSmem& E, const ColRec& r, bool from_sweep, int& pts) {
     v3 oA[4], oB[4];
     int cnt;
-    if (sp.aux_contacts && !from_sweep) cnt = build_manifold(E, r.sa, r.sb, r.qa, r.qb, r.pa, r.pb, pA, pB, n, oA, oB);
-    else { cnt = 1; oA[0] = pA; oB[0] = pB; }
+    if (sp.aux_contacts && !from_sweep) cnt = build_manifold(E, r.sa, r.sb, r.qa, r.qb, r.pa, r.pb, r.pA, r.pB, r.n, oA, oB);
+    else { cnt = 1; oA[0] = r.pA; oB[0] = r.pB; }
     if ((threadIdx.x & 31) == 0) {
         int idx = atomicAdd(&w.ctr->nstream, 1);
         float4 fa[4], fb[4];
         for (int k = 0; k < cnt; k++) { fa[k] = f4(oA[k], 0.f); fb[k] = f4(oB[k], 0.f); }
-        write_stream(w, idx, r.s1, r.s2, n, cnt, from_sweep, fa, fb);
+        write_stream(w, idx, r.s1, r.s2, r.n, cnt, from_sweep, fa, fb);
     }
     pts += cnt;
 }
@@ -1769,13 +1770,14 @@ __device__ __forceinline__ int next_item(int* cursor, int lane) {
 // saved portal (NarrowPhase.cs:39-95); on success the record takes the EPA result, otherwise the
 // MPR result stands; then the triangle-edge filter, as in stage 2.  A record near an edge: MPR
 // and EPA again with threshold zero (for a deep pair that is what EPA has just returned, and is
-// counted but not repeated), then edge_contact.  The other records go on to stage 4, or are taken
-// here too when the colliding records are no more than `few`.
+// counted but not repeated), then edge_snap.  The manifolds are left to stage 4 (in here a warp's
+// manifold, 60 KB of code, cost 84 us on the 100k pile and 30 on the 20k one), unless the colliding
+// records are no more than `few`: then the warps take all of them.
 // Both kinds of work are searches of very different lengths, and a launch for each ended in a few
 // warps twice.  What bounds a full GPU is instruction fetch (half of the cycles between two
 // instructions of a warp on the 100k pile) and the FP64 pipe, so rare and repeated code is kept in
 // one copy, out of line; as many CTAs as shared memory holds.  Two launches -> one, in ms: a
-// pile of 700 0.40 -> 0.24, of 20k 0.53 -> 0.33, of 100k 0.95 -> 0.82, 4096 worlds 1.93 -> 1.69.
+// pile of 700 0.40 -> 0.24, of 20k 0.53 -> 0.30, of 100k 0.95 -> 0.73, 4096 worlds 1.93 -> 1.69.
 __global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams sp, int few) {
     extern __shared__ __align__(16) unsigned char np_smem_raw[];
     EpaSmem* smem = reinterpret_cast<EpaSmem*>(np_smem_raw);
@@ -1809,19 +1811,13 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams s
             const int exact = st.exact, fail = epa_fail;
             run_epa(E, r.sa, r.sb, qmul(qconj(r.qa), r.qb), rotate_inv(r.pb - r.pa, r.qa), portal, r.pA, r.pB, r.n, r.pen, st,
                     epa_calls, epa_fail);
-            if (lane == 0 && !all) {
-                w.col_res[3 * c + 0] = f4(r.pA, 0.f);
-                w.col_res[3 * c + 1] = f4(r.pB, 0.f);
-                w.col_res[3 * c + 2] = f4(r.n, r.pen);
-            }
-            const bool filtered = edge_filtered(w, sp, r);
-            if (!filtered && !all) continue;
             record_to_world(r);
-            if (filtered) ev = edge_test(w, r, tn, nn);
-            if (ev == KEEP && !all) continue;
-            if (ev != KEEP) {
+            if (edge_filtered(w, sp, r)) ev = edge_test(w, r, tn, nn);
+            if (ev == DISCARD) {
                 if (lane == 0) w.col_pair[c].y = 0;
-                if (ev == DISCARD) continue;
+                continue;
+            }
+            if (ev == EDGE) {
                 epa_calls++;
                 epa_fail += epa_fail - fail;
                 st.exact += st.exact - exact;
@@ -1837,7 +1833,17 @@ __global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams s
                 if (ev == DISCARD) continue;
             }
         }
-        edge_contact(w, sp, E, r, ev != KEEP, spec, from_sweep, tn, nn, pts);
+        if (ev != KEEP && !edge_snap(r, spec, tn, nn)) {
+            if (lane == 0) w.col_pair[c].y = 0;
+            continue;
+        }
+        if (all) warp_contact(w, sp, E, r, from_sweep, pts);
+        else if (lane == 0) {
+            w.col_res[3 * c + 0] = f4(r.pA, 0.f);
+            w.col_res[3 * c + 1] = f4(r.pB, 0.f);
+            w.col_res[3 * c + 2] = f4(r.n, r.pen);
+            w.col_pair[c].y = from_sweep ? 3 : COL_WORLD;
+        }
     }
     if (lane == 0) {
         if (epa_calls) atomicAdd(&w.ctr->nepa, epa_calls);
@@ -1858,13 +1864,13 @@ __global__ void __launch_bounds__(128) k_manifold(WorldDev w, StepParams sp, int
     for (int base = blockIdx.x * blockDim.x; base < ncol; base += gridDim.x * blockDim.x) {
         const int c = base + threadIdx.x;
         const int2 cp = c < ncol ? w.col_pair[c] : make_int2(0, 0);
-        const bool emit = cp.y > 0 && cp.y < COL_EDGE, spec = cp.y == 3;
+        const bool emit = cp.y > 0 && cp.y < COL_EDGE, spec = cp.y == 3;  // (3 and COL_WORLD are in world space)
         int cnt = 0;
         ColRec r;
         float4 oA[4], oB[4];
         if (emit) {
             load_record(w, c, cp, r);
-            if (!spec) record_to_world(r);
+            if (cp.y < 3) record_to_world(r);
             if (sp.aux_contacts && !spec) cnt = manifold_thread(r.sa, r.sb, r.qa, r.qb, r.pa, r.pb, r.pA, r.pB, r.n, oA, oB);
             else { cnt = 1; oA[0] = f4(r.pA, 0.f); oB[0] = f4(r.pB, 0.f); }
         }

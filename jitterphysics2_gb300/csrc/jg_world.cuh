@@ -193,7 +193,7 @@ struct WorldDev {
     int* pair_order;             // [cap_pairs] pair indices grouped by the two shapes' kinds
     int* pair_kind;              // [2 * 64] counts, then cursors from 0, per kind combination
     // narrowphase: overlapping pairs from the MPR stage, then the contact stream
-    int2* col_pair;              // [cap_arb] pair index, kind (1 final, 2 needs EPA, 3 speculative; 0 struck out, + 8 near a mesh edge)
+    int2* col_pair;              // [cap_arb] pair index, kind (1 final, 2 needs EPA, 3 speculative, 4 in world space; 0 struck out, + 8 near a mesh edge)
     float4* col_res;             // [3 * cap_arb] MPR result in A's frame: pA, pB, normal|depth
     float4* col_portal;          // [12 * cap_arb] MPR portal (4 vertices: V, A, B), by EPA-list slot
     int* epa_list;               // [cap_arb] colliding-record index of each deep pair

@@ -59,10 +59,10 @@ STATE_CACHE = os.environ.get("JG_BENCH_CACHE", "/tmp/jitter_gb300_bench")
 
 # Figures from ncu captures (profiles/), labelled with the commit they were taken at:
 # they do not follow later code changes.
-CAPTURE = {"k_solve_tasks_dram_bytes": 0.067e9, "k_mpr_fma_pipe_pct": 33.2,
+CAPTURE = {"k_solve_tasks_dram_bytes": 0.067e9, "k_mpr_fma_pipe_pct": 23.4,
            "source": "ncu captures of the formed 100k pile: k_solve_tasks at commit 0e4443c "
                      "(profiles/k_solve_tasks_pile100k.md; later commits keep its partition of this pile), "
-                     "k_mpr at commit 20319af (profiles/k_mpr_k_epa_pile100k.md); narrowphase unchanged since"}
+                     "k_mpr at commit 2411563 (profiles/k_mpr_k_deep_pile100k.md)"}
 
 
 def peaks():
@@ -479,7 +479,7 @@ def main():
                          "bytes_model": "S*((I+R)*276*C + 320*C + 116*N) + 52*N"},
             # the narrowphase is bound by the FP32 pipe, not HBM: FMA-pipe cycles active of the
             # MPR kernel from an ncu capture of this workload
-            "narrowphase": {"bound": "fp32 pipe", "kernel": "k_mpr", "fma_pipe_active_pct": CAPTURE["k_mpr_fma_pipe_pct"],
+            "narrowphase": {"bound": "instruction issue", "kernel": "k_mpr", "fma_pipe_active_pct": CAPTURE["k_mpr_fma_pipe_pct"],
                             "fma_source": CAPTURE["source"], "ms_per_step": stage_ms["narrowphase"]}
             if args.config == "c3" and nb == N_BODIES + 2 else None,
             "clocks": clk, "gpu_launches": launches,

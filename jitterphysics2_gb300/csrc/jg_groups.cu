@@ -138,7 +138,7 @@ __global__ void k_group_offsets(WorldDev w, int share_div) {
         for (int k = 0; k < 32; k++) {
             const int r = __shfl_sync(0xffffffffu, rows, k), by = __shfl_sync(0xffffffffu, bytes, k);
             if (r == 0) continue;
-            if (run_rows == 0 || run_rows + r > share || run_bytes + by > jg_group_budget(0)) { start = k; run_rows = 0; run_bytes = 0; }
+            if (run_rows == 0 || run_rows + r > share || run_bytes + by > jg_group_smem(0)) { start = k; run_rows = 0; run_bytes = 0; }
             run_rows += r; run_bytes += by;
             if (lane == k) first = start;
         }
@@ -165,11 +165,11 @@ __global__ void k_group_offsets(WorldDev w, int share_div) {
         r.ncon = ec - (pc - ncon);
         r.narb = oa + ea - r.arb; r.njoint = oj + ej - r.joint; r.nbody = ob + eb - r.body;
         const int need = jg_group_bytes(r.nbody, r.narb, r.njoint, r.ncon);
-        if (need > jg_group_budget(2) || r.nbody + r.njoint >= 65536 || (w.nworlds <= 1 && r.narb + r.njoint > JG_GROUP_MAXROWS)) {
+        if (need > jg_group_smem(2) || r.nbody + r.njoint >= 65536 || (w.nworlds <= 1 && r.narb + r.njoint > JG_GROUP_MAXROWS)) {
             w.gr->off = 1;
             continue;
         }
-        const int cls = need > jg_group_budget(1) ? 2 : (need > jg_group_budget(0) ? 1 : 0);
+        const int cls = need > jg_group_smem(1) ? 2 : (need > jg_group_smem(0) ? 1 : 0);
         const int k = atomicAdd(&w.gr->count[cls], 1);
         w.gr_rec[cls * (size_t)w.cap_bodies + k] = r;
     }

@@ -1,8 +1,8 @@
-// Narrowphase: one warp per broadphase pair.  MPR (NarrowPhase.cs:98-347), EPA with the
-// polytope in shared memory (NarrowPhase.cs:39-95, ConvexPolytope.cs), the triangle-edge
+// Narrowphase: MPR with a search per lane (NarrowPhase.cs:98-347), EPA with the polytope in shared
+// memory and a warp per deep pair (NarrowPhase.cs:39-95, ConvexPolytope.cs), the triangle-edge
 // filter (TriangleEdgeCollisionFilter.cs:243-420) and the one-shot manifold
-// (CollisionManifold.cs:393-566) run fused; colliding pairs append one record (key,
-// normal, up to four point pairs) to the compacted contact stream.
+// (CollisionManifold.cs:393-566) with a thread, or in small steps a warp, per record; colliding
+// pairs append one record (key, normal, up to four point pairs) to the compacted contact stream.
 //
 // In the warp-per-pair stages the lanes hold identical copies of the MPR state; point-cloud
 // support maps, the EPA face scans (closest face, visibility, horizon), the FP64 face geometry

@@ -1388,7 +1388,7 @@ int jg_solver_init() {
     if (cudaFuncSetAttribute(k_solve_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess) return -1;
     const void* groups[JG_GROUP_CLASSES] = {(const void*)k_solve_groups<0>, (const void*)k_solve_groups<1>, (const void*)k_solve_groups<2>};
     for (int c = 0; c < JG_GROUP_CLASSES; c++)
-        if (cudaFuncSetAttribute(groups[c], cudaFuncAttributeMaxDynamicSharedMemorySize, jg_group_budget(c)) != cudaSuccess)
+        if (cudaFuncSetAttribute(groups[c], cudaFuncAttributeMaxDynamicSharedMemorySize, jg_group_smem(c)) != cudaSuccess)
             return -1;
     return 0;
 }
@@ -1421,9 +1421,9 @@ bool jg_groups_middle(const WorldDev& w, int nsm) { return w.nworlds > 4 * nsm *
 void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
     const int large_ctas = nsm * jg_group_ctas(2);
     const bool middle = jg_groups_middle(w, nsm);
-    k_solve_groups<2><<<large_ctas, jg_group_threads(2), jg_group_budget(2), s>>>(w, p, large_ctas, middle);
-    if (middle) k_solve_groups<1><<<nsm * jg_group_ctas(1), jg_group_threads(1), jg_group_budget(1), s>>>(w, p, large_ctas, middle);
-    k_solve_groups<0><<<nsm * jg_group_ctas(0), jg_group_threads(0), jg_group_budget(0), s>>>(w, p, large_ctas, middle);
+    k_solve_groups<2><<<large_ctas, jg_group_threads(2), jg_group_smem(2), s>>>(w, p, large_ctas, middle);
+    if (middle) k_solve_groups<1><<<nsm * jg_group_ctas(1), jg_group_threads(1), jg_group_smem(1), s>>>(w, p, large_ctas, middle);
+    k_solve_groups<0><<<nsm * jg_group_ctas(0), jg_group_threads(0), jg_group_smem(0), s>>>(w, p, large_ctas, middle);
 }
 
 // The cooperative grid of each solve kernel is sized once per world (its device, block,

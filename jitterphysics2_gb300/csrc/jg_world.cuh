@@ -141,7 +141,7 @@ struct DevCounters {
 #define JG_GROUP_MAXROWS 320
 JG_HD int jg_group_threads(int cls) { return 64 << cls; }
 JG_HD int jg_group_ctas(int cls) { return 8 >> cls; }
-JG_HD int jg_group_budget(int cls) { return (cls == 0 ? 23 : (cls == 1 ? 51 : 106)) * 1024; }
+JG_HD int jg_group_smem(int cls) { return (cls == 0 ? 23 : (cls == 1 ? 51 : 106)) * 1024; }
 // Bytes of a group: per body slot (a constraint's non-dynamic body takes one too) the solver
 // record, its count and total of rows, and its id; per row its header, friction and first
 // contact; per contact its accumulated impulses; per constraint its record.

@@ -10,7 +10,8 @@
 //
 // The groups are used only when every one of them fits a CTA, and when no contact or
 // constraint touches a kinematic body (whose pose changes between substeps without belonging
-// to any group) or lacks a dynamic one; otherwise k_solve_tasks solves the step.  All of this is
+// to any group), lacks a dynamic one or joins dynamic bodies of two worlds of a batch (its bodies
+// would belong to two groups); otherwise k_solve_tasks solves the step.  All of this is
 // decided on the device, as the sizes live there.
 #include "jg_sync.cuh"
 
@@ -46,7 +47,10 @@ __device__ __forceinline__ bool awake(int4 bi) { return bi.x != JG_MOTION_STATIC
 __device__ __forceinline__ int member_kind(const WorldDev& w, int4 i1, int4 i2) {
     if (w.allow_deact && !awake(i1) && !awake(i2)) return 0;
     if (i1.x == JG_MOTION_KINEMATIC || i2.x == JG_MOTION_KINEMATIC) return 2;
-    return i1.x == JG_MOTION_DYNAMIC || i2.x == JG_MOTION_DYNAMIC ? 1 : 2;
+    const bool d1 = i1.x == JG_MOTION_DYNAMIC, d2 = i2.x == JG_MOTION_DYNAMIC;
+    // (a constraint may be added across worlds, and a body with rows moved to another one)
+    if (d1 && d2 && w.nworlds > 1 && i1.z != i2.z) return 2;
+    return d1 || d2 ? 1 : 2;
 }
 
 // Adds up over the lanes at the same counter first.

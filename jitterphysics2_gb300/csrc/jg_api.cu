@@ -545,6 +545,7 @@ int upload_bodies_device(jg_world* w, const jg_body_desc* b, int32_t n) {
     std::swap(w->d_desc, w->d_stage);  // the accepted descriptors
     if (D.nb != n) invalidate_graphs(w);
     D.nb = n;
+    D.nb_rows = std::max(D.nb_rows, n);
     return JG_OK;
 }
 

@@ -245,7 +245,7 @@ __global__ void k_color(WorldDev w) {
         if (tid == 0) { w.ctr->ncolors = 0; w.remaining[0] = 0; }
         return;
     }
-    for (int b = tid; b < w.nb; b += nth) { w.deg[b] = 0; w.bmask[2 * b] = 0ull; w.bmask[2 * b + 1] = 0ull; }
+    for (int b = tid; b < w.nb_rows; b += nth) { w.deg[b] = 0; w.bmask[2 * b] = 0ull; w.bmask[2 * b + 1] = 0ull; }
     for (int c = tid; c < JG_MAX_COLORS + 1; c += nth) { w.color_count[c] = 0; w.color_cursor[c] = 0; }
     if (tid < 2) w.remaining[tid] = 0;
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
@@ -261,15 +261,15 @@ __global__ void k_color(WorldDev w) {
     }
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
     // space for each body's list, in any order
-    for (int base = blockIdx.x * blockDim.x; base < w.nb; base += nth) {
+    for (int base = blockIdx.x * blockDim.x; base < w.nb_rows; base += nth) {
         const int i = base + threadIdx.x, lane = threadIdx.x & 31;
-        const int v = i < w.nb ? w.deg[i] : 0;
+        const int v = i < w.nb_rows ? w.deg[i] : 0;
         int x = v;
         for (int o = 1; o < 32; o <<= 1) { int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
         int off = 0;
         if (lane == 31 && x) off = atomicAdd(&w.remaining[1], x);
         off = __shfl_sync(0xffffffffu, off, 31);
-        if (i < w.nb) { w.adj_off[i] = off + x - v; w.deg[i] = 0; }
+        if (i < w.nb_rows) { w.adj_off[i] = off + x - v; w.deg[i] = 0; }
     }
     if (!grid_sync(w.bar_count, w.bar_gen, status)) return;
     for (int c = lo + tid; c < ncons; c += nth) {

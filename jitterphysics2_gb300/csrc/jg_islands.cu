@@ -48,7 +48,7 @@ __device__ __forceinline__ void uf_link(int* parent, int a, int b) {
 }
 
 __global__ void k_uf_init(WorldDev w) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nb; b += gridDim.x * blockDim.x) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nb_rows; b += gridDim.x * blockDim.x) {
         w.uf[b] = b;
         w.ufl[b] = 0;
     }

@@ -165,7 +165,8 @@ __global__ void k_sched_cells(WorldDev w) {
 }
 
 // Grid and cell of each arbiter; arbiter counts per cell; each cell claims slots for the
-// dynamic bodies its arbiters touch.
+// dynamic bodies its arbiters touch.  (A body beyond the uploaded ones, WorldDev::nb_rows, is in no
+// cell: its arbiters go to the remainder.)
 __global__ void k_sched_assign(WorldDev w) {
     const ArbStore& A = w.arb[w.cur];
     const int narb = min(w.ctr->narb, w.cap_arb);
@@ -178,7 +179,7 @@ __global__ void k_sched_assign(WorldDev w) {
         bool d1 = dyn(w, b.x), d2 = dyn(w, b.y);
         int g = 3, cell = -1;
         for (int k = 0; k < JG_SCHED_GRIDS; k++) {
-            int c1 = d1 ? w.sc_cell[k * cb + b.x] : -1, c2 = d2 ? w.sc_cell[k * cb + b.y] : -1;
+            int c1 = d1 && b.x < w.nb ? w.sc_cell[k * cb + b.x] : -1, c2 = d2 && b.y < w.nb ? w.sc_cell[k * cb + b.y] : -1;
             if (c1 < 0 && c2 < 0) continue;
             if ((d1 && c1 < 0) || (d2 && c2 < 0)) continue;
             if (c1 < 0 || c2 < 0 || c1 == c2) { g = k; cell = c1 >= 0 ? c1 : c2; break; }

@@ -161,6 +161,7 @@ struct WorldDev {
     // capacities
     int cap_bodies, cap_shapes, cap_pairs, cap_arb, cap_joints, cap_hull, cap_tris;
     int nb, ns, nj, nhull, ntris, nworlds;
+    int nb_rows;                 // bodies that rows may name: the most ever uploaded (constraints and cached contacts stay when fewer are)
     // bodies
     SBody* body;
     float4 *pos, *q, *dv, *dw, *il0, *il1, *force, *torque, *mat;

@@ -10,9 +10,10 @@
 //
 // The groups are used only when every one of them fits a CTA, and when no contact or
 // constraint touches a kinematic body (whose pose changes between substeps without belonging
-// to any group), lacks a dynamic one or joins dynamic bodies of two worlds of a batch (its bodies
-// would belong to two groups); otherwise k_solve_tasks solves the step.  All of this is
-// decided on the device, as the sizes live there.
+// to any group), lacks a dynamic one, joins dynamic bodies of two worlds of a batch (its bodies
+// would belong to two groups) or names a body beyond the uploaded ones (WorldDev::nb_rows; it has
+// no place here); otherwise k_solve_tasks solves the step.  All of this is decided on the
+// device, as the sizes live there.
 #include "jg_sync.cuh"
 
 namespace {
@@ -44,9 +45,9 @@ __device__ __forceinline__ bool awake(int4 bi) { return bi.x != JG_MOTION_STATIC
 
 // What a constraint means for the groups: 0 nothing to solve (asleep), 1 a group member,
 // 2 the groups cannot take it.
-__device__ __forceinline__ int member_kind(const WorldDev& w, int4 i1, int4 i2) {
+__device__ __forceinline__ int member_kind(const WorldDev& w, int2 b, int4 i1, int4 i2) {
     if (w.allow_deact && !awake(i1) && !awake(i2)) return 0;
-    if (i1.x == JG_MOTION_KINEMATIC || i2.x == JG_MOTION_KINEMATIC) return 2;
+    if (i1.x == JG_MOTION_KINEMATIC || i2.x == JG_MOTION_KINEMATIC || max(b.x, b.y) >= w.nb) return 2;
     const bool d1 = i1.x == JG_MOTION_DYNAMIC, d2 = i2.x == JG_MOTION_DYNAMIC;
     // (a constraint may be added across worlds, and a body with rows moved to another one)
     if (d1 && d2 && w.nworlds > 1 && i1.z != i2.z) return 2;
@@ -96,7 +97,7 @@ __global__ void k_group_link(WorldDev w) {
         if (c < narb) b = A.body[c];
         else { const int4 h = w.joints[c - narb].hdr; b = make_int2(h.y, h.z); }
         const int4 i1 = w.binfo[b.x], i2 = w.binfo[b.y];
-        if (i1.x != JG_MOTION_DYNAMIC || i2.x != JG_MOTION_DYNAMIC || member_kind(w, i1, i2) != 1) continue;
+        if (i1.x != JG_MOTION_DYNAMIC || i2.x != JG_MOTION_DYNAMIC || member_kind(w, b, i1, i2) != 1) continue;
         join(w.gr_root, b.x, b.y);
     }
 }
@@ -111,7 +112,7 @@ __global__ void k_group_count(WorldDev w) {
         if (c < narb) b = A.body[c];
         else { const int4 h = w.joints[c - narb].hdr; b = make_int2(h.y, h.z); }
         const int4 i1 = w.binfo[b.x], i2 = w.binfo[b.y];
-        const int kind = member_kind(w, i1, i2);
+        const int kind = member_kind(w, b, i1, i2);
         if (kind == 2) w.gr->off = 1;
         if (kind != 1) { w.gr_pos[c] = make_int2(-1, 0); continue; }
         const bool d1 = i1.x == JG_MOTION_DYNAMIC, d2 = i2.x == JG_MOTION_DYNAMIC;

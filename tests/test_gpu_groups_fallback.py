@@ -87,3 +87,22 @@ def test_contact_between_two_of_the_worlds_that_share_a_cell():
         pair.append(w)
     assert (pair[1].contacts()["body2"] == 1).any()  # the contact between worlds is still cached
     assert_equal(*pair, False)
+
+
+@pytest.mark.parametrize("make", [lambda: scenes.limb_chains(n_chains=6, links=5),
+                                  lambda: scenes.batched_worlds(n_worlds=6, lo=20, hi=40, seed=5)])
+@pytest.mark.parametrize("new_shapes", [True, False])
+def test_constraints_of_bodies_beyond_the_uploaded_ones(make, new_shapes):
+    # fewer bodies than before: the constraints of the others stay
+    sc = make()
+    keep = max(max(j[1], j[2]) for j in sc["joints"]) - 1  # (at least two bodies of a constraint are dropped)
+    a, b = pair_of_worlds(sc)
+    for w in (a, b):
+        for _ in range(10):
+            w.step(sc["dt"])
+        w.set_bodies(w.bodies()[:keep])
+        if new_shapes:
+            w.set_shapes(sc["shapes"][sc["shapes"]["body"] < keep], sc["hull"], sc["triangles"])
+        for _ in range(20):
+            w.step(sc["dt"])
+    assert_equal(a, b, True)

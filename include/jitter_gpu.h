@@ -385,6 +385,9 @@ int jg_get_constraints(jg_world* world, int32_t* order_keys, float* impulses, in
                        int32_t* out_count);
 int jg_get_counters(jg_world* world, jg_counters* out);
 int jg_get_timings(jg_world* world, jg_timings* out);
+/* Independent parts of the scene that the last step solved one CTA each, by the size of their CTA
+ * (small, middle, large); all zero when the task solve took the step. */
+int jg_get_solve_groups(jg_world* world, int32_t out[3]);
 /* Per-iteration residual of the first substep of the last step (record_residual=1), for up
  * to the first 2048 iterations:
  * r_k = |lambda_k - lambda_{k-1}| / max(|lambda_k|, 1e-12) over all contact rows. */

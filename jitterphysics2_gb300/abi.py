@@ -125,6 +125,7 @@ SIGNATURES = {
     "jg_get_constraints": (_I, [_P, _P, _P, _I, _PI]),
     "jg_get_counters": (_I, [_P, _P]),
     "jg_get_timings": (_I, [_P, _P]),
+    "jg_get_solve_groups": (_I, [_P, _P]),
     "jg_get_residuals": (_I, [_P, _P, _I, _PI]),
     "jg_export_state": (_I, [_P, _P, _I64, ctypes.POINTER(_I64)]),
     "jg_import_state": (_I, [_P, _P, _I64]),

@@ -59,6 +59,7 @@ struct jg_world {
     std::vector<void*> allocs;
     bool mlp_ready = false;
     int launches = 0;
+    bool groups = false;              // the last step was one that the groups may solve
     // jg_collide_pairs scratch, grown on demand: pairs, 10 floats and a hit flag per pair
     int2* q_pairs = nullptr;
     float* q_out = nullptr;
@@ -923,6 +924,7 @@ static int step_impl(jg_world* w, float dt, bool graph) {
     w->host_current = false;
     StepParams sp = make_params(w, dt);
     if (w->d.ns == 0 && w->d.nb == 0) return JG_OK;
+    w->groups = sp.groups != 0;
     int parity = w->d.cur;
     if (graph) {
         if (!w->graph[parity] || w->graph_dt[parity] != dt) {
@@ -971,6 +973,7 @@ int jg_stabilize(jg_world* w, float dt, int32_t iterations, int32_t relax) {
     sp.relax = relax;
     sp.stabilize = 1;
     sp.groups = 0;
+    w->groups = false;
     sp.record_residual = 0;
     WorldDev& d = w->d;
     cudaStream_t s = w->stream;
@@ -1115,6 +1118,15 @@ int jg_get_counters(jg_world* w, jg_counters* out) {
 int jg_get_timings(jg_world* w, jg_timings* out) {
     if (!w || !out) return JG_ERR_INVALID_ARG;
     *out = w->timings;
+    return JG_OK;
+}
+
+int jg_get_solve_groups(jg_world* w, int32_t out[3]) {
+    if (!w || !out) return JG_ERR_INVALID_ARG;
+    static_assert(JG_GROUP_CLASSES == 3, "out");
+    GroupCtl c{};
+    if (w->groups) CK(cudaMemcpy(&c, w->d.gr, sizeof(c), cudaMemcpyDeviceToHost));
+    for (int k = 0; k < JG_GROUP_CLASSES; k++) out[k] = c.off ? 0 : c.count[k];
     return JG_OK;
 }
 

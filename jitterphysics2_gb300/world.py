@@ -205,6 +205,13 @@ class World:
         check(self._lib.jg_get_timings(self._h, ptr(buf)), "jg_get_timings")
         return dict(zip(abi.TIMING_NAMES, buf.tolist()))
 
+    def solve_groups(self):
+        """Independent parts the last step solved one CTA each, by CTA size (small, middle, large); all
+        zero when the task solve took the step."""
+        out = np.zeros(3, np.int32)
+        check(self._lib.jg_get_solve_groups(self._h, ptr(out)), "jg_get_solve_groups")
+        return tuple(out.tolist())
+
     def residuals(self):
         buf = np.zeros(abi.RESID_MAX, np.float32)
         n = ctypes.c_int32()

@@ -76,3 +76,55 @@ def test_groups_and_tasks_give_the_same_bits(name):
     assert np.array_equal(ca, cb)
     if sc["joints"]:
         assert all(np.array_equal(x, y) for x, y in zip(a.constraints(), b.constraints()))
+
+
+@pytest.mark.parametrize("name", [n for n in CASES if n != "kinematic"])
+def test_the_groups_solve_these_scenes(name):
+    # (otherwise both worlds of the test above run the task solve)
+    make, steps, extra = CASES[name]
+    sc = make()
+    a = world_for_scene(sc, **extra)
+    by_tasks = []
+    for k in range(steps):
+        a.step(sc["dt"])
+        if a.counters()["arbiters"] or sc["joints"]:
+            asleep = not (a.bodies()["flags"] & abi.BODY_ACTIVE)[sc["bodies"]["motion_type"] == abi.MOTION_DYNAMIC].any()
+            if any(a.solve_groups()) == asleep:
+                by_tasks.append(k)
+    if name == "pile_above_the_row_limit":  # packed at first, then the bodies fall apart
+        assert 0 < len(by_tasks) < steps
+    else:
+        assert not by_tasks
+
+
+def test_solve_groups_is_zero_after_the_task_solve():
+    sc = stacks(3)
+    a, b, c = (world_for_scene(sc, **kw) for kw in ({}, dict(record_residual=1), dict(partitioned_solve=0)))
+    for w in (a, b, c):
+        w.step(sc["dt"])
+    assert [sum(w.solve_groups()) for w in (a, b, c)] == [9, 0, 0]
+    a.stabilize(sc["dt"], 2)
+    assert a.solve_groups() == (0, 0, 0)
+    k = world_for_scene(kinematic_floor())
+    k.step(sc["dt"])
+    assert k.counters()["arbiters"] > 0 and k.solve_groups() == (0, 0, 0)
+
+
+@pytest.mark.parametrize("n,by_groups", [(160, True), (161, False)])
+def test_part_at_the_row_limit(n, by_groups):
+    # a row of boxes, each touching the floor and its neighbours: one part of up to 2 n - 1 rows, 319 or
+    # 321 on both sides of the limit of 320
+    sc = scenes.box_grid(n_side=1, friction=0.6)
+    sc["bodies"] = sc["bodies"][[0] + [1] * n].copy()
+    sc["shapes"] = sc["shapes"][[0] + [1] * n].copy()
+    sc["shapes"]["body"] = np.arange(n + 1)
+    sc["bodies"]["position"][1:] = np.stack([0.999 * (np.arange(n) - n / 2), np.full(n, 0.5), np.zeros(n)], 1)
+    a, b = world_for_scene(sc), world_for_scene(sc, record_residual=1)
+    for _ in range(5):
+        a.step(sc["dt"])
+        b.step(sc["dt"])
+        assert (a.counters()["arbiters"] <= 320) == by_groups
+        assert any(a.solve_groups()) == by_groups
+    assert np.array_equal(a.bodies(), b.bodies())
+    key = ["shape1", "shape2", "slot"]
+    assert np.array_equal(*(np.sort(w.contacts(), order=key) for w in (a, b)))

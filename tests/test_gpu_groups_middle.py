@@ -24,3 +24,11 @@ def test_middle_groups_and_tasks_give_the_same_bits(lo, hi):
     ca, cb = (np.sort(w.contacts(), order=key) for w in (a, b))
     assert np.array_equal(ca, cb)
     assert all(np.array_equal(x, y) for x, y in zip(a.constraints(), b.constraints()))
+
+
+def test_the_middle_launch_has_groups():
+    sc = scenes.batched_worlds(n_worlds=2600, lo=24, hi=300, seed=21)
+    a = world_for_scene(sc)
+    for _ in range(3):
+        a.step(sc["dt"])
+        assert all(n > 0 for n in a.solve_groups())

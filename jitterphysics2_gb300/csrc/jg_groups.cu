@@ -74,9 +74,10 @@ __global__ void k_group_init(WorldDev w) {
     if (tid == 0) {
         GroupCtl c;
         memset(&c, 0, sizeof(c));
-        // (arbiters outside the tasks interleave with the constraints' levels)
+        // (arbiters outside the tasks interleave with the constraints' levels; in a step that has run out of
+        // colours two rows of a body share a level, and a group would wait for a row that never comes)
         const int narb = min(w.ctr->narb, w.cap_arb);
-        c.off = (w.nworlds <= 1 && narb > JG_GROUP_MAXARB) || narb > w.ctr->narb_task ? 1 : 0;
+        c.off = (w.nworlds <= 1 && narb > JG_GROUP_MAXARB) || narb > w.ctr->narb_task || w.ctr->status != 0 ? 1 : 0;
         *w.gr = c;
     }
     for (int b = tid; b < w.nb; b += nth) {

@@ -106,3 +106,32 @@ def test_constraints_of_bodies_beyond_the_uploaded_ones(make, new_shapes):
         for _ in range(20):
             w.step(sc["dt"])
     assert_equal(a, b, True)
+
+
+def test_more_constraints_on_a_body_than_colours():
+    # 140 constraints on one body, 128 colours: the step reports it, and no group waits for a row
+    n = 140
+    b = np.zeros(n + 1, abi.BODY_DTYPE)
+    b["orientation"][:, 3] = 1.0
+    b["position"][1:, 0] = 2.0 + 1.5 * np.arange(n)
+    b["flags"] = abi.BODY_ACTIVE
+    b["inv_mass"] = 1.0
+    b["inv_inertia"][:, [0, 3, 5]] = 6.0
+    b["linear_damping"] = b["angular_damping"] = 1.0
+    s = np.zeros(n + 1, abi.SHAPE_DTYPE)
+    s["kind"] = abi.SHAPE_BOX
+    s["body"] = np.arange(n + 1)
+    s["dims"][:, :3] = 0.5
+    w = World(max_bodies=n + 1, max_constraints=n, allow_deactivation=0)
+    w.set_bodies(b)
+    w.set_shapes(s)
+    for k in range(100):
+        w.add_constraint(abi.CONSTRAINT_BALLSOCKET, 0, k + 1, (1.0, 0.0, 0.0))
+    w.step(1.0 / 100.0)
+    assert sum(w.solve_groups()) == 1
+    for k in range(100, n):
+        w.add_constraint(abi.CONSTRAINT_BALLSOCKET, 0, k + 1, (1.0, 0.0, 0.0))
+    with pytest.raises(abi.JitterError) as e:
+        w.step(1.0 / 100.0)
+    assert e.value.code == abi.JG_ERR_CAPACITY
+    assert w.solve_groups() == (0, 0, 0)

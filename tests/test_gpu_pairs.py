@@ -58,3 +58,63 @@ def test_pairs_match_all_pairs(n, n_worlds):
     want = reference(b, s)
     assert len(got) == len(want) == w.counters()["pairs"]
     assert np.array_equal(got[np.lexsort(got.T[::-1])], want[np.lexsort(want.T[::-1])])
+
+
+def rods(n, n_worlds, seed):
+    """Parallel thin rods along (1, 1, 1), close together without touching: every two boxes overlap,
+    a 128 x 128 tile of them is 16,384 pairs."""
+    b, s = spheres(n, n_worlds, seed)
+    d = np.array([1.0, 1.0, 1.0]) / np.sqrt(3.0)
+    u = np.array([1.0, -1.0, 0.0]) / np.sqrt(2.0)
+    v = np.cross(d, u)
+    side = int(np.ceil(np.sqrt(n)))
+    i = np.arange(n)
+    g = np.stack([i % side, i // side], 1) / side - 0.5
+    b["position"] = 0.5 * (g[:, :1] * u + g[:, 1:] * v)
+    axis = np.cross([0.0, 1.0, 0.0], d)  # turns the capsule's y axis to d
+    q = np.append(axis, 1.0 + d[1])
+    b["orientation"] = q / np.linalg.norm(q)
+    s["kind"] = abi.SHAPE_CAPSULE
+    s["body"] = i
+    s["dims"][:, 0] = 1e-3
+    s["dims"][:, 1] = 2.0
+    return b, s
+
+
+def all_pairs(b, s):
+    world, dyn = b["world"][s["body"]], b["motion_type"][s["body"]] == abi.MOTION_DYNAMIC
+    act = (b["flags"][s["body"]] & abi.BODY_ACTIVE) != 0
+    i, j = np.triu_indices(len(s), 1)
+    keep = (world[i] == world[j]) & (dyn[i] | dyn[j]) & (act[i] | act[j])
+    return np.stack([i[keep], j[keep]], 1)
+
+
+@pytest.mark.parametrize("n,n_worlds", [(128, 1), (300, 2), (1000, 1), (4500, 1)])
+def test_dense_pairs_match_all_pairs(n, n_worlds):
+    # more pairs than a block's buffer holds, in one tile (up to 1,000) and over the tiles of a block (4,500)
+    b, s = rods(n, n_worlds, seed=n)
+    want = all_pairs(b, s)
+    w = World(max_bodies=n, max_shapes=n, max_pairs=len(want) + 1, n_worlds=n_worlds, allow_deactivation=0)
+    w.set_bodies(b)
+    w.set_shapes(s)
+    w.step(1.0 / 100.0)
+    got = w.pairs()
+    assert len(got) == len(want) == w.counters()["pairs"]
+    assert np.array_equal(got[np.lexsort(got.T[::-1])], want)
+
+
+def test_dense_pairs_beyond_the_pool():
+    b, s = rods(1000, 1, seed=1000)
+    want = all_pairs(b, s)
+    cap = len(want) // 4
+    w = World(max_bodies=1000, max_shapes=1000, max_pairs=cap, allow_deactivation=0)
+    w.set_bodies(b)
+    w.set_shapes(s)
+    with pytest.raises(abi.JitterError) as e:
+        w.step(1.0 / 100.0)
+    assert e.value.code == abi.JG_ERR_CAPACITY
+    got = w.pairs()
+    assert len(got) == cap
+    n = len(s)
+    key = np.sort(got[:, 0].astype(np.int64) * n + got[:, 1])
+    assert (np.diff(key) > 0).all() and np.isin(key, want[:, 0] * n + want[:, 1]).all()

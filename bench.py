@@ -446,6 +446,9 @@ def main():
     solve_timed = all(t > 0 for t in solve_ms)
     if not solve_timed:
         solve_ms = step_ms
+    # the solve that took the steps: the task solve returns at once where the groups have (batched worlds and
+    # scenes of small parts), and the solve stage holds the launches of both
+    solve_kernel = "k_solve_groups" if any(w.solve_groups()) else "k_solve_tasks"
     achieved = float(np.mean([b / (s / 1e3) for b, s in zip(sbytes, solve_ms)])) / 1e9
     nb = len(sc["bodies"])
     cnt = w.counters()
@@ -467,7 +470,7 @@ def main():
             "body_steps_per_s": nb * args.steps * ws / (total_ms / 1e3),
             "e2e": {"value": e2e_c / e2e_s, "unit": "contacts/s", "h2d_bytes_per_step": nbytes,
                     "d2h_bytes_per_step": nbytes},
-            "roofline": {"bound": "hbm", "kernel": "k_solve_tasks", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "hbm", "kernel": solve_kernel, "achieved": achieved, "peak": peak,
                          "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                          # DRAM bytes read + written by one k_solve_tasks launch of the formed
                          # 100k pile, from an ncu capture (rows stay in L2 across passes, so
@@ -475,10 +478,10 @@ def main():
                          "traffic": CAPTURE["k_solve_tasks_dram_bytes"] if args.config == "c3" and nb == N_BODIES + 2
                          else None, "traffic_source": CAPTURE["source"],
                          "solve_ms_per_step": float(np.mean(solve_ms)),
-                         "timed_span": "solve kernel" if solve_timed else "whole step (graph replay)",
+                         "timed_span": "solve stage" if solve_timed else "whole step (graph replay)",
                          "bytes_model": "S*((I+R)*276*C + 320*C + 116*N) + 52*N"},
-            # the narrowphase is bound by the FP32 pipe, not HBM: FMA-pipe cycles active of the
-            # MPR kernel from an ncu capture of this workload
+            # the narrowphase is not bound by HBM: its MPR kernel by instruction issue, with the FMA-pipe
+            # cycles active from an ncu capture of this workload
             "narrowphase": {"bound": "instruction issue", "kernel": "k_mpr", "fma_pipe_active_pct": CAPTURE["k_mpr_fma_pipe_pct"],
                             "fma_source": CAPTURE["source"], "ms_per_step": stage_ms["narrowphase"]}
             if args.config == "c3" and nb == N_BODIES + 2 else None,

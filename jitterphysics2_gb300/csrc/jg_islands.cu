@@ -68,11 +68,15 @@ __global__ void k_uf_link(WorldDev w) {
     }
 }
 
-// The island flags: the OR of the bodies' flags at each root (roots stored in uf).
+// The island flags: the OR of the bodies' flags at each root (roots stored in uf).  The paths are not
+// halved here: a halving store that comes late would put an inner node over the root another
+// thread has stored, and k_uf_apply would look up the flags there.
 __global__ void k_uf_flags(WorldDev w) {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < w.nb; b += gridDim.x * blockDim.x) {
-        int r = uf_find(w.uf, b);
-        w.uf[b] = r;
+        volatile int* p = w.uf;
+        int r = b;
+        for (int up = p[r]; up != r; up = p[r]) r = up;
+        p[b] = r;
         int f = w.binfo[b].w & 3;
         if (f) atomicOr(&w.ufl[r], f);
     }

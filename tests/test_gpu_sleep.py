@@ -209,3 +209,27 @@ def test_sleep_settings_reject_invalid_values():
             w.set_body_sleep(0, *args)
     with pytest.raises(abi.JitterError):
         w.activate_body(5)
+
+
+def test_an_island_sleeps_and_wakes_as_one():
+    # stacks that come to rest together: at every step all boxes of a stack, one island, are awake or all
+    # are asleep, and so they are when one box of every other stack is woken
+    side = 20
+    sc = scenes.box_grid(n_side=side)
+    level = (np.arange(side ** 3) // side) % side
+    stack = np.arange(side ** 3) % side + side * (np.arange(side ** 3) // (side * side))
+    sc["bodies"]["position"][1:, 1] = 0.5 + level
+    w = world_for_scene(sc, allow_deactivation=1, substeps=1, solver_iterations=6, relax_iterations=0)
+    up = np.full(side * side, side)
+    slept = woken = 0
+    for k in range(260):
+        if k % 40 == 39:
+            for s in np.flatnonzero(up == 0)[::2]:
+                w.activate_body(1 + int(np.flatnonzero(stack == s)[k % side]))
+        w.step(sc["dt"])
+        count = np.bincount(stack, weights=awake(w.bodies())[1:], minlength=side * side)
+        assert np.isin(count, (0, side)).all(), (k, np.unique(count))
+        slept += int(((up > 0) & (count == 0)).sum())
+        woken += int(((up == 0) & (count > 0)).sum())
+        up = count
+    assert slept > side * side // 4 and woken > side

@@ -61,8 +61,8 @@ STATE_CACHE = os.environ.get("JG_BENCH_CACHE", "/tmp/jitter_gb300_bench")
 # they do not follow later code changes.
 CAPTURE = {"k_solve_tasks_dram_bytes": 0.067e9, "k_mpr_fma_pipe_pct": 23.4,
            "source": "ncu captures of the formed 100k pile: k_solve_tasks at commit 0e4443c "
-                     "(profiles/k_solve_tasks_pile100k.md; later commits keep its partition of this pile), "
-                     "k_mpr at commit 2411563 (profiles/k_mpr_k_deep_pile100k.md)"}
+                     "(profiles/k_solve_tasks_pile100k.md; the same figure at commit 1481eac), "
+                     "k_mpr at commit 1481eac (profiles/k_mpr_k_deep_pile100k.md)"}
 
 
 def peaks():

@@ -223,7 +223,7 @@ __device__ __forceinline__ bool is_safe(v3 p) { return safe_coord(p.x) && safe_c
 // signs or orders are needed of decided without a division.  Every value that is used comes
 // from the reference's operations in their order, so it is that of the one-lane form bit for bit.
 // EPA of a settled 100k-body pile (7.2k deep pairs) 1374 -> 597 us, of a few hundred pairs that leave
-// only the latency of the longest one 545 -> 249; pairs near mesh edges of the former 513 -> 387.
+// only the latency of the longest one 545 -> 249 (as a launch of its own; k_deep has more to do).
 // Signs and maxima of finite doubles are decided on their bit patterns (integer pipe).
 __device__ __forceinline__ double grp(double x, int src) { return __shfl_sync(FULL, x, src, 4); }
 __device__ __forceinline__ bool x_nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
@@ -1777,7 +1777,8 @@ __device__ __forceinline__ int next_item(int* cursor, int lane) {
 // warps twice.  What bounds a full GPU is instruction fetch (half of the cycles between two
 // instructions of a warp on the 100k pile) and the FP64 pipe, so rare and repeated code is kept in
 // one copy, out of line; as many CTAs as shared memory holds.  Two launches -> one, in ms: a
-// pile of 700 0.40 -> 0.24, of 20k 0.53 -> 0.30, of 100k 0.95 -> 0.73, 4096 worlds 1.93 -> 1.69.
+// pile of 700 0.40 -> 0.24, of 20k 0.53 -> 0.33, of 100k 0.95 -> 0.82, 4096 worlds 1.93 -> 1.69;
+// with the manifolds of many records in stage 4, 0.30 and 0.73 on the two larger piles.
 __global__ void __launch_bounds__(NP_WARPS * 32) k_deep(WorldDev w, StepParams sp, int few) {
     extern __shared__ __align__(16) unsigned char np_smem_raw[];
     EpaSmem* smem = reinterpret_cast<EpaSmem*>(np_smem_raw);

@@ -128,15 +128,17 @@ struct DevCounters {
 };
 
 // Solve groups (jg_groups.cu): independent parts of the step's constraint graph, one CTA each.
-// Launches by size: many small groups (64 threads, eight CTAs an SM: 1024 limb chains solve in 0.53
-// ms, against 0.64 with 128 threads and four CTAs), and few or large ones (256 threads, two
-// an SM: 48 worlds in 1.07 ms, against 1.22 with 128 threads), and one between for batches of
-// thousands; the dynamic shared memory of one CTA bounds a group.
+// Launches by size: many small groups (64 threads, eight CTAs an SM: 1024 limb chains solve in 0.50
+// ms, against 0.62 with 128 threads and four CTAs), and few or large ones (256 threads, two
+// an SM: 48 worlds in 1.02 ms, against 1.23 with 128 threads), and one between for batches of
+// thousands; the dynamic shared memory of one CTA bounds a group.  (Whole solve stages, with the
+// search for the groups.)
 #define JG_GROUP_CLASSES 3
-// Single worlds are not split into groups above this many arbiters (a scene of that size is
-// one pile, whose components would be found for nothing), nor when a component has more rows
-// than this: a pile of 200 bodies (about 250 rows) solves in 0.79 ms as a group and 1.13 as tasks,
-// one of 400 (600 rows) in 1.35 as a group and 1.12 as tasks.
+// Single worlds are not split into groups above this many arbiters (piles of that size are
+// mostly one component, which would be found for nothing), nor when a component has more rows
+// than this.  Solve stage of mixed piles as groups and as tasks, in ms: 158 arbiters 0.54 and 0.81,
+// 340 0.81 and 1.04, 451 1.00 and 1.23, 596 0.98 and 1.05, 818 1.26 and 1.14: the two meet
+// at about 700, and the line, drawn when the passes were slower, lies safely below.
 #define JG_GROUP_MAXARB 16384
 #define JG_GROUP_MAXROWS 320
 JG_HD int jg_group_threads(int cls) { return 64 << cls; }

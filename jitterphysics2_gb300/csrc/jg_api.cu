@@ -16,8 +16,7 @@
 void jg_flip_store(WorldDev& w);
 void jg_launch_update_contacts(WorldDev& w, cudaStream_t s, int nsm);
 void jg_solver_reset_launch_cache(WorldDev& w);
-void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
-bool jg_groups_middle(const WorldDev& w, int nsm);
+int jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
 int jg_solver_init();
 int jg_schedule_init();
 void jg_launch_activate(WorldDev& w, int body, cudaStream_t s);
@@ -284,7 +283,7 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     }
     if (timed) cudaEventRecord(w->ev[3], s);
     jg_launch_schedule(d, sp, s, w->nsm);
-    if (jg_launch_color(d, s, w->nsm) < 0) {
+    if (jg_launch_color(d, s, w->nsm, sp.groups != 0) < 0) {
         g_err = "cooperative launch of the colouring failed";
         return JG_ERR_CUDA;
     }
@@ -292,8 +291,7 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     if (timed) cudaEventRecord(w->ev[4], s);
     if (sp.groups) {
         jg_launch_groups(d, s, w->nsm);
-        jg_launch_solve_groups(d, sp, s, w->nsm);
-        w->launches += jg_group_launches(d) + 2 + jg_groups_middle(d, w->nsm);
+        w->launches += jg_group_launches(d) + jg_launch_solve_groups(d, sp, s, w->nsm);
     }
     if (jg_launch_solve(d, sp, s, w->nsm, w->prm.solver_block, w->prm.solver_ctas_per_sm) < 0) {
         g_err = "cooperative launch of the solver failed";
@@ -981,7 +979,7 @@ int jg_stabilize(jg_world* w, float dt, int32_t iterations, int32_t relax) {
     k_reset_counters<<<1, 1, 0, s>>>(d.ctr);
     if (sp.allow_deact) jg_launch_islands(d, s, w->nsm);
     jg_launch_schedule(d, sp, s, w->nsm);
-    if (jg_launch_color(d, s, w->nsm) < 0) { g_err = "cooperative launch of the colouring failed"; return JG_ERR_CUDA; }
+    if (jg_launch_color(d, s, w->nsm, false) < 0) { g_err = "cooperative launch of the colouring failed"; return JG_ERR_CUDA; }
     jg_flip_store(d);
     if (jg_launch_solve(d, sp, s, w->nsm, w->prm.solver_block, w->prm.solver_ctas_per_sm) < 0) {
         g_err = "cooperative launch of the solver failed";

@@ -375,8 +375,9 @@ __global__ void k_color(WorldDev w) {
 // Moves every arbiter with contacts to the other buffer at its colour slot, four lanes per
 // arbiter, one for each contact slot (a lane that copied them one after another waited for
 // memory four times: 22 -> 9 us at a thousand arbiters).  Counts the contacts on the way; the
-// last block sets the new arbiter count.
-__global__ void k_permute(WorldDev w, int2* ev_removed, int* dst_index) {
+// last block sets the new arbiter count.  With `groups` it also clears what the search for the solve
+// groups counts in (jg_groups.cu).
+__global__ void k_permute(WorldDev w, int2* ev_removed, int* dst_index, bool groups) {
     const ArbStore& S = w.arb[w.cur];
     const ArbStore& D = w.arb[1 - w.cur];
     const int narb = w.ctr->narb < w.cap_arb ? w.ctr->narb : w.cap_arb;
@@ -450,7 +451,25 @@ __global__ void k_permute(WorldDev w, int2* ev_removed, int* dst_index) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&w.remaining[0], 1) == (int)gridDim.x - 1) w.ctr->narb = w.color_start[JG_MAX_COLORS];
+        if (atomicAdd(&w.remaining[0], 1) == (int)gridDim.x - 1) {
+            const int n = w.color_start[JG_MAX_COLORS];
+            w.ctr->narb = n;
+            if (groups) {
+                GroupCtl c;
+                memset(&c, 0, sizeof(c));
+                // (arbiters outside the tasks interleave with the constraints' levels; in a step that has run
+                // out of colours two rows of a body share a level, and a group would wait for a row that
+                // never comes)
+                c.off = (w.nworlds <= 1 && n > JG_GROUP_MAXARB) || n > w.ctr->narb_task || __ldcg(&w.ctr->status) != 0 ? 1 : 0;
+                *w.gr = c;
+            }
+        }
+    }
+    if (!groups) return;
+    const int nb = max(w.nb, w.nworlds);
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
+        if (b < w.nb) { w.gr_root[b] = b; w.gr_slot[b] = -1; }
+        w.gr_narb[b] = 0; w.gr_njoint[b] = 0; w.gr_nbody[b] = 0; w.gr_ncon[b] = 0;
     }
 }
 
@@ -505,7 +524,7 @@ void jg_launch_merge(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) 
 }
 
 // Returns 0, or -1 when the cooperative colouring launch is refused.
-int jg_launch_color(WorldDev& w, cudaStream_t s, int nsm) {
+int jg_launch_color(WorldDev& w, cudaStream_t s, int nsm, bool groups) {
     if (w.lc_color_grid == 0) {
         int occ = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_color, 256, 0);
@@ -516,7 +535,7 @@ int jg_launch_color(WorldDev& w, cudaStream_t s, int nsm) {
     void* args[] = {(void*)&w};
     cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_color, dim3(w.lc_color_grid), dim3(256), args, 0, s);
     if (e != cudaSuccess) return -1;
-    k_permute<<<nsm * 4, 256, 0, s>>>(w, w.ev_removed, w.dst_index);
+    k_permute<<<nsm * 4, 256, 0, s>>>(w, w.ev_removed, w.dst_index, groups);
     return 0;
 }
 

@@ -12,8 +12,8 @@
 // constraint touches a kinematic body (whose pose changes between substeps without belonging
 // to any group), lacks a dynamic one, joins dynamic bodies of two worlds of a batch (its bodies
 // would belong to two groups) or names a body beyond the uploaded ones (WorldDev::nb_rows; it has
-// no place here); otherwise k_solve_tasks solves the step.  All of this is decided on the
-// device, as the sizes live there.
+// no place here), and when the groups are not those that the tasks solve faster (jg_group_dense);
+// otherwise k_solve_tasks solves the step.  All of this is decided on the device, as the sizes live there.
 #include "jg_sync.cuh"
 
 namespace {
@@ -69,25 +69,6 @@ __device__ __forceinline__ int take_place(int* counter) {
     return __shfl_sync(act, base, leader) + __popc(same & ((1u << lane) - 1u));
 }
 
-__global__ void k_group_init(WorldDev w) {
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    if (tid == 0) {
-        GroupCtl c;
-        memset(&c, 0, sizeof(c));
-        // (arbiters outside the tasks interleave with the constraints' levels; in a step that has run out of
-        // colours two rows of a body share a level, and a group would wait for a row that never comes)
-        const int narb = min(w.ctr->narb, w.cap_arb);
-        c.off = (w.nworlds <= 1 && narb > JG_GROUP_MAXARB) || narb > w.ctr->narb_task || w.ctr->status != 0 ? 1 : 0;
-        *w.gr = c;
-    }
-    for (int b = tid; b < w.nb; b += nth) {
-        w.gr_root[b] = b;
-        w.gr_slot[b] = -1;
-    }
-    const int n = max(w.nb, w.nworlds);
-    for (int i = tid; i < n; i += nth) { w.gr_narb[i] = 0; w.gr_njoint[i] = 0; w.gr_nbody[i] = 0; w.gr_ncon[i] = 0; }
-}
-
 // Single worlds: the connected components.
 __global__ void k_group_link(WorldDev w) {
     if (w.gr->off) return;
@@ -128,9 +109,11 @@ __global__ void k_group_count(WorldDev w) {
 
 // Space of each component (or world), and the groups: neighbouring ones (32 keys, one warp) share
 // a CTA up to `share` rows, so that a scene of many small parts fills the lanes of a warp with
-// rows of one level; a part above that is a group by itself.
-__global__ void k_group_offsets(WorldDev w, int share_div) {
+// rows of one level; a part above that is a group by itself.  `roomy`: groups up to which the step has
+// an SM for each; `dense_class`: the smallest CTA whose groups may count as dense.
+__global__ void k_group_offsets(WorldDev w, int share_div, int roomy, int dense_class) {
     if (w.gr->off) return;
+    int contacts = 0, dense = 0, roomy_dense = 0;
     const int n = w.nworlds > 1 ? w.nworlds : w.nb;
     const int share = max((min(w.ctr->narb, w.cap_arb) + w.nj) / share_div, 1);
     const int lane = threadIdx.x & 31;
@@ -176,9 +159,34 @@ __global__ void k_group_offsets(WorldDev w, int share_div) {
             continue;
         }
         const int cls = need > jg_group_smem(1) ? 2 : (need > jg_group_smem(0) ? 1 : 0);
+        contacts += r.ncon;
+        if (cls >= dense_class && 2 * r.ncon >= 5 * (r.narb + r.njoint)) {
+            if (r.ncon > jg_group_dense(false, w.nworlds > 1)) dense += r.ncon;
+            if (r.ncon > jg_group_dense(true, w.nworlds > 1)) roomy_dense += r.ncon;
+        }
         const int k = atomicAdd(&w.gr->count[cls], 1);
         w.gr_rec[cls * (size_t)w.cap_bodies + k] = r;
     }
+    // Dense parts (mostly four contacts to a row, and more of them than the L1 holds): one of them decides
+    // for a single world, whose time is that of its longest part, more than half of the contacts for a
+    // batch.
+    contacts = __reduce_add_sync(0xffffffffu, contacts);
+    dense = __reduce_add_sync(0xffffffffu, dense);
+    roomy_dense = __reduce_add_sync(0xffffffffu, roomy_dense);
+    if (lane == 0 && contacts) {
+        atomicAdd(&w.gr->contacts, contacts);
+        if (dense) atomicAdd(&w.gr->dense, dense);
+        if (roomy_dense) atomicAdd(&w.gr->roomy_dense, roomy_dense);
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&w.gr->blocks, 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    int groups = 0;
+    for (int c = 0; c < JG_GROUP_CLASSES; c++) groups += __ldcg(&w.gr->count[c]);
+    const int d = groups <= roomy ? __ldcg(&w.gr->roomy_dense) : __ldcg(&w.gr->dense);
+    if (d > (w.nworlds > 1 ? __ldcg(&w.gr->contacts) / 2 : 0)) w.gr->off = 1;
 }
 
 // Member lists; a body's slot becomes its place among all groups' bodies.
@@ -204,13 +212,15 @@ __global__ void k_group_scatter(WorldDev w) {
 
 }  // namespace
 
-// After the colour permutation: the groups of the arbiters in the live store.
+// After the colour permutation, which has cleared what is counted here: the groups of the arbiters in the
+// live store.
 void jg_launch_groups(WorldDev& w, cudaStream_t s, int nsm) {
-    k_group_init<<<nsm * 4, 256, 0, s>>>(w);
     if (w.nworlds <= 1) k_group_link<<<nsm * 4, 256, 0, s>>>(w);
     k_group_count<<<nsm * 4, 256, 0, s>>>(w);
-    k_group_offsets<<<nsm * 2, 256, 0, s>>>(w, nsm * jg_group_ctas(0));
+    const bool batch = w.nworlds > 1;
+    k_group_offsets<<<nsm * 2, 256, 0, s>>>(w, nsm * jg_group_ctas(0), !batch || w.nworlds <= nsm ? nsm : 0,
+                                            batch && w.nworlds > 2 * nsm ? 1 : 0);
     k_group_scatter<<<nsm * 4, 256, 0, s>>>(w);
 }
 
-int jg_group_launches(const WorldDev& w) { return w.nworlds <= 1 ? 5 : 4; }
+int jg_group_launches(const WorldDev& w) { return w.nworlds <= 1 ? 4 : 3; }

@@ -1109,15 +1109,21 @@ __device__ __forceinline__ void integrate_free_bodies(const WorldDev& w, const S
     }
 }
 
-// The large launch takes the groups that need its shared memory, and all of them when they are
-// no more than its CTAs; the small and the middle launch take the others of a step with many (the
-// middle ones go to the large launch where there is no middle one).
+// What the launches of a step take: the large one the groups that need its shared memory, and all of them
+// when they are no more than `few`; the small and the middle launch take the others of a step with
+// many (the middle ones go to the large launch where there is no middle one).
+struct GroupLaunch {
+    int least, most;   // groups of the steps that the launch is for
+    int few;
+    bool middle;       // there is a middle launch
+    bool free_bodies;  // also integrate the bodies without rows
+};
 // Up to eight groups of an SM are at different places of this code at once, so its size is a
 // bound: with the passes in the code four times (biased or not, with and without constraints)
 // half of the small launch's issue slots waited for instructions.  One copy: 4096 worlds of
 // boxes and chains 4.35 -> 2.60 ms in the small launch, 5.19 -> 4.77 ms in the large one.
 template <int kClass>
-__global__ void __launch_bounds__(64 << kClass, 8 >> kClass) k_solve_groups(WorldDev w, StepParams sp, int large_ctas, bool middle) {
+__global__ void __launch_bounds__(64 << kClass, 8 >> kClass) k_solve_groups(WorldDev w, StepParams sp, GroupLaunch L) {
     constexpr bool kLarge = kClass == 2;
     extern __shared__ float4 solve_smem[];
     __shared__ int s_bucket[GROUP_BUCKETS];
@@ -1126,11 +1132,12 @@ __global__ void __launch_bounds__(64 << kClass, 8 >> kClass) k_solve_groups(Worl
     const ArbStore& A = w.arb[w.cur];
     const int tid = threadIdx.x, bs = blockDim.x;
     int* status = &w.ctr->status;
-    if (kLarge) integrate_free_bodies(w, sp, blockIdx.x * bs + tid, gridDim.x * bs);
+    if (kLarge && L.free_bodies) integrate_free_bodies(w, sp, blockIdx.x * bs + tid, gridDim.x * bs);
     if (tid == 0) s_abort = 0;
     const int small = w.gr->count[0], mid = w.gr->count[1], large = w.gr->count[2];
-    const bool few = small + mid + large <= large_ctas;
-    const int more = few || !middle ? mid : 0;  // middle ones that the large launch takes
+    const bool few = small + mid + large <= L.few;
+    if (small + mid + large < L.least || small + mid + large > L.most) return;
+    const int more = few || !L.middle ? mid : 0;  // middle ones that the large launch takes
     const int count = kLarge ? large + more + (few ? small : 0) : (few ? 0 : (kClass == 1 ? mid : small));
     // the first groups go one to each block in order, which spreads them over the SMs
     for (int item = blockIdx.x; item < count; ) {
@@ -1414,16 +1421,43 @@ static size_t task_smem(const StepParams& p, int block) {
 // one idle, where they fill its CTAs several times over; below that a third launch adds a third
 // tail.  Solve in ms, without and with it: 800 worlds 3.09 and 3.61, 2000 4.73 and 4.90, 2500 5.53
 // and 5.33, 3200 6.96 and 6.25, 4096 8.44 and 7.59.
-bool jg_groups_middle(const WorldDev& w, int nsm) { return w.nworlds > 4 * nsm * jg_group_ctas(1); }
+static bool jg_groups_middle(const WorldDev& w, int nsm) { return w.nworlds > 4 * nsm * jg_group_ctas(1); }
 
-// The group solve.  (The launches on streams of their own cost more in event records and waits than
-// their overlap gives where launches count, and nothing in between has work for both.)
-void jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
-    const int large_ctas = nsm * jg_group_ctas(2);
-    const bool middle = jg_groups_middle(w, nsm);
-    k_solve_groups<2><<<large_ctas, jg_group_threads(2), jg_group_smem(2), s>>>(w, p, large_ctas, middle);
-    if (middle) k_solve_groups<1><<<nsm * jg_group_ctas(1), jg_group_threads(1), jg_group_smem(1), s>>>(w, p, large_ctas, middle);
-    k_solve_groups<0><<<nsm * jg_group_ctas(0), jg_group_threads(0), jg_group_smem(0), s>>>(w, p, large_ctas, middle);
+template <int kClass>
+static void launch_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int ctas, bool roomy, const GroupLaunch& g) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(ctas);
+    c.blockDim = dim3(jg_group_threads(kClass));
+    c.dynamicSmemBytes = jg_group_smem(kClass);
+    c.stream = s;
+    cudaLaunchAttribute carveout;
+    carveout.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    carveout.val.sharedMemCarveout = 50;  // percent of the SM's memory: one large CTA
+    c.attrs = &carveout;
+    c.numAttrs = roomy ? 1 : 0;
+    cudaLaunchKernelEx(&c, k_solve_groups<kClass>, w, p, g);
+}
+
+// The group solve; returns the kernels launched.
+// One large CTA an SM is enough when there are no more groups than SMs.  It then leaves more than half
+// of an SM's memory to the L1, where the rows of its contacts stay from pass to pass (with two CTAs
+// an SM the L1 is 28 KB, and every pass reads them from the L2).  Solve in ms, one and two: ten blocks of
+// 27 touching boxes 2.13 and 2.76, as 48 worlds 1.99 and 2.54, a thousand boxes in stacks 0.26 and 0.30, 48
+// mixed worlds 0.89 and 1.04; 300 worlds need the two.  A batch has as many groups as worlds at most, a
+// single world as bodies; one that has more bodies than SMs gets both launches, of which one returns.
+// No launch where its groups cannot come about.  (The launches on streams of their own cost more in event
+// records and waits than their overlap gives where launches count, and nothing in between has work
+// for both.)
+int jg_launch_solve_groups(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
+    const int most = w.nworlds > 1 ? w.nworlds : w.nb, ctas = nsm * jg_group_ctas(2);
+    const bool roomy = most <= nsm || w.nworlds <= 1, middle = jg_groups_middle(w, nsm);
+    if (roomy) launch_groups<2>(w, p, s, nsm, true, GroupLaunch{0, nsm, nsm, false, true});
+    if (most <= nsm) return 1;
+    const GroupLaunch g = {roomy ? nsm + 1 : 0, most, ctas, middle, !roomy};
+    launch_groups<2>(w, p, s, ctas, false, g);
+    if (middle) launch_groups<1>(w, p, s, nsm * jg_group_ctas(1), false, g);
+    if (most > ctas) launch_groups<0>(w, p, s, nsm * jg_group_ctas(0), false, g);
+    return 1 + roomy + middle + (most > ctas);
 }
 
 // The cooperative grid of each solve kernel is sized once per world (its device, block,

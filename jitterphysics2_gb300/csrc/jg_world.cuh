@@ -141,6 +141,14 @@ struct DevCounters {
 // at about 700, and the line, drawn when the passes were slower, lies safely below.
 #define JG_GROUP_MAXARB 16384
 #define JG_GROUP_MAXROWS 320
+// Parts of mostly four contacts to a row (2.5 and more; piles of mixed shapes have 1.5) with more contacts
+// than this go to the tasks: their rows, 80 bytes a contact, do not stay in the L1 beside the groups'
+// shared memory.  One large CTA an SM (most of the L1 left), solve in ms, groups and tasks: parts of 724
+// contacts 1.28 and 1.41, of 936 1.32 and 1.10.  Two: batches of 160 worlds of 408 contacts 1.35 and 1.11, of
+// 633 2.01 and 1.65, 2000 of 998 12.9 and 10.3.  Small CTAs: ten parts among 400 boxes of 414 1.45 and 1.48,
+// of 488 2.58 and 2.49; but small groups in batches of more worlds than there are large CTAs stay, as the tasks
+// have their waves too (1000 worlds of 633 2.66 and 6.37).
+JG_HD int jg_group_dense(bool roomy, bool batch) { return roomy ? 800 : (batch ? 350 : 450); }
 JG_HD int jg_group_threads(int cls) { return 64 << cls; }
 JG_HD int jg_group_ctas(int cls) { return 8 >> cls; }
 JG_HD int jg_group_smem(int cls) { return (cls == 0 ? 23 : (cls == 1 ? 51 : 106)) * 1024; }
@@ -157,6 +165,8 @@ struct GroupCtl {
     int arbs, joints, bodies;        // space handed out
     int count[JG_GROUP_CLASSES];     // groups by the smallest CTA that fits them
     int next[JG_GROUP_CLASSES];      // work cursors of the launches
+    int contacts, dense, roomy_dense; // contacts of the groups, and of the dense ones by either limit
+    int blocks;                      // blocks of the offsets kernel that are done
 };
 
 struct WorldDev {
@@ -324,7 +334,7 @@ int  jg_launch_aabb(WorldDev& w, float dt, cudaStream_t s);
 int  jg_launch_broadphase(WorldDev& w, cudaStream_t s, int nsm);
 void jg_launch_narrowphase(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm, int tile);
 void jg_launch_merge(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
-int  jg_launch_color(WorldDev& w, cudaStream_t s, int nsm);
+int  jg_launch_color(WorldDev& w, cudaStream_t s, int nsm, bool groups);
 void jg_launch_schedule(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);
 int  jg_launch_solve(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm, int block, int ctas_per_sm);
 void jg_launch_update(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm);

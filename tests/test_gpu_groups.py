@@ -110,21 +110,48 @@ def test_solve_groups_is_zero_after_the_task_solve():
     assert k.counters()["arbiters"] > 0 and k.solve_groups() == (0, 0, 0)
 
 
-@pytest.mark.parametrize("n,by_groups", [(160, True), (161, False)])
-def test_part_at_the_row_limit(n, by_groups):
-    # a row of boxes, each touching the floor and its neighbours: one part of up to 2 n - 1 rows, 319 or
-    # 321 on both sides of the limit of 320
+def row_of(n, kind):
+    """n bodies side by side on the floor, each touching its neighbours: one part of up to 2 n - 1 rows."""
     sc = scenes.box_grid(n_side=1, friction=0.6)
     sc["bodies"] = sc["bodies"][[0] + [1] * n].copy()
     sc["shapes"] = sc["shapes"][[0] + [1] * n].copy()
+    sc["shapes"]["kind"][1:] = kind
     sc["shapes"]["body"] = np.arange(n + 1)
-    sc["bodies"]["position"][1:] = np.stack([0.999 * (np.arange(n) - n / 2), np.full(n, 0.5), np.zeros(n)], 1)
+    sc["bodies"]["position"][1:] = np.stack([0.999 * (np.arange(n) - n / 2), np.full(n, 0.495), np.zeros(n)], 1)
+    return sc
+
+
+def assert_route_and_bits(sc, rows, by_groups):
     a, b = world_for_scene(sc), world_for_scene(sc, record_residual=1)
     for _ in range(5):
         a.step(sc["dt"])
         b.step(sc["dt"])
-        assert (a.counters()["arbiters"] <= 320) == by_groups
+        assert rows(a.counters())
         assert any(a.solve_groups()) == by_groups
     assert np.array_equal(a.bodies(), b.bodies())
     key = ["shape1", "shape2", "slot"]
     assert np.array_equal(*(np.sort(w.contacts(), order=key) for w in (a, b)))
+
+
+@pytest.mark.parametrize("n,by_groups", [(160, True), (161, False)])
+def test_part_at_the_row_limit(n, by_groups):
+    # spheres: one contact to a row, 319 or 321 rows on both sides of the limit of 320
+    assert_route_and_bits(row_of(n, abi.SHAPE_SPHERE), lambda c: (c["arbiters"] <= 320) == by_groups, by_groups)
+
+
+@pytest.mark.parametrize("n,by_groups", [(95, True), (105, False)])
+def test_part_at_the_contact_limit(n, by_groups):
+    # boxes: four contacts to a row, and no more than 8 n - 4 of them; the limit is 800
+    assert_route_and_bits(row_of(n, abi.SHAPE_BOX), lambda c: (c["contacts"] <= 800) == by_groups and c["arbiters"] <= 320, by_groups)
+
+
+@pytest.mark.parametrize("worlds,by_groups", [(150, True), (160, False), (310, True)])
+def test_batch_of_dense_worlds(worlds, by_groups):
+    # 64 boxes side by side in each world, some 508 contacts: between the two limits for one and for two groups an SM,
+    # and small enough for a small CTA, of which large batches keep eight an SM
+    one = row_of(64, abi.SHAPE_BOX)
+    n = len(one["bodies"])
+    sc = dict(one, n_worlds=worlds, bodies=np.tile(one["bodies"], worlds), shapes=np.tile(one["shapes"], worlds))
+    sc["bodies"]["world"] = np.repeat(np.arange(worlds), n)
+    sc["shapes"]["body"] = np.arange(n * worlds)
+    assert_route_and_bits(sc, lambda c: 350 * worlds < c["contacts"] <= 800 * worlds, by_groups)

@@ -2035,15 +2035,17 @@ void jg_launch_manifold_query(WorldDev& w, const int2* pairs, int n, const float
 void jg_launch_collide_query(WorldDev& w, const int2* pairs, int n, float threshold, float* out, int* hit,
                              cudaStream_t s, int nsm) {
     if (n <= 0) return;
+    // the stages take as many pairs at a time as the world's lists hold deep ones
+    const int chunk = w.cap_arb < w.cap_pairs ? w.cap_arb : w.cap_pairs, few = nsm * 12 * NP_WARPS;
     // up to three pairs a warp: 1 pair 35 us a call (two stages 45), 1000 pairs 424 (472), 6000
-    // 954 (976), 12000 1043 (866)
-    if (n <= nsm * 12 * NP_WARPS) {
+    // 954 (976), 12000 1043 (866).  So where lists that hold no more would make several chunks, each of which
+    // ends in its longest pair alone: 200,000 pairs with lists of 1,024 40.5 ms in chunks and 10.0 in one
+    // launch, 30,000 with lists of 4,096 2.5 and 1.9; 12,000 (three chunks) 1.01 and 1.06.
+    if (n <= few || (chunk <= few && n > 3 * chunk)) {
         const int blocks = (n + NP_WARPS - 1) / NP_WARPS;
         k_collide_query<<<blocks < nsm * 4 ? blocks : nsm * 4, NP_WARPS * 32, kNpSmem, s>>>(w, pairs, n, threshold, out, hit);
         return;
     }
-    // as many pairs at a time as the world's lists hold deep ones
-    const int chunk = w.cap_arb < w.cap_pairs ? w.cap_arb : w.cap_pairs;
     for (int first = 0; first < n; first += chunk) {
         const int m = n - first < chunk ? n - first : chunk;
         const int2* pr = pairs + first;

@@ -31,3 +31,18 @@ def test_batch_sizes_agree(world, n):
     assert want[0].any() and not want[0].all()
     for f in range(5):
         assert np.array_equal(got[f], want[f][pick])
+
+
+@pytest.mark.parametrize("lists", [1024, 6667, 6666, 7297, 8000])
+def test_small_lists_agree(world, lists):
+    # lists of up to 7,296 pairs and more than three chunks: one launch; else chunks of two stages
+    w, base, parts = world
+    want = [np.concatenate([p[f] for p in parts]) for f in range(5)]
+    sc = scenes.free_cluster(n=150, spacing=1.2)
+    small = World(max_bodies=len(sc["bodies"]), max_arbiters=lists, max_pairs=lists)
+    small.set_bodies(sc["bodies"])
+    small.set_shapes(sc["shapes"], sc["hull"])
+    pick = np.random.default_rng(lists).integers(0, len(base), 20001)
+    got = small.collide_pairs(base[pick])
+    for f in range(5):
+        assert np.array_equal(got[f], want[f][pick])

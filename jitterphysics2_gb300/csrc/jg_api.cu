@@ -216,12 +216,21 @@ JG_HD void body_world_inertia(const jg_body_desc& b, float* i0, float* i1, float
     i1[0] = I.m23; i1[1] = I.m33;
 }
 
-__global__ void k_reset_counters(DevCounters* c) {
-    int narb = c->narb;
+// The counters and the schedule of a step start afresh.
+__global__ void k_reset_counters(WorldDev w, int partition) {
+    int narb = w.ctr->narb;
     DevCounters z;
     memset(&z, 0, sizeof(z));
     z.narb = narb;
-    *c = z;
+    *w.ctr = z;
+    SchedInfo* S = w.sc;
+    S->nrem = partition ? 0 : 1;
+    S->span_bits = 0;
+    S->bbox[0] = S->bbox[1] = 0xffffffffu;
+    S->bbox[2] = S->bbox[3] = 0u;
+    S->tag += 1;
+    S->ntasks = 0; S->narb_task = 0; S->overflow = 0; S->maxc = 0;
+    for (int g = 0; g < JG_SCHED_GRIDS; g++) { S->ntask[g] = 0; S->task_base[g] = 0; }
 }
 
 // The partition's cell density: 0 (the default) or a finite value in (0, 64].
@@ -264,7 +273,7 @@ int launch_step(jg_world* w, const StepParams& sp, bool timed) {
     WorldDev& d = w->d;
     cudaStream_t s = w->stream;
     if (timed) cudaEventRecord(w->ev[0], s);
-    k_reset_counters<<<1, 1, 0, s>>>(d.ctr);
+    k_reset_counters<<<1, 1, 0, s>>>(d, sp.partition);
     if (sp.record_residual) cudaMemsetAsync(d.resid, 0, sizeof(float) * 2 * JG_RESID_MAX, s);
     w->launches = jg_launch_aabb(d, sp.dt, s);
     w->launches += jg_launch_broadphase(d, s, w->nsm);
@@ -976,7 +985,7 @@ int jg_stabilize(jg_world* w, float dt, int32_t iterations, int32_t relax) {
     WorldDev& d = w->d;
     cudaStream_t s = w->stream;
     d.allow_deact = sp.allow_deact;
-    k_reset_counters<<<1, 1, 0, s>>>(d.ctr);
+    k_reset_counters<<<1, 1, 0, s>>>(d, sp.partition);
     if (sp.allow_deact) jg_launch_islands(d, s, w->nsm);
     jg_launch_schedule(d, sp, s, w->nsm);
     if (jg_launch_color(d, s, w->nsm, false) < 0) { g_err = "cooperative launch of the colouring failed"; return JG_ERR_CUDA; }

@@ -44,17 +44,6 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
     return x;
 }
 
-__global__ void k_sched_reset(WorldDev w, int partition) {
-    SchedInfo* S = w.sc;
-    S->nrem = partition ? 0 : 1;
-    S->span_bits = 0;
-    S->bbox[0] = S->bbox[1] = 0xffffffffu;
-    S->bbox[2] = S->bbox[3] = 0u;
-    S->tag += 1;
-    S->ntasks = 0; S->narb_task = 0; S->overflow = 0; S->maxc = 0;
-    for (int g = 0; g < JG_SCHED_GRIDS; g++) { S->ntask[g] = 0; S->task_base[g] = 0; }
-}
-
 // Bounds of the dynamic bodies and the largest horizontal span of a two-dynamic arbiter.
 __global__ void k_sched_bounds(WorldDev w) {
     const ArbStore& A = w.arb[w.cur];
@@ -464,7 +453,6 @@ size_t jg_task_color_smem(int maxb) {
 }
 
 void jg_launch_schedule(WorldDev& w, const StepParams& p, cudaStream_t s, int nsm) {
-    k_sched_reset<<<1, 1, 0, s>>>(w, p.partition);
     if (p.partition) {
         k_sched_bounds<<<nsm * 4, 256, 0, s>>>(w);
         k_sched_setup<<<1, 1, 0, s>>>(w, nsm, p.cells_per_sm, p.solve_blocks);
@@ -490,4 +478,4 @@ int jg_schedule_init() {
 }
 
 // Kernels launched by jg_launch_schedule.
-int jg_schedule_launches(const StepParams& p) { return p.partition ? 8 : 1; }
+int jg_schedule_launches(const StepParams& p) { return p.partition ? 7 : 0; }

@@ -130,8 +130,8 @@ struct DevCounters {
 // Solve groups (jg_groups.cu): independent parts of the step's constraint graph, one CTA each.
 // Launches by size: many small groups (64 threads, eight CTAs an SM: 1024 limb chains solve in 0.50
 // ms, against 0.62 with 128 threads and four CTAs), and few or large ones (256 threads, two
-// an SM: 48 worlds in 1.02 ms, against 1.23 with 128 threads), and one between for batches of
-// thousands; the dynamic shared memory of one CTA bounds a group.  (Whole solve stages, with the
+// an SM, or one where there are so few: 48 worlds in 1.02 and 0.89 ms, against 1.23 with 128 threads), and one
+// between for batches of thousands; the dynamic shared memory of one CTA bounds a group.  (Whole solve stages, with the
 // search for the groups.)
 #define JG_GROUP_CLASSES 3
 // Single worlds are not split into groups above this many arbiters (piles of that size are

@@ -136,9 +136,9 @@ struct DevCounters {
 #define JG_GROUP_CLASSES 3
 // Single worlds are not split into groups above this many arbiters (piles of that size are
 // mostly one component, which would be found for nothing), nor when a component has more rows
-// than this.  Solve stage of mixed piles as groups and as tasks, in ms: 158 arbiters 0.54 and 0.81,
-// 340 0.81 and 1.04, 451 1.00 and 1.23, 596 0.98 and 1.05, 818 1.26 and 1.14: the two meet
-// at about 700, and the line, drawn when the passes were slower, lies safely below.
+// than this.  Solve stage of mixed piles as groups and as tasks, in ms: 158 arbiters 0.43 and 0.81,
+// 340 0.68 and 1.05, 451 0.86 and 1.24, 596 0.89 and 1.05, 818 1.22 and 1.13: the two meet
+// at about 750, and the line, drawn when the passes were slower, lies safely below.
 #define JG_GROUP_MAXARB 16384
 #define JG_GROUP_MAXROWS 320
 // Parts of mostly four contacts to a row (2.5 and more; piles of mixed shapes have 1.5) with more contacts

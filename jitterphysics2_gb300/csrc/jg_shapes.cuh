@@ -124,7 +124,7 @@ __device__ __forceinline__ v3 support_lane(const ShapeRef& s, v3 d) {
             float4 p = __ldg(s.hull + i);
             float dx = p.x * d.x, dy = p.y * d.y, dz = p.z * d.z;
             float dp = dx + (dy + dz);
-            if (dp < best) continue;
+            if (!(dp >= best)) continue;  // (a direction that is not a number: the first vertex, as the warp's)
             best = dp; bi = i;
         }
         float4 p = __ldg(s.hull + bi);

@@ -46,3 +46,23 @@ def test_small_lists_agree(world, lists):
     got = small.collide_pairs(base[pick])
     for f in range(5):
         assert np.array_equal(got[f], want[f][pick])
+
+
+def test_batch_sizes_agree_where_a_pose_has_overflowed():
+    # a body thrown out of the float range: its queries miss, and the points they report are the same in every batch
+    sc = scenes.free_cluster(n=60, spacing=1.2)
+    lost = 7
+    sc["bodies"]["velocity"][lost] = 3e38
+    w = World(max_bodies=60, max_pairs=30000, max_arbiters=30000, gravity=(0.0, 0.0, 0.0), allow_deactivation=0)
+    w.set_bodies(sc["bodies"])
+    w.set_shapes(sc["shapes"], sc["hull"])
+    w.step(1.0)
+    w.step(1.0)
+    assert not np.isfinite(w.bodies()["position"][lost]).all()
+    other = np.delete(np.arange(60), lost)
+    base = np.concatenate([np.stack([other, np.full(59, lost)], 1), np.stack([np.full(59, lost), other], 1)]).astype(np.int32)
+    alone = w.collide_pairs(base)
+    pick = np.random.default_rng(3).integers(0, len(base), 9000)
+    got = w.collide_pairs(base[pick])
+    for f in range(5):
+        assert np.array_equal(got[f], alone[f][pick], equal_nan=f > 0)
